@@ -72,3 +72,62 @@ def test_noalloc_rejects_oversize(ctx):
     one = C.c_void_p(1)
     rc = lib.bp_residual_noalloc(4101, 4101, 1, 1, *([one] * 12), None)
     assert rc == 10
+
+
+@pytest.mark.parametrize("dims", [(6, 6, 1, 1), (6, 9, 3, 0), (9, 7, 3, 1), (40, 23, 11, 1), (64, 64, 15, 0)],
+                         ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("offset", [0, 1])
+def test_noalloc_residual_chunk_edges(dims, offset):
+    """Chunks of 32 rows: odd and even numbers of rows, one level, rows whose
+    chunk ends the arrays, no active vertex, matrix pointers 16-byte aligned
+    (bulk copies) and not (plain loads), more chunks than resident blocks.
+    27 products of random values in [-1, 1] per row and block: rounding below
+    60 x 2^-53 x 108 < 1e-12 absolute; the norms to the same, relative."""
+    import torch
+
+    nx, ny, nz, periodic = dims
+    lib = solver.lib()
+    lib.bp_residual_noalloc.argtypes = [C.c_int] * 4 + [_dp] * 13
+    rng = np.random.default_rng(sum(dims) + offset)
+    V, W = nx - 1, ny - 1
+    A = [rng.uniform(-1, 1, (W, V, nz, 27)) for _ in range(4)]
+    xu, xv, bu, bv = (rng.uniform(-1, 1, (W, V, nz)) for _ in range(4))
+    for share in (0.0, 0.5, 1.0):
+        av = (rng.uniform(size=(W, V)) < share).astype(np.int32)
+        lo = 2 if periodic else 1
+        rows = np.zeros((W, V), bool)
+        rows[lo:ny - 2, lo:nx - 2] = True
+        rows &= av.astype(bool)
+        eu, ev = np.zeros((W, V, nz)), np.zeros((W, V, nz))
+        X = [np.pad(a, 1) for a in (xu, xv)]
+        for m in range(27):
+            i, j, k = m % 3, (m // 3) % 3, m // 9
+            su, sv = (a[j:j + W, i:i + V, k:k + nz] for a in X)
+            eu += A[0][..., m] * su + A[1][..., m] * sv
+            ev += A[2][..., m] * su + A[3][..., m] * sv
+        eu = np.where(rows[..., None], eu - bu, 0.0)
+        ev = np.where(rows[..., None], ev - bv, 0.0)
+        dev = torch.device("cuda:0")
+
+        def up(a, off=0):  # off: start the array 8 bytes past a 16-byte boundary
+            t = torch.zeros(a.size + 2, device=dev, dtype=torch.float64)
+            t[off:off + a.size] = torch.from_numpy(a.reshape(-1))
+            return t[off:off + a.size]
+
+        dA = [up(a, offset) for a in A]
+        d = [up(a) for a in (xu, xv, bu, bv)]
+        dav = torch.from_numpy(av).to(dev)
+        out = [torch.full((W * V * nz,), np.nan, device=dev, dtype=torch.float64) for _ in range(2)]
+        dn = torch.full((3,), np.nan, device=dev, dtype=torch.float64)
+        rc = lib.bp_residual_noalloc(nx, ny, nz, periodic, dav.data_ptr(), *[a.data_ptr() for a in dA],
+                                     *[a.data_ptr() for a in d], *[a.data_ptr() for a in out], dn.data_ptr(),
+                                     torch.cuda.current_stream(dev).cuda_stream)
+        assert rc == 0
+        ru, rv = (o.cpu().numpy().reshape(W, V, nz) for o in out)
+        assert np.max(np.abs(ru - eu)) <= 1e-12 and np.max(np.abs(rv - ev)) <= 1e-12
+        r3 = rows[..., None]
+        nr = np.sqrt(np.sum(eu ** 2 + ev ** 2))
+        nb = np.sqrt(np.sum(np.where(r3, bu ** 2 + bv ** 2, 0.0)))
+        nrm = dn.cpu().numpy()
+        assert abs(nrm[0] - nr) <= 1e-12 * max(nr, 1.0) and abs(nrm[1] - nb) <= 1e-12 * max(nb, 1.0)
+        assert abs(nrm[2] - (nr / nb if nb > 0 else 0.0)) <= 1e-11
