@@ -28,13 +28,14 @@
 #include <cuda_runtime.h>
 #else
 #define BP_HD inline
-#include <vector_types.h>  // double2 / float2 (plain structs under a host compiler)
+#include <vector_types.h>  // double2 / float2 / ulonglong2 (plain structs under a host compiler)
 #endif
 
 namespace bp {
 
 constexpr int kNzMax = 64;     // largest supported number of levels
 constexpr int kTile = 256;     // nodes per tile; one CTA of kTile threads per tile
+constexpr int kXchSumCopies = 8;  // resident PCG: copies of every published sum
 constexpr double kVol0 = 1.0e9;  // volume scale, glissade_velo_higher.F90:1111
 
 // Velocity-dependent sliding law of an instance (calcbeta,
@@ -192,6 +193,20 @@ struct DevView {
   // reductions
   double* partials;        // [3][ntiles]
   unsigned* tile_counter;  // [ninst]
+  // resident PCG (xch null: the problem's PCG runs as one launch per step):
+  // [2][kXchSumCopies][ntiles][4] 16-byte (value, epoch) slots of the tiles' block sums,
+  // [2][npad][2] of the node vectors that neighbouring tiles exchange (z, x),
+  // and the last epoch used by each instance; the columns each tile reads from
+  // other tiles (their nodes at level 0, tile t's at [halo_begin[t],
+  // halo_begin[t+1])) and each column's stencil neighbours as slots of its
+  // tile: own column c - tile_col0, W + h for halo column h, -1 = none
+  ulonglong2* xch;
+  ulonglong2* xch_node;
+  unsigned long long* xch_epoch;
+  const int* halo_begin;   // [ntiles + 1]
+  const int* halo_node;
+  const int* col_loc;      // [9][ncols]
+  int halo_max;            // most halo columns of a tile
 };
 
 // Node of (col, k) in the blocked level-major layout.

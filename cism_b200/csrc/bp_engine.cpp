@@ -271,6 +271,35 @@ DevView make_view(Arena& a, cudaStream_t s, const HostPlan& p, bool with_cells, 
   return v;
 }
 
+// The resident PCG (launch_pcg_resident) where every tile of the problem
+// fits on the GPU at once.
+void use_resident_pcg(bp_ctx* c, Arena& a, DevView* v, const HostPlan& p) {
+  if (p.ntiles == 0 || p.ntiles > kResidentMaxTiles) return;
+  const HaloPlan h = build_halo(p);
+  v->halo_max = h.max_cols;
+  if (p.ntiles > resident_ctas(*v, p.inst[0].variant, c->num_sms)) return;
+  cudaStream_t s = c->stream;
+  // one block: the slots, the epochs, then the halo tables
+  const size_t sums = 2 * (size_t)kXchSumCopies * p.ntiles * 4, nodes = 2 * 2 * (size_t)p.npad;
+  const size_t epochs = ((size_t)p.ninst + 1) / 2;
+  std::vector<int> tables(h.begin);
+  tables.insert(tables.end(), h.node.begin(), h.node.end());
+  tables.insert(tables.end(), h.col_loc.begin(), h.col_loc.end());
+  const size_t head = sums + nodes + epochs;
+  ulonglong2* block = a.get<ulonglong2>(s, "resident", head + (tables.size() + 3) / 4);
+  // epochs count from 1: no slot may hold one from an earlier problem
+  CK(cudaMemsetAsync(block, 0, sizeof(ulonglong2) * head, s));
+  int* t = reinterpret_cast<int*>(block + head);
+  upload(s, t, tables);
+  CK(cudaStreamSynchronize(s));  // tables is a host temporary
+  v->xch = block;
+  v->xch_node = block + sums;
+  v->xch_epoch = reinterpret_cast<unsigned long long*>(block + sums + nodes);
+  v->halo_begin = t;
+  v->halo_node = t + h.begin.size();
+  v->col_loc = t + h.begin.size() + h.node.size();
+}
+
 void init_state(cudaStream_t s, const DevView& v, const HostPlan& p, bool picard, bool pcg) {
   const int ninst = p.ninst;
   std::vector<InstState> st(ninst);
@@ -417,8 +446,11 @@ int pcg_head(bp_problem* P) {
   return n;
 }
 
-// FP64 PCG for all instances with pcg_active, after MV_INIT: the head,
-// then check chunks until the device counter shows no active instance (the
+// Timing runs (events around every launch) keep the launched PCG.
+bool resident_pcg(const bp_problem* P) { return P->v.xch && !P->timing.on; }
+
+// FP64 PCG for all instances with pcg_active, after MV_INIT: one launch of
+// the resident kernel, or the head, then check chunks until the device counter shows no active instance (the
 // host learns it one chunk late; the extra chunk's kernels find no active
 // instance and return at once).
 void run_pcg_fp64(bp_problem* P) {
@@ -426,6 +458,10 @@ void run_pcg_fp64(bp_problem* P) {
   const DevView& v = P->v;
   bp_ctx* c = P->c;
   const int variant = p.inst[0].variant;
+  if (resident_pcg(P)) {
+    CK(launch_pcg_resident(v, variant, c->stream));
+    return;
+  }
   const int ncheck = std::max(1, p.inst[0].ncheck);
   const int maxit = max_pcg_iters(p);
   int n = pcg_head(P);
@@ -480,6 +516,7 @@ void autotune(bp_problem* P) {
   bp_ctx* c = P->c;
   DevView& v = P->v;
   P->tuned = true;
+  if (v.xch) return;  // the resident PCG has no launch shape to choose
   if (const char* e = std::getenv("BP_MV_CONFIG")) {
     int a[4] = {0, 0, 0, 0};
     const int n = std::sscanf(e, "%d,%d,%d,%d", &a[0], &a[1], &a[2], &a[3]);
@@ -551,7 +588,7 @@ void autotune(bp_problem* P) {
 
 // The Picard loop of glissade_velo_higher_solve on the device.
 // Keeps the FP32 Krylov matrix of the mixed path (A32 with its FP64
-// diagonal, one block) in L2 across the PCG iterations of a run.  Every
+// diagonal, one block; the resident PCG holds it in shared memory) in L2 across the PCG iterations of a run.  Every
 // matvec re-reads the whole block, and the update kernels stream about as
 // many bytes of vectors in between, which would evict it.  The PCG
 // kernels' launches carry an access-policy window that marks the block
@@ -570,7 +607,7 @@ struct L2Pin {
     bp_ctx* c = P->c;
     v.l2_bytes = 0;
     const char* e = std::getenv("BP_L2_PIN");
-    if (!v.A32 || (e && e[0] == '0') || c->l2_max_persist <= 0 || c->l2_max_window <= 0) return;
+    if (!v.A32 || v.xch || (e && e[0] == '0') || c->l2_max_persist <= 0 || c->l2_max_window <= 0) return;
     // offsets 14..26 and the FP64 diagonal (entry 0 of A32 is not read)
     const size_t bytes = 15 * sizeof(float4) * (size_t)v.npad;
     if (bytes > (size_t)c->l2_max_window) return;
@@ -635,7 +672,8 @@ int max_picard_iters(const HostPlan& p) {
 
 // The whole Picard loop as one CUDA graph that stays on the device:
 //   reset -> WHILE (some instance in Picard, passes < cap) {
-//     picard_head, PCG head, reset -> WHILE (some instance in PCG, chunks < cap) {
+//     picard_head, then the resident PCG's one launch, or
+//     PCG head, reset -> WHILE (some instance in PCG, chunks < cap) {
 //       one check chunk of ncheck iterations; count }
 //     picard_tail; count }
 // The loop conditions are set by one-thread kernels (cudaGraphSetConditional)
@@ -662,7 +700,7 @@ bool build_loop_graph(bp_problem* P, bool pdl) {
   bool ok = false;
   try {
     CK(cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle hP, hK;
+    cudaGraphConditionalHandle hP, hK = 0;
     CK(cudaGraphConditionalHandleCreate(&hP, g, 0, 0));
     CK(cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, mode));
     capturing = true;
@@ -680,13 +718,17 @@ bool build_loop_graph(bp_problem* P, bool pdl) {
     cudaGraphNode_t wP;
     CK(cudaGraphAddNode(&wP, g, &start, 1, &wp));
     cudaGraph_t bP = wp.conditional.phGraph_out[0];
-    CK(cudaGraphConditionalHandleCreate(&hK, bP, 0, 0));
+    if (!resident_pcg(P)) CK(cudaGraphConditionalHandleCreate(&hK, bP, 0, 0));
     // Picard body, up to the PCG loop
     CK(cudaStreamBeginCaptureToGraph(s, bP, nullptr, nullptr, 0, mode));
     capturing = true;
     picard_head(P, false);
-    pcg_head(P);
-    launch_loop_cond(hK, v, false, it + 1, cap_chunks, true, s);
+    if (resident_pcg(P)) {
+      CK(launch_pcg_resident(v, variant, s));
+    } else {
+      pcg_head(P);
+      launch_loop_cond(hK, v, false, it + 1, cap_chunks, true, s);
+    }
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t* deps = nullptr;
     size_t nd = 0;
@@ -694,23 +736,26 @@ bool build_loop_graph(bp_problem* P, bool pdl) {
     std::vector<cudaGraphNode_t> last(deps, deps + nd);
     CK(cudaStreamEndCapture(s, &bP));
     capturing = false;
-    cudaGraphNodeParams wk = {};
-    wk.type = cudaGraphNodeTypeConditional;
-    wk.conditional.handle = hK;
-    wk.conditional.type = cudaGraphCondTypeWhile;
-    wk.conditional.size = 1;
-    cudaGraphNode_t wK;
-    CK(cudaGraphAddNode(&wK, bP, last.data(), last.size(), &wk));
-    cudaGraph_t bK = wk.conditional.phGraph_out[0];
-    // PCG body: one check chunk
-    CK(cudaStreamBeginCaptureToGraph(s, bK, nullptr, nullptr, 0, mode));
-    capturing = true;
-    for (int j = 0; j < ncheck; ++j) enqueue_iteration(P, variant, j == ncheck - 1);
-    launch_loop_cond(hK, v, false, it + 1, cap_chunks, false, s);
-    CK(cudaStreamEndCapture(s, &bK));
-    capturing = false;
-    // the rest of the Picard body, after the PCG loop
-    CK(cudaStreamBeginCaptureToGraph(s, bP, &wK, nullptr, 1, mode));
+    if (!resident_pcg(P)) {
+      cudaGraphNodeParams wk = {};
+      wk.type = cudaGraphNodeTypeConditional;
+      wk.conditional.handle = hK;
+      wk.conditional.type = cudaGraphCondTypeWhile;
+      wk.conditional.size = 1;
+      cudaGraphNode_t wK;
+      CK(cudaGraphAddNode(&wK, bP, last.data(), last.size(), &wk));
+      cudaGraph_t bK = wk.conditional.phGraph_out[0];
+      // PCG body: one check chunk
+      CK(cudaStreamBeginCaptureToGraph(s, bK, nullptr, nullptr, 0, mode));
+      capturing = true;
+      for (int j = 0; j < ncheck; ++j) enqueue_iteration(P, variant, j == ncheck - 1);
+      launch_loop_cond(hK, v, false, it + 1, cap_chunks, false, s);
+      CK(cudaStreamEndCapture(s, &bK));
+      capturing = false;
+      last.assign(1, wK);
+    }
+    // the rest of the Picard body, after the PCG
+    CK(cudaStreamBeginCaptureToGraph(s, bP, last.data(), nullptr, last.size(), mode));
     capturing = true;
     picard_tail(P);
     launch_loop_cond(hP, v, true, it, cap_picard, false, s);
@@ -821,6 +866,7 @@ bp_problem* problem_new(bp_ctx* c, Arena* arena, int n, const bp_inputs* in, std
   g_h2d = 0.0;
   P->v = make_view(*P->arena, c->stream, P->plan, true, P->mixed);
   P->h2d_bytes = g_h2d;
+  use_resident_pcg(c, *P->arena, &P->v, P->plan);
   P->x0 = P->arena->get<double2>(c->stream, "x0", P->plan.npad);
   CK(cudaMemsetAsync(P->x0, 0, sizeof(double2) * P->plan.npad, c->stream));
   if (P->plan.diva) {
@@ -1331,6 +1377,7 @@ int bp_pcg(bp_ctx* c, int nx, int ny, int nz, int periodic,
   P.mixed = false;
   P.use_graphs = false;
   P.v = make_view(*P.arena, c->stream, P.plan, false, P.mixed);
+  use_resident_pcg(c, *P.arena, &P.v, P.plan);
   const DevView& v = P.v;
   std::vector<double2> A(2 * 27 * (size_t)P.plan.npad);
   gather_matrix(P.plan, Auu, Auv, Avu, Avv, A.data());

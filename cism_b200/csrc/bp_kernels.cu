@@ -8,6 +8,7 @@
 // scalar update (alpha, beta, convergence) on the device.  The result is
 // bitwise reproducible run to run and needs no host round trip.
 #include <cstdio>
+#include <type_traits>
 
 #include "bp_body.h"
 #include "bp_b200.h"
@@ -92,24 +93,31 @@ __device__ __forceinline__ void tile_finish(const DevView& v, int t, int inst,
   __syncthreads();
 }
 
+// How a scalar update ends an instance's linear solve or its run.  The
+// launched kernels (Shared = true: one thread per instance, on the state in
+// device memory) count it off in the problem's counters at once; the CTAs
+// of a resident PCG each update their own copy of the state, and one of
+// them settles the counters when it writes the state back.
+template <bool Shared>
 __device__ __forceinline__ void pcg_stop(const DevView& v, InstState& S, bool converged) {
   S.pcg_active = 0;
   S.pcg_converged = converged ? 1 : 0;
   S.pcg_iters_last = S.pcg_iter;
   S.pcg_iters_total += S.pcg_iter;
-  atomicSub(&v.cnt->pcg_active, 1);
+  if (Shared) atomicSub(&v.cnt->pcg_active, 1);
 }
 
+template <bool Shared>
 __device__ __forceinline__ void fail(const DevView& v, InstState& S, int code) {
   if (S.status == BP_OK || S.status == BP_WARN_PCG_NOT_CONVERGED) S.status = code;
-  if (S.pcg_active) pcg_stop(v, S, false);
+  if (S.pcg_active) pcg_stop<Shared>(v, S, false);
   if (S.refine_active) {
     S.refine_active = 0;
-    atomicSub(&v.cnt->refine_active, 1);
+    if (Shared) atomicSub(&v.cnt->refine_active, 1);
   }
   if (S.picard_active) {
     S.picard_active = 0;
-    atomicSub(&v.cnt->picard_active, 1);
+    if (Shared) atomicSub(&v.cnt->picard_active, 1);
   }
 }
 
@@ -455,11 +463,11 @@ __global__ void __launch_bounds__(kTile) k_rhs(DevView v) {
       S.bb = s[0];
       S.L2_rhs = sqrt(s[0]);
       if (S.status == BP_ERR_SINGULAR_JAC || S.status == BP_ERR_BAD_BETA) {
-        fail(v, S, S.status);
+        fail<true>(v, S, S.status);
       } else if (!S.nonzero) {
         S.status = BP_ZERO_MATRIX;
         S.zero_x = 1;
-        fail(v, S, BP_ZERO_MATRIX);
+        fail<true>(v, S, BP_ZERO_MATRIX);
       } else if (v.solve2d && !v.diva && v.inst[inst].which_babc == 6) {
         // 2-D solve on a no-slip bed: the 2-D velocity is zero and nothing is solved
         // (glissade_velo_higher.F90:3227-3240)
@@ -467,7 +475,7 @@ __global__ void __launch_bounds__(kTile) k_rhs(DevView v) {
         S.L2_norm = 0.0;
         S.L2_rel = 0.0;
         S.pcg_iter = 0;
-        pcg_stop(v, S, true);
+        pcg_stop<true>(v, S, true);
         if (S.refine_active) {
           S.refine_active = 0;
           atomicSub(&v.cnt->refine_active, 1);
@@ -569,6 +577,41 @@ __device__ __forceinline__ void refine_request(const InstParams& ip, InstState& 
     S.need_true = 1;
 }
 
+// After a residual r = b - A x with (r,z), (r,r) = s[0], s[1].
+template <int MODE, bool Shared>
+__device__ __forceinline__ void resid_fin(const DevView& v, const InstParams& ip, InstState& S, const double* s) {
+  const double rt = sqrt(s[1]);
+  if (MODE == MV_INIT) {
+    S.L2_norm = rt;
+    S.L2_rel = S.L2_rhs > 0.0 ? S.L2_norm / S.L2_rhs : 0.0;
+    S.r_true = rt;
+    S.last_true_iter = S.pcg_iter;
+  } else {
+    S.err = rt / S.L2_rhs;
+    S.refine_steps_total += 1;
+    if (MODE == MV_REFINE) {
+      S.need_true = 0;
+      S.last_true_iter = S.pcg_iter;
+    }
+    if (S.err < ip.pcg_tol) { pcg_stop<Shared>(v, S, true); return; }
+    if (S.pcg_iter >= ip.pcg_maxiters) { pcg_stop<Shared>(v, S, false); return; }
+    if (MODE == MV_REFINE) {
+      // a cycle that did not halve the residual: the FP32 operator is
+      // too coarse for this system, finish with the FP64 matrix
+      if (rt > 0.5 * S.r_true) S.krylov_fp64 = 1;
+      S.r_true = rt;
+    }
+  }
+  if (ip.variant != 3) {  // standard PCG: eta1 of the next iteration
+    if (is_nan(s[0])) { fail<Shared>(v, S, BP_ERR_NAN); return; }
+    S.beta = MODE == MV_REFINE ? 0.0 : s[0] / S.rz;  // refinement restarts: d = z
+    S.rz = s[0];
+    if (MODE == MV_CHECK) S.pcg_iter += 1;
+  } else if (MODE == MV_REFINE) {
+    S.restart = 1;
+  }
+}
+
 // r = b - A x with the FP64 matrix; z = D^-1 r stored; (r,z) and (r,r).
 // MV_INIT starts a linear solve (also compute_residual_vector_3d's norms);
 // MV_CHECK is the every-ncheck true residual (pcg:478-536, 1542-1597);
@@ -601,38 +644,7 @@ __global__ void __launch_bounds__(kTile, MINB) k_resid(DevView v) {
       part[1] = r.x * r.x + r.y * r.y;
     }
     tile_finish<2, false>(v, t, R.inst, part, [&](int inst, const double* s) {
-      InstState& S = v.st[inst];
-      const InstParams& ip = v.inst[inst];
-      const double rt = sqrt(s[1]);
-      if (MODE == MV_INIT) {
-        S.L2_norm = rt;
-        S.L2_rel = S.L2_rhs > 0.0 ? S.L2_norm / S.L2_rhs : 0.0;
-        S.r_true = rt;
-        S.last_true_iter = S.pcg_iter;
-      } else {
-        S.err = rt / S.L2_rhs;
-        S.refine_steps_total += 1;
-        if (MODE == MV_REFINE) {
-          S.need_true = 0;
-          S.last_true_iter = S.pcg_iter;
-        }
-        if (S.err < ip.pcg_tol) { pcg_stop(v, S, true); return; }
-        if (S.pcg_iter >= ip.pcg_maxiters) { pcg_stop(v, S, false); return; }
-        if (MODE == MV_REFINE) {
-          // a cycle that did not halve the residual: the FP32 operator is
-          // too coarse for this system, finish with the FP64 matrix
-          if (rt > 0.5 * S.r_true) S.krylov_fp64 = 1;
-          S.r_true = rt;
-        }
-      }
-      if (ip.variant != 3) {  // standard PCG: eta1 of the next iteration
-        if (is_nan(s[0])) { fail(v, S, BP_ERR_NAN); return; }
-        S.beta = MODE == MV_REFINE ? 0.0 : s[0] / S.rz;  // refinement restarts: d = z
-        S.rz = s[0];
-        if (MODE == MV_CHECK) S.pcg_iter += 1;
-      } else if (MODE == MV_REFINE) {
-        S.restart = 1;
-      }
+      resid_fin<MODE, true>(v, v.inst[inst], v.st[inst], s);
     });
   }
 }
@@ -669,33 +681,42 @@ __device__ __forceinline__ void count_tile(const DevView& v, const InstState& S,
 }
 
 // alpha = eta1 / (d, q) of the standard PCG (pcg:426-463).
-__device__ __forceinline__ void std_mv_fin(const DevView& v, int inst, const double* s) {
-  if (v.dry) return;
-  InstState& S = v.st[inst];
+template <bool Shared>
+__device__ __forceinline__ void std_mv_fin(const DevView& v, InstState& S, const double* s) {
   const double alpha = S.rz / s[0];
-  if (is_nan(alpha)) { fail(v, S, BP_ERR_NAN); return; }
+  if (is_nan(alpha)) { fail<Shared>(v, S, BP_ERR_NAN); return; }
   S.alpha = alpha;
+}
+
+// beta and eta1 of the standard PCG's next iteration from (r,z), (r,r)
+// (pcg:347-407).
+template <bool Shared>
+__device__ __forceinline__ void std_update_fin(const DevView& v, const InstParams& ip, InstState& S,
+                                               const double* s) {
+  if (S.pcg_iter >= ip.pcg_maxiters) { pcg_stop<Shared>(v, S, false); return; }
+  if (is_nan(s[0])) { fail<Shared>(v, S, BP_ERR_NAN); return; }
+  S.beta = s[0] / S.rz;
+  S.rz = s[0];
+  if (v.A32) refine_request(ip, S, s[1]);
+  S.pcg_iter += 1;
 }
 
 // The Chronopoulos-Gear scalar recurrences from (r,z), (Az,z), (r,r)
 // (pcg:1461-1512); FIRST: the first pass (pcg:1304-1405).
-template <bool FIRST>
-__device__ __forceinline__ void cg_mv_fin(const DevView& v, int inst, const double* s) {
-  if (v.dry) return;
-  InstState& S = v.st[inst];
+template <bool FIRST, bool Shared>
+__device__ __forceinline__ void cg_mv_fin(const DevView& v, const InstParams& ip, InstState& S, const double* s) {
   if (FIRST) {
     S.rz_old = s[0];
     S.sigma = s[1];
     const double alpha = s[0] / s[1];
-    if (is_nan(alpha)) { fail(v, S, BP_ERR_NAN); return; }
+    if (is_nan(alpha)) { fail<Shared>(v, S, BP_ERR_NAN); return; }
     S.alpha = alpha;
     return;
   }
-  const InstParams& ip = v.inst[inst];
   S.pcg_iter += 1;
   if (S.pcg_iter > ip.pcg_maxiters) {
     S.pcg_iter = ip.pcg_maxiters;
-    pcg_stop(v, S, false);
+    pcg_stop<Shared>(v, S, false);
     return;
   }
   const double rho = s[0], delta = s[1];
@@ -712,7 +733,7 @@ __device__ __forceinline__ void cg_mv_fin(const DevView& v, int inst, const doub
   S.rz_old = rho;
   S.beta = beta;
   S.sigma = sigma;
-  if (is_nan(alpha)) { fail(v, S, BP_ERR_NAN); return; }
+  if (is_nan(alpha)) { fail<Shared>(v, S, BP_ERR_NAN); return; }
   S.alpha = alpha;
   if (v.A32) refine_request(ip, S, s[2]);
 }
@@ -738,7 +759,9 @@ __global__ void __launch_bounds__(kTile, MINB) k_std_mv(DevView v) {
       v.q[n] = y;
       part[0] = d.x * y.x + d.y * y.y;
     }
-    tile_finish<1, false>(v, t, R.inst, part, [&](int inst, const double* s) { std_mv_fin(v, inst, s); });
+    tile_finish<1, false>(v, t, R.inst, part, [&](int inst, const double* s) {
+      if (!v.dry) std_mv_fin<true>(v, v.st[inst], s);
+    });
   }
 }
 
@@ -781,14 +804,7 @@ __global__ void __launch_bounds__(kTile) k_std_update(DevView v) {
     }
     if (!CHECK) {
       tile_finish<2, false>(v, t, R.inst, part, [&](int inst, const double* s) {
-        InstState& S2 = v.st[inst];
-        const InstParams& ip = v.inst[inst];
-        if (S2.pcg_iter >= ip.pcg_maxiters) { pcg_stop(v, S2, false); return; }
-        if (is_nan(s[0])) { fail(v, S2, BP_ERR_NAN); return; }
-        S2.beta = s[0] / S2.rz;
-        S2.rz = s[0];
-        if (v.A32) refine_request(ip, S2, s[1]);
-        S2.pcg_iter += 1;
+        std_update_fin<true>(v, v.inst[inst], v.st[inst], s);
       });
     }
   }
@@ -843,7 +859,9 @@ __global__ void __launch_bounds__(kTile, MINB) k_cg_mv(DevView v) {
       part[1] = y.x * z.x + y.y * z.y;
       part[2] = r.x * r.x + r.y * r.y;
     }
-    tile_finish<3, false>(v, t, R.inst, part, [&](int inst, const double* s) { cg_mv_fin<FIRST>(v, inst, s); });
+    tile_finish<3, false>(v, t, R.inst, part, [&](int inst, const double* s) {
+      if (!v.dry) cg_mv_fin<FIRST, true>(v, v.inst[inst], v.st[inst], s);
+    });
   }
 }
 
@@ -909,6 +927,572 @@ __global__ void __launch_bounds__(kTile) k_cg_update(DevView v) {
       const double2 z = precondition(v, R, mine, n, r);
       if (mine) v.z[n] = z;
     }
+  }
+}
+
+// ---------------------------------------------------------------------
+// Resident PCG: the whole linear solve of a problem whose tiles all fit on
+// the GPU at once, in one cooperative launch of one CTA per tile.
+//
+// At these sizes (a few hundred tiles and fewer) a launched PCG step does
+// microseconds of work between launches that cost as much again, so the
+// solve is bound by launches and by the drain and refill at each of them.
+// Here a CTA keeps its tile for the whole solve: x, r, d, q in registers,
+// the matrix rows, the SIA factors and the source vector of the tile and of
+// its halo columns in shared memory.  Two things pass between CTAs, both as
+// 16-byte (value, epoch) slots, each written by one relaxed 128-bit store
+// and read by polling 128-bit loads, so that a value and the news of its
+// arrival are one trip through L2 with no fence and no atomic:
+//  * the global sums: every tile publishes its block sums, every CTA reads
+//    those of its instance, adds them in the order of tile_finish and runs
+//    the scalar recurrences on its own copy of the state;
+//  * the halo: every tile publishes its nodes of the new z, and for a
+//    residual of x; the standard PCG's halo direction z + beta d is formed
+//    by each reader as its owner forms it.
+// Instances of a batch never wait for one another.  All arithmetic is the
+// launched kernels', in their order, so the results are the same bitwise.
+//
+// Slots are rewritten only after every reader is past them.  Sums are
+// double-buffered by the epoch's parity: a tile publishes sum e + 2 after it
+// has every tile's e + 1, each published after its CTA has read all of sum
+// e.  Nodes: a tile publishes the next z (or x) after a sum that every CTA
+// contributed to after its product with the last one.  Every wait is bounded:
+// past the limit the CTA leaves, and the instance ends with BP_ERR_BUDGET.
+//
+// What bounds it: the trips through L2.  One slot takes about 500 cycles to
+// another SM of the same die and 900 to the other die, an iteration makes
+// two trips in a row (three with a sum between), and each is followed by
+// two shuffle trees; the product from shared memory (864 B a node) is 1,900
+// of the 11,000 cycles of an iteration of the 34-tile dome.
+// Measured, launched kernels -> this one: 31 x 31 x 10 dome, FP64, standard
+// PCG, 34 tiles: 21 -> 6.1 us an iteration; 128 x 128 2-D marine sheet,
+// Chronopoulos-Gear, 39 tiles: 18 -> 5.7 us; 48 x 48 x 11 slab, 144 tiles:
+// 23 -> 7.1 us.  The limit (every tile resident: 148 tiles of FP64 rows, 296
+// of FP32 ones) is where shared memory ends.
+// ---------------------------------------------------------------------
+constexpr int kXchSpins = 1 << 22;  // a second or more of polling
+
+__device__ __forceinline__ void xch_put(ulonglong2* p, double val, unsigned long long tag) {
+  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
+               "l"(__double_as_longlong(val)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ void xch_ld(const ulonglong2* p, double* val, unsigned long long* tag) {
+  unsigned long long lo;
+  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(lo), "=l"(*tag)
+               : "l"(p)
+               : "memory");
+  *val = __longlong_as_double((long long)lo);
+}
+// NS slots from p on with epoch e into w, loaded together; false past the limit.
+template <int NS>
+__device__ __forceinline__ bool xch_poll(const ulonglong2* p, unsigned long long e, double* w) {
+  for (int spin = 0; spin < kXchSpins; ++spin) {
+    unsigned long long tag[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) xch_ld(p + i, &w[i], &tag[i]);
+    bool there = true;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) there = there && tag[i] == e;
+    if (there) return true;
+  }
+  return false;
+}
+
+// a.x b.x + a.y b.y in one fixed fused form, the one the compiler gives the
+// launched kernels' sums (left to it, a product that appears twice in this
+// kernel would be formed once and rounded).
+__device__ __forceinline__ double dot2(double2 a, double2 b) {
+  return __fma_rn(a.x, b.x, __dmul_rn(a.y, b.y));
+}
+
+__device__ __forceinline__ int xch_copies(const DevView& v) { return v.ntiles > 64 ? kXchSumCopies : 1; }
+
+// The sum of NV values of every thread of the instance's CTAs, in
+// tile_finish's order, in two steps so that other waiting can go between
+// them.  xch_put_sum publishes the tile's block sums; a tile has at most
+// eight warps, so the second stage of block_reduce's tree over 32 lanes is
+// its three last steps.  Past 64 tiles each sum goes to kXchSumCopies copies,
+// each read by every kXchSumCopies-th CTA only: all CTAs polling one line queue
+// up at its L2 slice (an all-to-all round of bare slots takes 1,430 cycles
+// among 34 CTAs and 1,890 with eight copies, but 3,030 and 2,460 among 144).
+// xch_get_sum waits for all tiles' sums and returns
+// their total in val on every thread.  red: two arrays of 8 x 4 doubles.
+template <int NV>
+__device__ __forceinline__ void xch_put_sum(const DevView& v, int t, unsigned long long e, const double* val,
+                                            double* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    double x = val[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane == 0) red[warp * 4 + i] = x;
+  }
+  __syncthreads();
+  if (warp == 0) {  // the lanes w * 4 + i sum value i over the warps w
+    const int w = lane >> 2, i = lane & 3;
+    double x = (w < nw && i < NV) ? red[w * 4 + i] : 0.0;
+    x += __shfl_xor_sync(0xffffffffu, x, 16);
+    x += __shfl_xor_sync(0xffffffffu, x, 8);
+    x += __shfl_xor_sync(0xffffffffu, x, 4);
+    x = __shfl_sync(0xffffffffu, x, lane % NV);
+    const int copy = lane / NV;
+    if (copy < xch_copies(v))
+      xch_put(v.xch + ((size_t)((e & 1) * kXchSumCopies + copy) * v.ntiles + t) * 4 + lane % NV, x, e);
+  }
+}
+template <int NV>
+__device__ __forceinline__ bool xch_get_sum(const DevView& v, const InstParams& ip, int t, unsigned long long e,
+                                            double* val, double* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const ulonglong2* slots =
+      v.xch + ((size_t)((e & 1) * kXchSumCopies + t % xch_copies(v)) * v.ntiles + ip.tile_begin) * 4;
+  double s[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) s[i] = 0.0;
+  bool ok = true;
+  const int ntl = ip.tile_end - ip.tile_begin;
+  for (int tt = threadIdx.x; tt < ntl && ok; tt += blockDim.x) {
+    double w[NV];
+    ok = xch_poll<NV>(slots + (size_t)tt * 4, e, w);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) s[i] += w[i];
+  }
+  double* red2 = red + 32;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    double x = s[i];
+    if (warp * 32 < ntl) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    }
+    if (lane == 0) red2[warp * 4 + i] = x;
+  }
+  ok = __syncthreads_and(ok);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    double w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = j < nw ? red2[j * 4 + i] : 0.0;
+    val[i] = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+  }
+  return ok;
+}
+template <int NV>
+__device__ __forceinline__ bool xch_sum(const DevView& v, const InstParams& ip, int t, unsigned long long e,
+                                        double* val, double* red) {
+  xch_put_sum<NV>(v, t, e, val, red);
+  return xch_get_sum<NV>(v, ip, t, e, val, red);
+}
+
+// Shared memory of a tile: the matrix rows -- offset m (3 x 9; nz = 1: the 9
+// of the level) of node i at [m * slots + i], (uu, uv) and (vu, vv) in FP64,
+// or packed FP32 with the FP64 diagonal block after them --; the source
+// vector, level k of column slot c at [(k + 1) * ls + c], with a level of
+// zeros above and below and a last column of zeros that absent neighbours
+// read (twice for the standard PCG: its residuals read x while the
+// directions stay); the SIA sweeps' s, a, beta, gamma; and each node's
+// nine neighbour columns as slots, [q * slots + i].
+struct ResidentShape {
+  int slots, offsets, ls;
+  size_t matrix, source, sia, bytes;
+};
+__host__ __device__ inline ResidentShape resident_shape(const DevView& v, bool f32, int variant) {
+  ResidentShape h;
+  h.slots = v.W * v.nz;
+  h.offsets = v.nz == 1 ? 9 : 27;
+  h.ls = v.W + v.halo_max + 1;
+  h.matrix = (size_t)h.slots * (f32 ? 16 * h.offsets + 32 : 32 * h.offsets);
+  h.source = 16 * (size_t)(v.nz + 2) * h.ls;
+  h.sia = v.sia_f ? sizeof(double) * 8 * h.slots : 0;
+  h.bytes = h.matrix + h.source * (variant == 3 ? 1 : 2) + h.sia + sizeof(uint16_t) * 9 * h.slots;
+  return h;
+}
+
+// PER_SM: CTAs the kernel is built to run on an SM: 1, or 2 for FP32 tiles of
+// at most 192 threads.
+template <int STORE, int VARIANT, int PER_SM>
+__global__ void __launch_bounds__(PER_SM == 2 ? 192 : kTile, PER_SM) k_pcg_resident(DevView v) {
+  extern __shared__ __align__(16) unsigned char rs_sm[];
+  __shared__ InstState S;
+  __shared__ double red[2 * 32];
+  constexpr bool MIXED = STORE == ST_SYM32;
+  const int t = blockIdx.x, i = threadIdx.x;
+  const TileRange R = tile_range(v, t);
+  InstState& G = v.st[R.inst];
+  if (!G.pcg_active) return;  // the same for all CTAs of the instance: none writes G before all have begun
+  const InstParams& ip = v.inst[R.inst];
+  unsigned long long es = v.xch_epoch[R.inst], en = es;  // epochs of the sums and of the nodes
+  const ResidentShape H = resident_shape(v, MIXED, VARIANT);
+  const int nz = v.nz, W = v.W, slots = H.slots, ls = H.ls;
+  const int ncheck = ip.ncheck > 0 ? ip.ncheck : 1;
+  const size_t np = (size_t)v.npad;
+  const bool mine = tile_mine(v, R, i);
+  const size_t n = (size_t)R.n0 + i;
+  const int col = mine ? tile_col(v, R, i) : 0, k = mine ? tile_k(v, i) : 0;
+  const int lev = (k + 1) * ls, me = lev + (i & (W - 1));  // this node in the source vector
+  double2* M0 = reinterpret_cast<double2*>(rs_sm);
+  double2* M1 = M0 + (size_t)slots * H.offsets;
+  float4* MF = reinterpret_cast<float4*>(rs_sm);
+  double2* DG = reinterpret_cast<double2*>(MF + (size_t)slots * H.offsets);
+  double2* src = reinterpret_cast<double2*>(rs_sm + H.matrix);
+  double2* srcx = VARIANT == 3 ? src : reinterpret_cast<double2*>(rs_sm + H.matrix + H.source);
+  double* sia = reinterpret_cast<double*>(rs_sm + H.matrix + H.source * (VARIANT == 3 ? 1 : 2));
+  uint16_t* nbr = reinterpret_cast<uint16_t*>(reinterpret_cast<unsigned char*>(sia) + H.sia) + i;
+  const int js = 2 * ((i & (W - 1)) * nz + k), so = 2 * slots;
+  const bool column_pc = ip.precond == 2;
+  const int h0 = v.halo_begin[t], nh = v.halo_begin[t + 1] - h0;
+  const double2 zero = make_double2(0.0, 0.0);
+  double2 x = zero, r = zero, z = zero, d = zero, q = zero, di = zero;
+
+  if (i == 0) S = G;
+  for (int o = i; o < (nz + 2) * ls; o += blockDim.x) {
+    src[o] = zero;
+    srcx[o] = zero;
+  }
+  __syncthreads();
+  if (mine) {
+    for (int c = 0; c < 9; ++c) {
+      const int lc = v.col_loc[c * v.ncols + col], cq = v.col_nbn[c * v.ncols + col];
+      nbr[c * slots] = (uint16_t)(lc >= 0 ? lc : ls - 1);
+      for (int kA = nz == 1 ? 0 : -1; kA <= (nz == 1 ? 0 : 1); ++kA) {
+        const int m = (kA + 1) * 9 + c, o = (nz == 1 ? c : m) * slots + i, kn = k + kA;
+        const bool there = lc >= 0 && kn >= 0 && kn < nz;
+        const size_t p = there ? (size_t)cq + ((size_t)kn << v.lsh) : n;
+        if (STORE == ST_SYM32) {
+          float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (there && m > 13) a = v.A32[(size_t)(m - 13) * np + n];
+          if (there && m < 13) {
+            const float4 b = v.A32[(size_t)(13 - m) * np + p];
+            a = make_float4(b.x, b.z, b.y, b.w);
+          }
+          MF[o] = a;
+        } else {
+          double2 a0 = zero, a1 = zero;
+          if (there && STORE == ST_FULL) {
+            a0 = v.A[(size_t)m * np + n];
+            a1 = v.A[(size_t)(27 + m) * np + n];
+          } else if (there && m >= 13) {
+            a0 = v.A[(size_t)(m - 13) * np + n];
+            a1 = v.A[(size_t)(m + 1) * np + n];
+          } else if (there) {
+            const double2 b0 = v.A[(size_t)(13 - m) * np + p], b1 = v.A[(size_t)(27 - m) * np + p];
+            a0 = make_double2(b0.x, b1.x);
+            a1 = make_double2(b0.y, b1.y);
+          }
+          M0[o] = a0;
+          M1[o] = a1;
+        }
+      }
+    }
+    if (STORE == ST_SYM32) {
+      DG[i] = v.A32d[n];
+      DG[slots + i] = v.A32d[np + n];
+    }
+    x = v.x[n];
+    r = v.r[n];
+    z = v.z[n];
+    src[me] = z;
+    if (column_pc) {
+#pragma unroll
+      for (int f = 0; f < 3; ++f) {
+        const double2 c = v.sia_f[(size_t)f * np + n];
+        sia[(f + 1) * so + js] = c.x;
+        sia[(f + 1) * so + js + 1] = c.y;
+      }
+    } else {
+      di = v.Dinv[n];
+    }
+  }
+  // halo node h (slot c of level kk): its node, its place in the source vector
+  auto halo_at = [&](int h, size_t* node) {
+    const int kk = h / nh, c = h - kk * nh;
+    *node = (size_t)v.halo_node[h0 + c] + ((size_t)kk << v.lsh);
+    return (kk + 1) * ls + W + c;
+  };
+  for (int h = i; h < nh * nz; h += blockDim.x) {  // MV_INIT's z of the halo
+    size_t p;
+    const int o = halo_at(h, &p);
+    src[o] = v.z[p];
+  }
+  // a thread's first nodes of the halo, which is two to three times the CTA
+  // in the tiles of a filled grid, stay known to it
+  constexpr int B = 3;
+  const ulonglong2* hp[B];
+  int ho[B];
+  unsigned hmine = 0;
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    const int h = i + j * blockDim.x;
+    size_t p = 0;
+    ho[j] = h < nh * nz ? halo_at(h, &p) : 0;
+    hp[j] = v.xch_node + 2 * p;
+    if (h < nh * nz) hmine |= 1u << j;
+  }
+  __syncthreads();
+
+  // this node's value to the tiles that read it; the halo's new values, each
+  // through f(value, source slot), once per halo node
+  auto publish = [&](double2 a, unsigned long long e, size_t buf) {
+    xch_put(v.xch_node + 2 * n + buf, a.x, e);
+    xch_put(v.xch_node + 2 * n + buf + 1, a.y, e);
+  };
+  constexpr size_t ZBUF = 0;
+  const size_t XBUF = 2 * np;
+  double2 ha[B];
+  auto halo_wait = [&](unsigned long long e, size_t buf) -> bool {  // the thread's first nodes
+    unsigned left = hmine;
+    for (int spin = 0; spin < kXchSpins && left; ++spin) {  // those still missing, loaded together
+      unsigned long long tx[B], ty[B];
+#pragma unroll
+      for (int j = 0; j < B; ++j)
+        if (left >> j & 1) {
+          xch_ld(hp[j] + buf, &ha[j].x, &tx[j]);
+          xch_ld(hp[j] + buf + 1, &ha[j].y, &ty[j]);
+        }
+#pragma unroll
+      for (int j = 0; j < B; ++j)
+        if ((left >> j & 1) && tx[j] == e && ty[j] == e) left &= ~(1u << j);
+    }
+    return left == 0;
+  };
+  auto halo_take = [&](unsigned long long e, size_t buf, auto f) -> bool {  // all of them, after halo_wait
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+      if (hmine >> j & 1) f(ha[j], ho[j]);
+    for (int h = i + B * blockDim.x; h < nh * nz && ok; h += blockDim.x) {  // the rest of a ragged tile's halo
+      size_t p;
+      const int o = halo_at(h, &p);
+      double w[2];
+      ok = xch_poll<2>(v.xch_node + 2 * p + buf, e, w);
+      f(make_double2(w[0], w[1]), o);
+    }
+    return ok;
+  };
+  auto precondition_r = [&] {  // z = M^-1 r
+    if (column_pc) {
+      if (mine) {
+        sia[js] = r.x;
+        sia[js + 1] = r.y;
+      }
+      __syncthreads();
+      if (i < 2 * R.ncols) {
+        const int o = 2 * (i >> 1) * nz + (i & 1);
+        sia_sweeps(
+            nz,
+            [&](int kk) { return SiaFac{sia[so + o + 2 * kk], sia[2 * so + o + 2 * kk], sia[3 * so + o + 2 * kk]}; },
+            &sia[o], 2);
+      }
+      __syncthreads();
+      if (mine) z = make_double2(sia[js], sia[js + 1]);
+    } else if (mine) {
+      z = make_double2(r.x * di.x, r.y * di.y);
+    }
+  };
+  // this node's row times the source vector s, from the tile's rows in
+  // shared memory, in matvec_row's order (FULL: levels outer) or
+  // matvec_row_sym's (neighbour columns outer)
+  auto row = [&](const double2* s) -> double2 {
+    double yu = 0.0, yv = 0.0;
+    if (!mine) return zero;
+    auto term = [&](int c, int kA) {
+      const int m = ((nz == 1 ? 0 : (kA + 1) * 9) + c) * slots + i;
+      const double2 sv = s[lev + kA * ls + nbr[c * slots]];
+      if (MIXED && !(kA == 0 && c == 4)) {
+        const float4 a = MF[m];
+        yu += dot2(make_double2(a.x, a.y), sv);
+        yv += dot2(make_double2(a.z, a.w), sv);
+      } else {
+        yu += dot2(MIXED ? DG[i] : M0[m], sv);
+        yv += dot2(MIXED ? DG[slots + i] : M1[m], sv);
+      }
+    };
+    if (nz == 1) {
+#pragma unroll
+      for (int c = 0; c < 9; ++c) term(c, 0);
+    } else if (STORE == ST_FULL) {
+#pragma unroll
+      for (int kA = -1; kA <= 1; ++kA)
+#pragma unroll
+        for (int c = 0; c < 9; ++c) term(c, kA);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 9; ++c)
+#pragma unroll
+        for (int kA = -1; kA <= 1; ++kA) term(c, kA);
+    }
+    return make_double2(yu, yv);
+  };
+  // the same with the FP64 matrix of a mixed solve, from device memory
+  auto row64 = [&](const double2* s) -> double2 {
+    double yu = 0.0, yv = 0.0;
+    if (!mine) return zero;
+#pragma unroll 3
+    for (int c = 0; c < 9; ++c) {
+      const int lc = v.col_loc[c * v.ncols + col], cq = v.col_nbn[c * v.ncols + col];
+#pragma unroll
+      for (int kA = -1; kA <= 1; ++kA) {
+        const int m = (kA + 1) * 9 + c, kn = k + kA;
+        const bool there = lc >= 0 && kn >= 0 && kn < nz;
+        const size_t p = there ? (size_t)cq + ((size_t)kn << v.lsh) : n;
+        const double2 sv = s[lev + kA * ls + (lc >= 0 ? lc : ls - 1)];
+        if (m >= 13) {
+          yu += dot2(v.A[(size_t)(m - 13) * np + n], sv);
+          yv += dot2(v.A[(size_t)(m + 1) * np + n], sv);
+        } else {
+          const double2 b0 = v.A[(size_t)(13 - m) * np + p], b1 = v.A[(size_t)(27 - m) * np + p];
+          yu += dot2(make_double2(b0.x, b1.x), sv);
+          yv += dot2(make_double2(b0.y, b1.y), sv);
+        }
+      }
+    }
+    return make_double2(yu, yv);
+  };
+  double val[3];
+  bool ok = true;
+  // r = b - A x, z and their sums with the scalar update
+  auto residual = [&](auto mode) {
+    constexpr int MODE = decltype(mode)::value;
+    ++en;
+    if (mine) {
+      publish(x, en, XBUF);
+      srcx[me] = x;
+    }
+    ok = __syncthreads_and(halo_wait(en, XBUF) && halo_take(en, XBUF, [&](double2 a, int o) { srcx[o] = a; }));
+    if (!ok) return;
+    const double2 y = MIXED ? row64(srcx) : row(srcx);
+    if (mine) {
+      const double2 b = v.b[n];
+      r = make_double2(b.x - y.x, b.y - y.y);
+    }
+    precondition_r();
+    ++en;
+    if (mine) publish(z, en, ZBUF);
+    val[0] = mine ? dot2(r, z) : 0.0;
+    val[1] = mine ? dot2(r, r) : 0.0;
+    xch_put_sum<2>(v, t, ++es, val, red);
+    const bool zs = halo_wait(en, ZBUF);  // z arrives with the sums
+    ok = xch_get_sum<2>(v, ip, t, es, val, red);
+    ok = __syncthreads_and(ok && zs);
+    if (i == 0 && ok) resid_fin<MODE, false>(v, ip, S, val);
+    __syncthreads();
+  };
+  using Check = std::integral_constant<int, MV_CHECK>;
+  using Refine = std::integral_constant<int, MV_REFINE>;
+
+  if (VARIANT == 2) {
+    for (int it = 1; ok; ++it) {
+      const bool check = it % ncheck == 0;
+      // d = z + beta d (k_std_dir) here and in the halo
+      const double beta = S.beta;
+      if (it > 1) {
+        if (mine) {
+          d = make_double2(z.x + beta * d.x, z.y + beta * d.y);
+          src[me] = d;
+        }
+        ok = __syncthreads_and(halo_take(en, ZBUF, [&](double2 a, int o) {
+          const double2 b = src[o];
+          src[o] = make_double2(a.x + beta * b.x, a.y + beta * b.y);
+        }));
+        if (!ok) break;
+      } else {
+        d = z;
+      }
+      const double2 y = MIXED && S.krylov_fp64 ? row64(src) : row(src);
+      val[0] = mine ? dot2(d, y) : 0.0;
+      ok = xch_sum<1>(v, ip, t, ++es, val, red);
+      if (i == 0 && ok) std_mv_fin<false>(v, S, val);
+      __syncthreads();
+      if (!ok || !S.pcg_active) break;
+      const double alpha = S.alpha;
+      if (mine) {
+        x.x = x.x + alpha * d.x;
+        x.y = x.y + alpha * d.y;
+      }
+      if (check && !MIXED) {
+        residual(Check{});
+      } else {
+        if (mine) {
+          r.x = r.x - alpha * y.x;
+          r.y = r.y - alpha * y.y;
+        }
+        precondition_r();
+        ++en;
+        if (mine) publish(z, en, ZBUF);
+        val[0] = mine ? dot2(r, z) : 0.0;
+        val[1] = mine ? dot2(r, r) : 0.0;
+        xch_put_sum<2>(v, t, ++es, val, red);
+        const bool zs = halo_wait(en, ZBUF);  // the next z arrives with the sums
+        ok = xch_get_sum<2>(v, ip, t, es, val, red);
+        ok = __syncthreads_and(ok && zs);
+        if (i == 0 && ok) std_update_fin<false>(v, ip, S, val);
+        __syncthreads();
+        if (ok && MIXED && check && S.pcg_active && S.need_true) residual(Refine{});
+      }
+      if (!S.pcg_active) break;
+    }
+  } else {
+    bool z_waited = false;
+    for (int it = 1; ok; ++it) {
+      const bool check = it > 1 && it % ncheck == 0;
+      const bool waited = z_waited;  // a residual has fetched the halo of its z
+      if (it > 1) {
+        if (mine) src[me] = z;
+        ok = __syncthreads_and((waited || halo_wait(en, ZBUF)) &&
+                               halo_take(en, ZBUF, [&](double2 a, int o) { src[o] = a; }));
+        if (!ok) break;
+      }
+      const double2 y = MIXED && S.krylov_fp64 ? row64(src) : row(src);
+      val[0] = mine ? dot2(r, z) : 0.0;
+      val[1] = mine ? dot2(y, z) : 0.0;
+      val[2] = mine ? dot2(r, r) : 0.0;
+      ok = xch_sum<3>(v, ip, t, ++es, val, red);
+      if (i == 0 && ok) {
+        if (it == 1) cg_mv_fin<true, false>(v, ip, S, val);
+        else cg_mv_fin<false, false>(v, ip, S, val);
+      }
+      __syncthreads();
+      if (!ok || !S.pcg_active) break;
+      const double alpha = S.alpha, beta = S.beta;
+      const bool keep_r = it == 1 || (!(check && !MIXED) && !S.need_true);
+      if (mine) {
+        if (it == 1) {
+          d = z;
+          q = y;
+        } else {
+          d.x = z.x + beta * d.x; d.y = z.y + beta * d.y;
+          q.x = y.x + beta * q.x; q.y = y.y + beta * q.y;
+        }
+        x.x = x.x + alpha * d.x; x.y = x.y + alpha * d.y;
+        if (keep_r) {
+          r.x = r.x - alpha * q.x;
+          r.y = r.y - alpha * q.y;
+        }
+      }
+      z_waited = !keep_r;
+      if (keep_r) {
+        precondition_r();
+        ++en;
+        if (mine) publish(z, en, ZBUF);
+      } else if (MIXED) {
+        residual(Refine{});
+      } else {
+        residual(Check{});
+      }
+      if (!S.pcg_active) break;
+    }
+  }
+  if (mine) v.x[n] = x;
+  if (t == ip.tile_begin && i == 0) {
+    if (!ok) fail<false>(v, S, BP_ERR_BUDGET);  // a wait ran out
+    if (!S.pcg_active) atomicSub(&v.cnt->pcg_active, 1);
+    if (G.refine_active && !S.refine_active) atomicSub(&v.cnt->refine_active, 1);
+    if (G.picard_active && !S.picard_active) atomicSub(&v.cnt->picard_active, 1);
+    G = S;
+    v.xch_epoch[R.inst] = (es > en ? es : en) + (ok ? 0 : 4);  // after a failed wait other CTAs may be ahead
   }
 }
 
@@ -1244,6 +1828,42 @@ void launch_cg_first_update(const DevView& v, cudaStream_t s) {
 }
 void launch_cg_update(bool check, const DevView& v, cudaStream_t s) {
   launch_pcg(check ? k_cg_update<true> : k_cg_update<false>, tile_grid(v), s, v);
+}
+template <int STORE, int PER_SM>
+static TileKernel resident_kernel_st(int variant) {
+  return variant == 3 ? k_pcg_resident<STORE, 3, PER_SM> : k_pcg_resident<STORE, 2, PER_SM>;
+}
+static TileKernel resident_kernel(const DevView& v, int variant, size_t* smem) {
+  *smem = resident_shape(v, v.sym && v.A32, variant).bytes;
+  if (!v.sym) return resident_kernel_st<ST_FULL, 1>(variant);
+  if (!v.A32) return resident_kernel_st<ST_SYM, 1>(variant);
+  return v.tile_threads <= 192 ? resident_kernel_st<ST_SYM32, 2>(variant) : resident_kernel_st<ST_SYM32, 1>(variant);
+}
+int resident_ctas(const DevView& v, int variant, int num_sms) {
+  size_t smem = 0;
+  TileKernel k = resident_kernel(v, variant, &smem);
+  int n = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, v.tile_threads, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n * num_sms;
+}
+cudaError_t launch_pcg_resident(const DevView& v, int variant, cudaStream_t s) {
+  size_t smem = 0;
+  TileKernel k = resident_kernel(v, variant, &smem);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(v.ntiles);
+  cfg.blockDim = dim3(v.tile_threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, v);
 }
 void launch_picard_check(const DevView& v, cudaStream_t s) {
   k_picard_check<<<tile_grid(v), v.tile_threads, 0, s>>>(v);

@@ -37,6 +37,13 @@ void launch_std_update(bool check, const DevView& v, cudaStream_t s);
 void launch_std_dir(const DevView& v, cudaStream_t s);
 void launch_cg_first_update(const DevView& v, cudaStream_t s);
 void launch_cg_update(bool check, const DevView& v, cudaStream_t s);
+// The whole PCG of every instance with pcg_active, from MV_INIT's residual
+// to convergence, in one cooperative launch of one CTA per tile.
+// resident_ctas: CTAs of that kernel the GPU holds at once (0 where its
+// shared memory does not fit or on an error); the launch needs v.ntiles of them.
+constexpr int kResidentMaxTiles = 1184;
+int resident_ctas(const DevView& v, int variant, int num_sms);
+cudaError_t launch_pcg_resident(const DevView& v, int variant, cudaStream_t s);
 void launch_picard_check(const DevView& v, cudaStream_t s);
 // Condition of a device-resident WHILE loop (graph conditional handle h):
 // *iter counts the passes (reset: set to 0); h = 1 while the counter

@@ -144,6 +144,40 @@ bool build_column_plan(int nx, int ny, int nz, int periodic,
   return true;
 }
 
+HaloPlan build_halo(const HostPlan& p) {
+  HaloPlan h;
+  const size_t NC = (size_t)p.ncols;
+  h.begin.assign(p.ntiles + 1, 0);
+  h.col_loc.assign(9 * NC, -1);
+  std::vector<int> slot(NC, -1), cols;  // slot: of the current tile's halo columns
+  for (int t = 0; t < p.ntiles; ++t) {
+    const int c0 = p.tile_col0[t], c1 = c0 + p.tile_ncols[t];
+    cols.clear();
+    for (int q = 0; q < 9; ++q)
+      for (int c = c0; c < c1; ++c) {
+        const int nb = p.col_nbr[(size_t)q * NC + c];
+        if (nb < 0 || (nb >= c0 && nb < c1) || slot[nb] >= 0) continue;
+        slot[nb] = 0;
+        cols.push_back(nb);
+      }
+    // in column order: neighbours of consecutive columns sit side by side
+    std::sort(cols.begin(), cols.end());
+    for (size_t i = 0; i < cols.size(); ++i) {
+      slot[cols[i]] = p.W + (int)i;
+      h.node.push_back(p.col_node[cols[i]]);
+    }
+    for (int q = 0; q < 9; ++q)
+      for (int c = c0; c < c1; ++c) {
+        const int nb = p.col_nbr[(size_t)q * NC + c];
+        if (nb >= 0) h.col_loc[(size_t)q * NC + c] = nb >= c0 && nb < c1 ? nb - c0 : slot[nb];
+      }
+    for (int c : cols) slot[c] = -1;
+    h.begin[t + 1] = (int)h.node.size();
+    h.max_cols = std::max(h.max_cols, (int)cols.size());
+  }
+  return h;
+}
+
 // calcbeta's velocity-dependent laws (glissade_basal_traction.F90:67-598):
 // the factors that do not depend on the speed, in the reference's order of
 // evaluation.  gn = 3 is an integer in the reference (glimmer_physcon.F90:75),

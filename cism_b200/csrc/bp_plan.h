@@ -79,6 +79,14 @@ void slide_vertex(const bp_sliding& L, int i, int j, int nx, double* c1, double*
 // Full plan for n solves.
 bool build_plan(const bp_inputs* in, int n, HostPlan* plan, std::string* err);
 
+// Halo columns of every tile for the resident PCG (DevView::halo_begin,
+// halo_node, col_loc).
+struct HaloPlan {
+  std::vector<int> begin, node, col_loc;
+  int max_cols = 0;
+};
+HaloPlan build_halo(const HostPlan& p);
+
 // velocity (nz,nx-1,ny-1) of instance b <-> node vector
 void gather_velocity(const HostPlan& p, int b, const double* uvel,
                      const double* vvel, double2* x);

@@ -153,3 +153,54 @@ def test_element_centric_assembly_equals_row_form(ctx, name):
     assert np.count_nonzero(outs[0][0]) > 0
     for a, b in zip(*outs):
         assert np.array_equal(a, b)
+
+
+def _resident_models():
+    """Sizes around the resident PCG's edges: one tile, a last tile of one
+    column, 64 levels (tiles of four columns), 256-node tiles, the 2-D solves
+    (256-column tiles), the most tiles that fit (144 and 147 of 11 levels) and
+    the first that does not (the launched kernels run both times)."""
+    cap = dict(pcg_maxiters=60, maxiter_nonlinear=3)
+    return [configs.dome(n=9, nz=3, radius=4.0e3).copy(**cap), configs.dome(n=21, nz=8, radius=15.0e3).copy(**cap),
+            configs.dome(n=13, nz=64, radius=7.0e3).copy(**cap), configs.slab(n=17, nz=11).copy(**cap),
+            configs.slab(n=49, ny_cells=48, nz=11).copy(**cap), configs.slab(n=48, nz=11).copy(**cap),
+            configs.slab(n=52, nz=11).copy(**cap), configs.marine(n=40, dx=4000.0).copy(**cap),
+            configs.marine(n=36, dx=4000.0).copy(approx_2d=configs.APPROX_SSA, **cap),
+            configs.slab(n=36).copy(approx_2d=configs.APPROX_DIVA, **cap)]
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("variant", [configs.SPARSE_PCG_STANDARD, configs.SPARSE_PCG_CHRONGEAR])
+@pytest.mark.parametrize("precond", [configs.PRECOND_NONE, configs.PRECOND_DIAG, configs.PRECOND_SIA])
+def test_resident_pcg_equals_launched(ctx, variant, precond, mixed):
+    """The resident PCG against the launched kernels (a timing run launches
+    every step): the same arithmetic in the same order, so bitwise the same
+    velocities, iterations and norms; also for a batch of uneven instances
+    that end at different iterations, and with a check every 1, 3 and 5."""
+    models = [m for m in _resident_models() if not (m.approx_2d and precond == configs.PRECOND_SIA)]
+    groups = [[m] for m in models]
+    groups.append([configs.slab(n=16).copy(pcg_maxiters=40, maxiter_nonlinear=4),
+                   configs.dome(n=15, nz=11, radius=11.0e3).copy(pcg_maxiters=400, maxiter_nonlinear=3),
+                   configs.dome(n=9, nz=11, radius=4.0e3).copy(pcg_maxiters=7, maxiter_nonlinear=2)])
+    for i, ms in enumerate(groups):
+        ncheck = (5, 1, 3)[i % 3]
+        ms = [m.copy(which_sparse=variant, which_precond=precond, pcg_ncheck=ncheck, pcg_tol=1e-5) for m in ms]
+        preps = [solver.prepare(m, precision=solver.MIXED if mixed else solver.FP64)[0] for m in ms]
+        prob = ctx.problem(preps)
+        zero = [np.zeros(m.vshape3) for m in ms]
+        got = []
+        for timing in (False, False, True):
+            prob.timing(timing)
+            prob.set_guess(zero, zero)
+            st = prob.run()
+            u, v, e = prob.get(want_efvs=True)
+            got.append((u, v, e, st))
+        prob.timing(False)
+        prob.close()
+        keys = ("status", "picard_iters", "pcg_iters_total", "pcg_iters_last", "refine_steps_total", "converged",
+                "pcg_err_last", "resid_velo", "L2_norm", "L2_norm_relative")
+        for other in got[1:]:
+            for a, b in zip(got[0][:3], other[:3]):
+                assert all(np.array_equal(x, y) for x, y in zip(a, b)), (ms[0].name, ncheck)
+            for s, r in zip(got[0][3], other[3]):
+                assert {k: s[k] for k in keys} == {k: r[k] for k in keys}, (ms[0].name, ncheck)
