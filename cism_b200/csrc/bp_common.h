@@ -207,6 +207,26 @@ struct DevView {
   const int* halo_node;
   const int* col_loc;      // [9][ncols]
   int halo_max;            // most halo columns of a tile
+  // staged Krylov matvec (desc null: not used): one descriptor of desc_bytes
+  // per tile (StagedDesc), and the warps' sums of every tile
+  const unsigned char* desc;
+  int staged;              // the Krylov matvecs run the staged kernel
+  double* wsum;            // [ntiles][8][3]
+};
+
+// Descriptor of a tile for the staged matvec.  16 bytes: its number,
+// columns, halo columns (-1: more than fit, the tile takes the plain path)
+// and instance.  Per column 64 bytes: the nine stencil neighbours as
+// one-byte slots (own column c, W + h for halo column h, zero_slot for
+// none), then from byte 16 their nodes at level 0 (the column's own for
+// none).  Then the node at level 0 of every slot.  A row of columns has
+// 2 W + 6 halo columns, a tile that wraps to the next row two or three
+// more; past 2 W + 8 it is cut into many rows.
+struct StagedDesc {
+  static BP_HD constexpr int halo_cap(int W) { return 2 * W + 8; }
+  static BP_HD constexpr int zero_slot(int W) { return W + halo_cap(W); }
+  static BP_HD constexpr int nodes_at(int W) { return 16 + 64 * W; }
+  static BP_HD constexpr int bytes(int W) { return nodes_at(W) + 4 * (W + halo_cap(W)); }
 };
 
 // Node of (col, k) in the blocked level-major layout.

@@ -100,8 +100,8 @@ struct bp_ctx {
   int num_sms = 0;
   int l2_max_persist = 0, l2_max_window = 0;  // bytes (0 = no persisting L2)
   // autotuner results: (node bucket, nz, storage, precision, PCG variant)
-  // -> (minb, grid) of the residual kernels, (minb_k, grid_k) of the Krylov matvecs
-  std::map<std::tuple<int, int, int, int, int>, std::array<int, 4>> tuned;
+  // -> (minb, grid) of the residual kernels, (minb_k, grid_k, staged) of the Krylov matvecs
+  std::map<std::tuple<int, int, int, int, int>, std::array<int, 5>> tuned;
   bp::GuessNet* net = nullptr;     // the learned guess's network (bp_guess_load)
   int net_launches = 0;            // kernels the network launched (bp_guess_launches)
 };
@@ -298,6 +298,18 @@ void use_resident_pcg(bp_ctx* c, Arena& a, DevView* v, const HostPlan& p) {
   v->halo_begin = t;
   v->halo_node = t + h.begin.size();
   v->col_loc = t + h.begin.size() + h.node.size();
+}
+
+// The staged Krylov matvec's descriptors, where the problem has its shape
+// and no resident PCG; the autotuner chooses between it and the per-node one.
+void use_staged_mv(bp_ctx* c, Arena& a, DevView* v, const HostPlan& p) {
+  if (p.ntiles == 0 || v->xch || staged_per_sm(*v) == 0) return;
+  cudaStream_t s = c->stream;
+  unsigned char* d = a.get<unsigned char>(s, "staged_desc", (size_t)p.ntiles * StagedDesc::bytes(p.W));
+  v->wsum = a.get<double>(s, "staged_sums", (size_t)p.ntiles * 8 * 3);
+  launch_staged_desc(*v, d, s);
+  CK(cudaGetLastError());
+  v->desc = d;
 }
 
 void init_state(cudaStream_t s, const DevView& v, const HostPlan& p, bool picard, bool pcg) {
@@ -499,7 +511,7 @@ void linear_solve(bp_problem* P) {
 //    (every tile, instance state untouched) for occupancy target 0, 4 or 6
 //    and grid one CTA per tile or one wave of resident CTAs.  Its register
 //    allocation, and so its occupancy, differs from the residual kernel's.
-// BP_MV_CONFIG="minb,grid[,minb_k,grid_k]" fixes the choice (for sweeps);
+// BP_MV_CONFIG="minb,grid[,minb_k,grid_k[,staged]]" fixes the choice (for sweeps);
 // BP_TUNE_LOG=1 prints every candidate's time to stderr.
 static float time_launches(bp_ctx* c, const std::function<void()>& launch) {
   launch();
@@ -518,13 +530,15 @@ void autotune(bp_problem* P) {
   P->tuned = true;
   if (v.xch) return;  // the resident PCG has no launch shape to choose
   if (const char* e = std::getenv("BP_MV_CONFIG")) {
-    int a[4] = {0, 0, 0, 0};
-    const int n = std::sscanf(e, "%d,%d,%d,%d", &a[0], &a[1], &a[2], &a[3]);
-    if (n == 2 || n == 4) {
+    int a[5] = {0, 0, 0, 0, 0};
+    const int n = std::sscanf(e, "%d,%d,%d,%d,%d", &a[0], &a[1], &a[2], &a[3], &a[4]);
+    if (n == 2 || n == 4 || n == 5) {
       v.minb = a[0];
       v.grid_cap = a[1];
-      v.minb_k = n == 4 ? a[2] : a[0];
-      v.grid_k = n == 4 ? a[3] : a[1];
+      v.minb_k = n >= 4 ? a[2] : a[0];
+      v.grid_k = n >= 4 ? a[3] : a[1];
+      v.staged = n == 5 && a[4] && v.desc ? 1 : 0;
+      if (v.staged && v.grid_k <= 0) v.grid_k = staged_per_sm(v) * c->num_sms;
       return;
     }
   }
@@ -536,6 +550,7 @@ void autotune(bp_problem* P) {
     v.grid_cap = it->second[1];
     v.minb_k = it->second[2];
     v.grid_k = it->second[3];
+    v.staged = it->second[4];
     return;
   }
   const bool log = std::getenv("BP_TUNE_LOG") != nullptr;
@@ -557,7 +572,7 @@ void autotune(bp_problem* P) {
   if (v.A32) launch_make_a32(v, c->stream);
   const int mode = variant == 3 ? MV_CG1 : MV_STD_A;
   best = 1e30f;
-  int km = 0, kg = 0;
+  int km = 0, kg = 0, ks = 0;
   struct DryPass {  // the dry flag never outlives the timing, not even on an error
     DevView& v;
     explicit DryPass(DevView& w) : v(w) { v.dry = 1; }
@@ -580,10 +595,20 @@ void autotune(bp_problem* P) {
       }
     }
   }
+  if (v.desc) {
+    const DryPass dry(v);
+    const int g = staged_per_sm(v) * c->num_sms;
+    v.staged = 1;
+    v.grid_k = g;
+    const float ms = time_launches(c, [&] { launch_mv(mode, v, c->stream); });
+    if (log) std::fprintf(stderr, "autotune krylov staged grid %d: %.2f us\n", g, ms * 1e3f);
+    if (ms < best) { best = ms; km = 0; kg = g; ks = 1; }
+  }
   CK(cudaGetLastError());
   v.minb_k = km;
   v.grid_k = kg;
-  c->tuned[key] = {bm, bg, km, kg};
+  v.staged = ks;
+  c->tuned[key] = {bm, bg, km, kg, ks};
 }
 
 // The Picard loop of glissade_velo_higher_solve on the device.
@@ -867,6 +892,7 @@ bp_problem* problem_new(bp_ctx* c, Arena* arena, int n, const bp_inputs* in, std
   P->v = make_view(*P->arena, c->stream, P->plan, true, P->mixed);
   P->h2d_bytes = g_h2d;
   use_resident_pcg(c, *P->arena, &P->v, P->plan);
+  use_staged_mv(c, *P->arena, &P->v, P->plan);
   P->x0 = P->arena->get<double2>(c->stream, "x0", P->plan.npad);
   CK(cudaMemsetAsync(P->x0, 0, sizeof(double2) * P->plan.npad, c->stream));
   if (P->plan.diva) {

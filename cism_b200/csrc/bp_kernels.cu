@@ -1303,8 +1303,8 @@ __global__ void __launch_bounds__(PER_SM == 2 ? 192 : kTile, PER_SM) k_pcg_resid
       const double2 sv = s[lev + kA * ls + nbr[c * slots]];
       if (MIXED && !(kA == 0 && c == 4)) {
         const float4 a = MF[m];
-        yu += dot2(make_double2(a.x, a.y), sv);
-        yv += dot2(make_double2(a.z, a.w), sv);
+        yu += dot2(make_double2((double)a.x, (double)a.y), sv);
+        yv += dot2(make_double2((double)a.z, (double)a.w), sv);
       } else {
         yu += dot2(MIXED ? DG[i] : M0[m], sv);
         yv += dot2(MIXED ? DG[slots + i] : M1[m], sv);
@@ -1493,6 +1493,459 @@ __global__ void __launch_bounds__(PER_SM == 2 ? 192 : kTile, PER_SM) k_pcg_resid
     if (G.picard_active && !S.picard_active) atomicSub(&v.cnt->picard_active, 1);
     G = S;
     v.xch_epoch[R.inst] = (es > en ? es : en) + (ok ? 0 : 4);  // after a failed wait other CTAs may be ahead
+  }
+}
+
+// ---------------------------------------------------------------------
+// Staged Krylov matvec: k_cg_mv and k_std_mv on half storage, for problems
+// too large for the resident PCG.
+//
+// The per-node kernels run at 0.4 of the copy bandwidth with no unit
+// saturated: a thread's 55 16-byte loads, two thirds of them gathers, go
+// through L1 with the few registers that eight CTAs an SM leave, and each
+// tile ends in a fence and a ticket that its warps wait for.  Here a CTA
+// walks its tiles as a pipeline.  A producer warp brings each tile's own
+// matrix rows (one bulk copy per offset: the DRAM stream) and its source
+// vector with the halo columns' (16-byte asynchronous copies, each value
+// once instead of up to 27 times) into one of two shared-memory stages
+// while the other is computed, so the stream never waits for arithmetic;
+// the consumer warps, one thread per node, hold the 13 transposed entries
+// of the neighbours' rows in registers and load the next tile's into the
+// same registers as they use this one's.  Sums: each warp stores its
+// tile's, and the CTA adds them, in block_reduce's order, and takes its
+// tickets once, after its last tile.  The arithmetic and its order are the
+// per-node kernels' (bitwise the same results).
+//
+// Barriers, all waits bounded (past the limit the CTA marks the instances'
+// sums as NaN, which ends their solve with BP_ERR_NAN): full[stage] -- the
+// stage's copies have landed (32 producer lanes and the bulk bytes);
+// empty[stage] -- every consumer warp is done with it; dfull[slot] -- a
+// descriptor (ring of four, two tiles ahead of the copies) has landed.
+//
+// What bounds it: the consumers, six warps a tile (one CTA an SM in FP64,
+// whose two stages are 177 KB; two in FP32), wait on shared memory and on
+// their own chains; DRAM is at 0.6-0.65 of the copy bandwidth in FP64.
+// Measured, the fastest per-node shape -> this kernel, a launch of
+// k_cg_mv's work: 400 x 400 x 11 marine sheet, FP64 (1.05 M nodes) 156 ->
+// 123 us; 160 x 160 x 11 slab, FP64, standard PCG 46.5 -> 37.7 us; four
+// 256 x 256 x 11 sheets, FP32 (1.73 M nodes) 172 -> 160 us; 16 uneven domains,
+// FP32 (0.62 M nodes) 65 -> 79 us.  The autotuner times both on the problem.
+// ---------------------------------------------------------------------
+constexpr int kStages = 2, kDescs = 4;
+
+
+template <int STORE>
+__host__ __device__ constexpr int staged_own() { return STORE == ST_SYM32 ? 15 : 28; }  // 16-byte rows per node
+struct StagedShape {
+  int slots, ls, desc;
+  size_t own, stage, bytes;
+};
+__host__ __device__ inline StagedShape staged_shape(const DevView& v, bool f32) {
+  StagedShape h;
+  h.slots = v.W * v.nz;
+  h.ls = StagedDesc::zero_slot(v.W) + 1;
+  h.desc = StagedDesc::bytes(v.W);
+  h.own = (size_t)16 * h.slots * (f32 ? staged_own<ST_SYM32>() : staged_own<ST_SYM>());
+  h.stage = h.own + (size_t)16 * (v.nz + 2) * h.ls;
+  h.bytes = kStages * h.stage + (size_t)kDescs * h.desc + 8 * (2 * kStages + kDescs);
+  return h;
+}
+
+__device__ __forceinline__ unsigned smem_at(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+  for (int i = 0; i < (1 << 22); ++i) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void bar_init(unsigned bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
+// One CTA per tile: the tile's halo columns, in order of first appearance
+// over (neighbour, column), and its descriptor.
+__global__ void __launch_bounds__(256) k_staged_desc(const __grid_constant__ DevView v, unsigned char* desc) {
+  extern __shared__ int sd[];  // [9 W] neighbour (-1: none or own), then its halo index
+  __shared__ int nh;
+  const int t = blockIdx.x, W = v.W, E = 9 * W, cap = StagedDesc::halo_cap(W);
+  const int c0 = v.tile_col0[t], ncols = v.tile_ncols[t];
+  unsigned char* d = desc + (size_t)t * StagedDesc::bytes(W);
+  int* node = reinterpret_cast<int*>(d + StagedDesc::nodes_at(W));
+  if (threadIdx.x == 0) nh = 0;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    const int q = e / W, c = e - q * W;
+    int nb = c < ncols ? v.col_nbr[(size_t)q * v.ncols + c0 + c] : -1;
+    if (nb >= c0 && nb < c0 + ncols) nb = -1;
+    sd[e] = nb;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {  // first[e]: where this column appears first
+    int first = e;
+    if (sd[e] >= 0)
+      for (int f = 0; f < e; ++f)
+        if (sd[f] == sd[e]) { first = f; break; }
+    sd[E + e] = sd[e] >= 0 && first == e ? 1 : 0;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    const int q = e / W, c = e - q * W;
+    int slot = StagedDesc::zero_slot(W);
+    const int nb = c < ncols ? v.col_nbr[(size_t)q * v.ncols + c0 + c] : -1;
+    if (nb >= c0 && nb < c0 + ncols) {
+      slot = nb - c0;
+    } else if (nb >= 0) {
+      int first = 0, h = 0;
+      while (sd[first] != nb) h += sd[E + first++];
+      slot = h < cap ? W + h : slot;
+      if (first == e) {
+        atomicAdd(&nh, 1);
+        if (h < cap) node[W + h] = v.col_node[nb];
+      }
+    }
+    d[16 + 64 * c + q] = (unsigned char)slot;
+    reinterpret_cast<int*>(d + 32 + 64 * c)[q] = nb >= 0 ? v.col_node[nb] : v.tile_start[t] + c;
+  }
+  for (int c = threadIdx.x; c < W; c += blockDim.x) node[c] = v.tile_start[t] + c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int* m = reinterpret_cast<int*>(d);
+    m[0] = t;
+    m[1] = ncols;
+    m[2] = nh <= cap ? nh : -1;
+    m[3] = v.tile_inst[t];
+  }
+}
+
+// The product of one row by the per-node bodies, out of line, for tiles of
+// an instance whose FP32 refinement stalled and tiles without a descriptor.
+template <int STORE>
+__device__ __noinline__ double2 plain_row_call(const DevView& v, bool fp64, int col, int k, size_t n,
+                                               const double2* s) {
+  const SrcX src{s};
+  if (STORE == ST_SYM32 && !fp64) return matvec_row_sym32(v, v.A32, col, k, n, src);
+  return matvec_row_sym(v, v.A, col, k, n, src);
+}
+
+// LS: slots per level of the source vector, compile-time for the usual 16
+// columns (0: from W).  THREADS: the most a CTA has (a tile's and the producer's 32); registers are
+// granted in groups of four warps, so 7 warps leave far more than 9.
+template <int STORE, int MODE, int THREADS, int LS>
+__global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
+    k_mv_staged(const __grid_constant__ DevView v) {
+  constexpr bool F32 = STORE == ST_SYM32;
+  constexpr int NV = MODE == MV_STD_A ? 1 : 3, NOWN = staged_own<STORE>();
+  extern __shared__ __align__(128) unsigned char st_sm[];
+  const StagedShape H = staged_shape(v, F32);
+  const int slots = H.slots, ls = LS > 0 ? LS : H.ls, nz = v.nz, W = LS > 0 ? 16 : v.W, G = gridDim.x;
+  const int i = threadIdx.x, lane = i & 31, warp = i >> 5, nw = (blockDim.x >> 5) - 1;
+  const double2* s = MODE == MV_STD_A ? v.d0 : v.z;
+  unsigned char* descs = st_sm + kStages * H.stage;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(descs + kDescs * H.desc);
+  auto full = [&](int b) { return smem_at(bars + b); };
+  auto empty = [&](int b) { return smem_at(bars + kStages + b); };
+  auto dfull = [&](int b) { return smem_at(bars + 2 * kStages + b); };
+  auto stage_own = [&](int b) { return st_sm + b * H.stage; };
+  auto stage_src = [&](int b) { return reinterpret_cast<double2*>(st_sm + b * H.stage + H.own); };
+  if (i == 0) {
+    for (int b = 0; b < kStages; ++b) {
+      bar_init(full(b), 33);
+      bar_init(empty(b), nw);
+    }
+    for (int b = 0; b < kDescs; ++b) bar_init(dfull(b), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // the zeros that absent neighbours read: the last slot of every level, and
+  // a level above and below
+  for (int e = i; e < kStages * (nz + 2) * ls; e += blockDim.x) {
+    const int b = e / ((nz + 2) * ls), o = e - b * (nz + 2) * ls, lev = o / ls;
+    if (lev == 0 || lev == nz + 1 || o - lev * ls == ls - 1) stage_src(b)[o] = make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  pdl_wait();
+  pdl_launch_next();
+  // the CTA's tiles: every G-th, of the instances that are solving
+  auto next_tile = [&](int t) {
+    for (; t < v.ntiles; t += G)
+      if (v.dry || v.st[v.tile_inst[t]].pcg_active) return t;
+    return -1;
+  };
+  bool ok = true;
+
+  if (warp == nw) {  // producer
+    int tn = next_tile(blockIdx.x);  // the next tile whose descriptor is fetched
+    auto fetch = [&](int j) {        // descriptor j of the sequence (after the last: tile -1)
+      unsigned char* d = descs + (j % kDescs) * H.desc;
+      if (lane == 0) {
+        if (tn >= 0) {
+          bar_expect(dfull(j % kDescs), H.desc);
+          bulk_load(smem_at(d), v.desc + (size_t)tn * H.desc, H.desc, dfull(j % kDescs));
+        } else {
+          *reinterpret_cast<int*>(d) = -1;
+          bar_arrive(dfull(j % kDescs));
+        }
+      }
+      if (tn >= 0) tn = next_tile(tn + G);
+    };
+    fetch(0);
+    fetch(1);
+    for (int j = 0; ok; ++j) {
+      const int b = j % kStages;
+      if (j >= kStages) ok = bar_wait(empty(b), ((j / kStages) - 1) & 1);
+      ok = ok && bar_wait(dfull(j % kDescs), (j / kDescs) & 1);
+      if (!ok) break;
+      const unsigned char* d = descs + (j % kDescs) * H.desc;
+      const int4 m = *reinterpret_cast<const int4*>(d);  // tile, columns, halo columns, instance
+      if (m.x < 0) break;
+      const int nc = m.z < 0 ? 0 : W + m.z;
+      if (lane == 0) bar_expect(full(b), nc ? 16u * slots * NOWN : 0u);
+      __syncwarp();
+      if (nc) {
+        const size_t n0 = (size_t)m.x * slots, np = (size_t)v.npad;
+        if (lane < NOWN) {
+          const void* g = F32 ? (lane < 13 ? static_cast<const void*>(v.A32 + (size_t)(lane + 1) * np + n0)
+                                           : static_cast<const void*>(v.A32d + (size_t)(lane - 13) * np + n0))
+                              : static_cast<const void*>(v.A + (size_t)lane * np + n0);
+          bulk_load(smem_at(stage_own(b)) + 16u * slots * lane, g, 16u * slots, full(b));
+        }
+        const int* node = reinterpret_cast<const int*>(d + StagedDesc::nodes_at(W));
+        const unsigned dst = smem_at(stage_src(b) + ls);
+        for (int c = lane; c < nc; c += 32) {
+          const double2* g = s + node[c];
+          unsigned a = dst + 16u * c;
+          for (int k = 0; k < nz; ++k, a += 16u * ls, g += W)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(g) : "memory");
+        }
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full(b)) : "memory");
+      fetch(j + 2);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else {  // consumers: thread i is node i of every tile
+    const bool inside = i < slots;
+    const int k = inside ? i >> v.lsh : 0, c = i & (W - 1);
+    constexpr int NT = F32 ? 13 : 26;
+    typedef typename std::conditional<F32, float4, double2>::type Entry;
+    Entry T[NT];  // entries of the neighbours' rows toward this node, offset m at [m] (FP64: [2 m], [2 m + 1])
+    const Entry* mat = F32 ? reinterpret_cast<const Entry*>(v.A32) : reinterpret_cast<const Entry*>(v.A);
+    const unsigned np = (unsigned)v.npad;
+    const int klev = k * W, kup = max(k - 1, 0) * W;
+    // nb: the neighbour columns' nodes; loads entry m of their tile into T
+    // (an absent neighbour's stand-in, this column's own node, meets a zero)
+    struct Nodes { int4 a, b; int c; };
+    auto load_t = [&](int m, const Nodes& nb) {
+      const int q = m % 9, kA = m / 9 - 1;
+      const int n0 = q == 0 ? nb.a.x : q == 1 ? nb.a.y : q == 2 ? nb.a.z : q == 3 ? nb.a.w : q == 4 ? nb.b.x
+                   : q == 5 ? nb.b.y : q == 6 ? nb.b.z : q == 7 ? nb.b.w : nb.c;
+      const unsigned p = (unsigned)(n0 + (kA < 0 ? kup : klev));
+      if (F32) {
+        T[m] = __ldg(mat + (size_t)(13 - m) * np + p);
+      } else {
+        T[2 * m] = __ldg(mat + (size_t)(13 - m) * np + p);
+        T[2 * m + 1] = __ldg(mat + (size_t)(27 - m) * np + p);
+      }
+    };
+    auto slot_of = [](const uint4& r, int q) {
+      const unsigned w = q < 4 ? r.x : (q < 8 ? r.y : r.z);
+      return (int)((w >> (8 * (q & 3))) & 255u);
+    };
+    auto desc_meta = [&](int j) { return *reinterpret_cast<const int4*>(descs + (j % kDescs) * H.desc); };
+    auto desc_rec = [&](int j) { return *reinterpret_cast<const uint4*>(descs + (j % kDescs) * H.desc + 16 + 64 * c); };
+    auto desc_nodes = [&](int j) {
+      const int4* p = reinterpret_cast<const int4*>(descs + (j % kDescs) * H.desc + 32 + 64 * c);
+      return Nodes{p[0], p[1], p[2].x};
+    };
+    ok = bar_wait(dfull(0), 0);
+    int4 m = ok ? desc_meta(0) : make_int4(-1, 0, 0, 0);
+    uint4 rec = make_uint4(0, 0, 0, 0);
+    Nodes nb = {make_int4(0, 0, 0, 0), make_int4(0, 0, 0, 0), 0};
+    if (m.x >= 0) {
+      rec = desc_rec(0);
+      nb = desc_nodes(0);
+#pragma unroll
+      for (int e = 0; e < 13; ++e) load_t(e, nb);
+    }
+    for (int j = 0; ok && m.x >= 0; ++j) {
+      const int b = j % kStages;
+      const bool mine = inside && c < m.y;
+      const size_t n = (size_t)m.x * slots + i;
+      const InstState& S0 = v.st[m.w];
+      const bool fp64 = F32 && S0.krylov_fp64;
+      double2 r = make_double2(0.0, 0.0);
+      if (MODE != MV_STD_A && mine) r = v.r[n];
+      ok = bar_wait(dfull((j + 1) % kDescs), ((j + 1) / kDescs) & 1);
+      const int4 mn = ok ? desc_meta(j + 1) : make_int4(-1, 0, 0, 0);
+      if (mn.x >= 0) nb = desc_nodes(j + 1);  // after the last tile its own entries once more
+      const uint4 recn = mn.x >= 0 ? desc_rec(j + 1) : rec;
+      ok = ok && bar_wait(full(b), (j / kStages) & 1);
+      if (!ok) break;
+      double yu = 0.0, yv = 0.0;
+      double2 sn = make_double2(0.0, 0.0);
+      const double2* src = stage_src(b);
+      if (m.z >= 0 && !fp64) {
+        const Entry* own = reinterpret_cast<const Entry*>(stage_own(b)) + (inside ? i : 0);
+        const double2* dg = reinterpret_cast<const double2*>(stage_own(b)) + (inside ? i : 0) + 13 * slots;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+          const double2* sq = src + (k + 1) * ls + slot_of(rec, q);
+#pragma unroll
+          for (int kA = -1; kA <= 1; ++kA) {
+            const int mm = (kA + 1) * 9 + q;
+            const double2 sv = sq[kA * ls];
+            if (mm == 13) sn = sv;
+            double2 a0, a1;
+            if (mm < 13) {
+              if constexpr (F32) {
+                a0 = make_double2((double)T[mm].x, (double)T[mm].z);
+                a1 = make_double2((double)T[mm].y, (double)T[mm].w);
+              } else {
+                a0 = make_double2(T[2 * mm].x, T[2 * mm + 1].x);
+                a1 = make_double2(T[2 * mm].y, T[2 * mm + 1].y);
+              }
+              load_t(mm, nb);
+            } else if constexpr (F32) {
+              if (mm == 13) {
+                a0 = dg[0];
+                a1 = dg[slots];
+              } else {
+                const Entry a = own[(mm - 14) * slots];
+                a0 = make_double2((double)a.x, (double)a.y);
+                a1 = make_double2((double)a.z, (double)a.w);
+              }
+            } else {
+              a0 = own[(mm - 13) * slots];
+              a1 = own[(mm + 1) * slots];
+            }
+            yu += dot2(a0, sv);
+            yv += dot2(a1, sv);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) bar_arrive(empty(b));
+      if (m.z < 0 || fp64) {
+        if (mine) {
+          const double2 y = plain_row_call<STORE>(v, fp64, v.tile_col0[m.x] + c, k, n, s);
+          yu = y.x;
+          yv = y.y;
+          sn = s[n];
+        }
+#pragma unroll
+        for (int e = 0; e < 13; ++e) load_t(e, nb);
+      }
+      double part[NV];
+#pragma unroll
+      for (int e = 0; e < NV; ++e) part[e] = 0.0;
+      if (mine) {
+        const double2 y = make_double2(yu, yv);
+        if (MODE == MV_CG_FIRST) v.d0[n] = sn;
+        if (MODE == MV_CG1) v.Az[n] = y;
+        else v.q[n] = y;
+        if (MODE == MV_STD_A) {
+          part[0] = dot2(sn, y);
+        } else {
+          part[0] = dot2(r, sn);
+          part[NV > 1 ? 1 : 0] = dot2(y, sn);
+          part[NV > 2 ? 2 : 0] = dot2(r, r);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < NV; ++e) {
+        double x = part[e];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) v.wsum[((size_t)m.x * 8 + warp) * 3 + e] = x;
+      }
+      if (i == 0 && v.mv_nodes && !v.dry) atomicAdd(&v.mv_nodes[F32 && !fp64 ? 1 : 0], (unsigned long long)m.y * nz);
+      m = mn;
+      rec = recn;
+    }
+  }
+  // the tiles' sums, tickets, and where this CTA brought an instance's last
+  // tile the instance's sums (tile_finish's order) and scalar update
+  const bool all_ok = __syncthreads_and(ok);
+  __shared__ double sm[NV * 32];
+  __shared__ int last;
+  for (int base = blockIdx.x; base < v.ntiles; base += G * blockDim.x) {
+    const long tl = (long)base + (long)i * G;
+    const int t = tl < v.ntiles ? (int)tl : -1;
+    int inst = -1, done = 0;
+    if (t >= 0) {
+      inst = v.tile_inst[t];
+      if (v.dry || v.st[inst].pcg_active) {
+#pragma unroll
+        for (int e = 0; e < NV; ++e) {
+          double w[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) w[q] = q < nw ? v.wsum[((size_t)t * 8 + q) * 3 + e] : 0.0;
+          const double x = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+          v.partials[(size_t)e * v.ntiles + t] = all_ok ? x : __longlong_as_double(0x7ff8000000000000LL);
+        }
+        __threadfence();
+        const InstParams& ip = v.inst[inst];
+        done = atomicAdd(&v.tile_counter[inst], 1u) == (unsigned)(ip.tile_end - ip.tile_begin) - 1u;
+      }
+    }
+    while (__syncthreads_or(done)) {
+      if (done) last = i;  // any one of them
+      __syncthreads();
+      const int who = last;
+      __syncthreads();
+      if (i == who) {
+        last = inst;
+        done = 0;
+      }
+      __syncthreads();
+      const int fin = last;
+      __threadfence();
+      const InstParams& ip = v.inst[fin];
+      const int bd = v.tile_threads;  // the threads tile_finish sums with
+      double x[NV];
+#pragma unroll
+      for (int e = 0; e < NV; ++e) x[e] = 0.0;
+      constexpr int U = 4;
+      if (i < bd)
+        for (int t0 = ip.tile_begin + i; t0 < ip.tile_end; t0 += U * bd) {
+          double p[U][NV];
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int e = 0; e < NV; ++e)
+              p[u][e] = t0 + u * bd < ip.tile_end ? __ldcg(v.partials + (size_t)e * v.ntiles + t0 + u * bd) : 0.0;
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (t0 + u * bd < ip.tile_end)
+#pragma unroll
+              for (int e = 0; e < NV; ++e) x[e] += p[u][e];
+        }
+      block_reduce<NV, false>(x, sm);
+      if (i == 0) {
+        v.tile_counter[fin] = 0;
+        if (!v.dry) {
+          if (MODE == MV_STD_A) std_mv_fin<true>(v, v.st[fin], x);
+          else cg_mv_fin<MODE == MV_CG_FIRST, true>(v, v.inst[fin], v.st[fin], x);
+        }
+        __threadfence();
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -1735,11 +2188,12 @@ static const bool g_pdl_env = [] {
 static thread_local bool g_pdl_on = true;
 void set_pdl(bool on) { g_pdl_on = on; }
 
-static void launch_pcg(void (*kernel)(DevView), int g, cudaStream_t s, const DevView& v, int block = 0) {
+static void launch_pcg(void (*kernel)(DevView), int g, cudaStream_t s, const DevView& v, int block = 0,
+                       size_t smem = 0) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g);
   cfg.blockDim = dim3(block > 0 ? block : v.tile_threads);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[2];
   unsigned na = 0;
@@ -1800,7 +2254,45 @@ static void launch_resid_minb(int mode, const DevView& v, cudaStream_t s, int g)
   if (v.minb == 4) launch_resid_store<STORE, 4>(mode, v, s, g);
   else launch_resid_store<STORE, 0>(mode, v, s, g);
 }
+template <int STORE, int THREADS, int LS>
+static TileKernel staged_kernel_st(int mode) {
+  switch (mode) {
+    case MV_STD_A: return k_mv_staged<STORE, MV_STD_A, THREADS, LS>;
+    case MV_CG_FIRST: return k_mv_staged<STORE, MV_CG_FIRST, THREADS, LS>;
+    default: return k_mv_staged<STORE, MV_CG1, THREADS, LS>;
+  }
+}
+static TileKernel staged_kernel(const DevView& v, int mode) {
+  constexpr int LS16 = StagedDesc::zero_slot(16) + 1;
+  if (v.W == 16 && v.tile_threads <= 192)
+    return v.A32 ? staged_kernel_st<ST_SYM32, 224, LS16>(mode) : staged_kernel_st<ST_SYM, 224, LS16>(mode);
+  return v.A32 ? staged_kernel_st<ST_SYM32, 288, 0>(mode) : staged_kernel_st<ST_SYM, 288, 0>(mode);
+}
+int staged_per_sm(const DevView& v) {
+  if (!v.sym || v.nz == 1 || StagedDesc::zero_slot(v.W) > 255) return 0;
+  const StagedShape h = staged_shape(v, v.A32 != nullptr);
+  int least = 0;
+  for (int mode : {(int)MV_STD_A, (int)MV_CG_FIRST, (int)MV_CG1}) {
+    TileKernel k = staged_kernel(v, mode);
+    int n = 0;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.bytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, v.tile_threads + 32, h.bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    least = least == 0 ? n : (n < least ? n : least);
+  }
+  return least;
+}
+void launch_staged_desc(const DevView& v, unsigned char* desc, cudaStream_t s) {
+  if (v.ntiles > 0) k_staged_desc<<<v.ntiles, 256, 2 * 9 * v.W * sizeof(int), s>>>(v, desc);
+}
 void launch_mv(int mode, const DevView& v, cudaStream_t s) {
+  if (is_krylov(mode) && v.staged) {
+    const int g = v.ntiles < v.grid_k ? v.ntiles : v.grid_k;
+    launch_pcg(staged_kernel(v, mode), g, s, v, v.tile_threads + 32, staged_shape(v, v.A32 != nullptr).bytes);
+    return;
+  }
   if (is_krylov(mode)) {
     int g = v.ntiles > 0 ? v.ntiles : 1;
     if (v.grid_k > 0 && g > v.grid_k) g = v.grid_k;

@@ -44,6 +44,11 @@ void launch_cg_update(bool check, const DevView& v, cudaStream_t s);
 constexpr int kResidentMaxTiles = 1184;
 int resident_ctas(const DevView& v, int variant, int num_sms);
 cudaError_t launch_pcg_resident(const DevView& v, int variant, cudaStream_t s);
+// The staged Krylov matvec: shared memory of a CTA, the most CTAs an SM
+// takes (0: not for this shape), and the kernel that writes the descriptors
+// (v.desc, StagedDesc).
+int staged_per_sm(const DevView& v);
+void launch_staged_desc(const DevView& v, unsigned char* desc, cudaStream_t s);
 void launch_picard_check(const DevView& v, cudaStream_t s);
 // Condition of a device-resident WHILE loop (graph conditional handle h):
 // *iter counts the passes (reset: set to 0); h = 1 while the counter

@@ -204,3 +204,54 @@ def test_resident_pcg_equals_launched(ctx, variant, precond, mixed):
                 assert all(np.array_equal(x, y) for x, y in zip(a, b)), (ms[0].name, ncheck)
             for s, r in zip(got[0][3], other[3]):
                 assert {k: s[k] for k in keys} == {k: r[k] for k in keys}, (ms[0].name, ncheck)
+
+
+def _staged_models():
+    """Past the resident PCG's sizes: odd rows (tiles that wrap from one row to
+    the next), a front, an outflow domain with ice at its edges, sheets with
+    scattered holes (tiles cut into many rows, some past a descriptor's halo),
+    tiles of 256 (8 levels), 224 (14), 160 (5) and 132 nodes (33 levels), and
+    columns too short for the staged kernel (2 levels: the per-node kernel)."""
+    cap = dict(pcg_maxiters=25, maxiter_nonlinear=2)
+    holes = configs.slab(n=90, nz=11)
+    rng = np.random.default_rng(8)
+    keep = rng.uniform(size=holes.thck.shape) < 0.55
+    thin = holes.copy(thck=configs.halo_fill_cells(np.where(keep, holes.thck, 0.0)), **cap)
+    return [configs.slab(n=75, ny_cells=71, nz=11).copy(**cap), configs.marine(n=100, dx=4000.0).copy(**cap),
+            configs.marine(n=100, dx=4000.0, radius_frac=0.7).copy(periodic=0, **cap), thin,
+            configs.slab(n=101, nz=8).copy(**cap), configs.slab(n=75, nz=14).copy(**cap),
+            configs.slab(n=111, nz=5).copy(**cap), configs.slab(n=41, nz=33).copy(**cap),
+            configs.slab(n=210, nz=2).copy(**cap)]
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("variant", [configs.SPARSE_PCG_STANDARD, configs.SPARSE_PCG_CHRONGEAR])
+def test_staged_matvec_equals_per_node(ctx, variant, mixed):
+    """The staged Krylov matvec against the per-node kernels: the same
+    arithmetic in the same order, so bitwise the same solves; also a batch
+    whose instances end at different iterations."""
+    groups = [[m] for m in _staged_models()]
+    groups.append([configs.slab(n=64).copy(pcg_maxiters=40, maxiter_nonlinear=3),
+                   configs.dome(n=31, nz=11).copy(pcg_maxiters=12, maxiter_nonlinear=2),
+                   configs.slab(n=50).copy(pcg_maxiters=7, maxiter_nonlinear=4)])
+    for i, ms in enumerate(groups):
+        pc = (configs.PRECOND_SIA, configs.PRECOND_DIAG)[i % 2]
+        ms = [m.copy(which_sparse=variant, which_precond=pc, pcg_tol=1e-6) for m in ms]
+        preps = [solver.prepare(m, precision=solver.MIXED if mixed else solver.FP64)[0] for m in ms]
+        zero = [np.zeros(m.vshape3) for m in ms]
+        got = []
+        for config in ("0,0,0,0,0", "0,0,0,0,1", "0,0,0,37,1"):
+            with _Env(BP_MV_CONFIG=config):
+                prob = ctx.problem(preps)
+                prob.set_guess(zero, zero)
+                prob.run()
+                st = prob.run()
+                u, v, _ = prob.get()
+                prob.close()
+            got.append((u, v, st))
+        keys = ("status", "picard_iters", "pcg_iters_total", "refine_steps_total", "pcg_err_last", "L2_norm")
+        for other in got[1:]:
+            for a, b in zip(got[0][:2], other[:2]):
+                assert all(np.array_equal(x, y) for x, y in zip(a, b)), ms[0].name
+            for s, r in zip(got[0][2], other[2]):
+                assert {k: s[k] for k in keys} == {k: r[k] for k in keys}, ms[0].name
