@@ -154,42 +154,83 @@ __device__ __forceinline__ bool tap_pixel(int b, int y, int x, int dy, int dx, i
   return true;
 }
 
-__global__ void k_im2col(const bf16* __restrict__ X, bf16* __restrict__ col, int B, int H, int W, int C,
-                         int Kp, int periodic) {
-  const long long total = (long long)B * H * W * Kp;
-  for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < total;
-       id += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(id % Kp);
-    const long long p = id / Kp;
-    bf16 val = __float2bfloat16(0.f);
-    if (k < 9 * C) {
-      const int tap = k / C, c = k - tap * C;
-      const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((long long)W * H));
-      long long q;
-      if (tap_pixel(b, y, x, tap / 3 - 1, tap % 3 - 1, H, W, periodic, &q)) val = X[q * C + c];
-    }
-    col[id] = val;
+// im2col of channel counts that are multiples of 8: one thread per (pixel, 8
+// channels) copies the nine taps' 16 bytes, so that the index arithmetic (one
+// division chain) is spent once per 288 bytes and not per 2-byte element.
+// Bound by the 18 C bytes written per pixel: 131,072 pixels of 32 channels
+// 25 us (256 us element by element).
+__global__ void __launch_bounds__(256) k_im2col8(const uint4* __restrict__ X, uint4* __restrict__ col, unsigned P,
+                                                 int H, int W, unsigned C8, int periodic) {
+  const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned p = id / C8, c = id - p * C8;
+  if (p >= P) return;
+  const unsigned row = p / (unsigned)W;
+  const int x = (int)(p - row * W), b = (int)(row / (unsigned)H), y = (int)(row - (unsigned)b * H);
+  uint4* out = col + (size_t)p * 9 * C8 + c;
+#pragma unroll
+  for (int tap = 0; tap < 9; ++tap) {
+    long long q;
+    uint4 val = make_uint4(0u, 0u, 0u, 0u);
+    if (tap_pixel(b, y, x, tap / 3 - 1, tap % 3 - 1, H, W, periodic, &q)) val = __ldg(X + (size_t)q * C8 + c);
+    out[tap * C8] = val;
+  }
+}
+
+// The same for any C (the network's few input fields): one thread per 8
+// entries of a row, stored as 16 bytes (VEC) where rows allow it.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_im2col_any(const bf16* __restrict__ X, bf16* __restrict__ col, unsigned P,
+                                                    int H, int W, int C, int Kp, int periodic) {
+  const unsigned Kp8 = (unsigned)(Kp + 7) / 8;
+  const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned p = id / Kp8, j = id - p * Kp8;
+  if (p >= P) return;
+  const unsigned row = p / (unsigned)W;
+  const int x = (int)(p - row * W), b = (int)(row / (unsigned)H), y = (int)(row - (unsigned)b * H);
+  __align__(16) bf16 v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int k = (int)(8 * j) + e, tap = k / C;
+    long long q;
+    v[e] = __float2bfloat16(0.f);
+    if (k < 9 * C && tap_pixel(b, y, x, tap / 3 - 1, tap % 3 - 1, H, W, periodic, &q)) v[e] = X[q * C + (k - tap * C)];
+  }
+  bf16* out = col + (size_t)p * Kp + 8 * j;
+  if (VEC) {
+    *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(v);
+  } else {
+    for (int e = 0; e < 8 && (int)(8 * j) + e < Kp; ++e) out[e] = v[e];
   }
 }
 
 // dX[p][c] = sum over taps of dcol[q][tap * C + c], q the pixel whose tap
-// lands on p (gather in tap order).
-__global__ void k_col2im(const float* __restrict__ dcol, float* __restrict__ dX, int B, int H, int W, int C,
-                         int Kp, int periodic) {
-  const long long total = (long long)B * H * W * C;
-  for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < total;
-       id += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(id % C);
-    const long long p = id / C;
-    const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((long long)W * H));
-    float s = 0.f;
-    for (int tap = 0; tap < 9; ++tap) {
-      long long q;
-      if (tap_pixel(b, y, x, -(tap / 3 - 1), -(tap % 3 - 1), H, W, periodic, &q))
-        s += dcol[q * Kp + tap * C + c];
+// lands on p (gather in tap order); V = 4: four channels a thread.
+template <int V>
+__global__ void __launch_bounds__(256) k_col2im(const float* __restrict__ dcol, float* __restrict__ dX, unsigned P,
+                                                int H, int W, unsigned CV, int Kp, int periodic) {
+  const unsigned id = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned p = id / CV, c = id - p * CV;
+  if (p >= P) return;
+  const unsigned row = p / (unsigned)W;
+  const int x = (int)(p - row * W), b = (int)(row / (unsigned)H), y = (int)(row - (unsigned)b * H);
+  float s[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) s[e] = 0.f;
+#pragma unroll
+  for (int tap = 0; tap < 9; ++tap) {
+    long long q;
+    if (!tap_pixel(b, y, x, -(tap / 3 - 1), -(tap % 3 - 1), H, W, periodic, &q)) continue;
+    const float* d = dcol + (size_t)q * Kp + (size_t)(tap * CV + c) * V;
+    if (V == 4) {
+      const float4 g = __ldg(reinterpret_cast<const float4*>(d));
+      s[0] += g.x; s[V > 1 ? 1 : 0] += g.y; s[V > 2 ? 2 : 0] += g.z; s[V > 3 ? 3 : 0] += g.w;
+    } else {
+      s[0] += *d;
     }
-    dX[id] = s;
   }
+  float* out = dX + ((size_t)p * CV + c) * V;
+  if (V == 4) *reinterpret_cast<float4*>(out) = make_float4(s[0], s[V > 1 ? 1 : 0], s[V > 2 ? 2 : 0], s[V > 3 ? 3 : 0]);
+  else *out = s[0];
 }
 
 // [R][Cc] -> [Cc][R] (BF16), 32 x 32 tiles through shared memory.
@@ -220,30 +261,152 @@ __device__ __forceinline__ float gelu_grad(float x) {
 #define GRID_LOOP(id, total) \
   for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < (total); id += (long long)gridDim.x * blockDim.x)
 
+// The pointwise kernels move V consecutive channels a thread: 16 bytes of
+// FP32 (V = 4) or BF16 (V = 8) where the channel counts, slice offsets, row
+// lengths and addresses are multiples of that, single elements (V = 1)
+// otherwise.  Element by element with 64-bit divisions they ran at 0.6-1.3
+// TB/s; each element's arithmetic is the same for every V.
+template <typename T, int V>
+struct alignas(sizeof(T) * V) Pack {
+  T e[V];
+};
+template <typename T, int V>
+__device__ __forceinline__ Pack<T, V> ld_pack(const T* p) {
+  return *reinterpret_cast<const Pack<T, V>*>(p);
+}
+template <typename T, int V>
+__device__ __forceinline__ void st_pack(T* p, const Pack<T, V>& v) {
+  *reinterpret_cast<Pack<T, V>*>(p) = v;
+}
+// id -> (row, first channel) of C channels in groups of V
+struct RowCol {
+  long long p;
+  int c;
+};
+template <int V>
+__device__ __forceinline__ RowCol row_col(long long id, int C) {
+  const unsigned g = (unsigned)C / V;
+  RowCol r;
+  if (id < (1LL << 32)) {
+    const unsigned q = (unsigned)id / g;
+    r.p = q;
+    r.c = (int)((unsigned)id - q * g) * V;
+  } else {
+    r.p = id / g;
+    r.c = (int)(id % g) * V;
+  }
+  return r;
+}
+// pixel p of [B][H][W] -> (b, y, x)
+struct Pix {
+  long long b;
+  int y, x;
+};
+__device__ __forceinline__ Pix pixel(long long p, int H, int W) {
+  Pix r;
+  if (p < (1LL << 32)) {
+    const unsigned row = (unsigned)p / (unsigned)W, b = row / (unsigned)H;
+    r.x = (int)((unsigned)p - row * W);
+    r.y = (int)(row - b * H);
+    r.b = b;
+  } else {
+    r.x = (int)(p % W);
+    r.y = (int)((p / W) % H);
+    r.b = p / ((long long)W * H);
+  }
+  return r;
+}
+
 // Y = act(Z) in BF16 into a channel slice [p][c0 .. c0 + C) of rows of ldy.
-__global__ void k_act(const float* __restrict__ Z, bf16* __restrict__ Y, long long P, int C, int ldy, int c0,
-                      int act) {
-  GRID_LOOP(id, P * C) {
-    const long long p = id / C;
-    const int c = (int)(id % C);
-    const float z = Z[id];
-    Y[p * ldy + c0 + c] = __float2bfloat16(act ? gelu(z) : z);
+template <int V>
+__global__ void __launch_bounds__(256) k_act(const float* __restrict__ Z, bf16* __restrict__ Y, long long P, int C,
+                                             int ldy, int c0, int act) {
+  GRID_LOOP(id, P * C / V) {
+    const RowCol r = row_col<V>(id, C);
+    const Pack<float, V> z = ld_pack<float, V>(Z + id * V);
+    Pack<bf16, V> y;
+#pragma unroll
+    for (int e = 0; e < V; ++e) y.e[e] = __float2bfloat16(act ? gelu(z.e[e]) : z.e[e]);
+    st_pack(Y + r.p * ldy + c0 + r.c, y);
   }
 }
 
 // dZ = dY * act'(Z), dY read from a channel slice of rows of ldd (FP32).
-__global__ void k_act_grad(const float* __restrict__ Z, const float* __restrict__ dY, float* __restrict__ dZ,
-                           long long P, int C, int ldd, int c0, int act) {
-  GRID_LOOP(id, P * C) {
-    const long long p = id / C;
-    const int c = (int)(id % C);
-    const float d = dY[p * ldd + c0 + c];
-    dZ[id] = act ? d * gelu_grad(Z[id]) : d;
+template <int V>
+__global__ void __launch_bounds__(256) k_act_grad(const float* __restrict__ Z, const float* __restrict__ dY,
+                                                  float* __restrict__ dZ, long long P, int C, int ldd, int c0,
+                                                  int act) {
+  GRID_LOOP(id, P * C / V) {
+    const RowCol r = row_col<V>(id, C);
+    const Pack<float, V> d = ld_pack<float, V>(dY + r.p * ldd + c0 + r.c), z = ld_pack<float, V>(Z + id * V);
+    Pack<float, V> o;
+#pragma unroll
+    for (int e = 0; e < V; ++e) o.e[e] = act ? d.e[e] * gelu_grad(z.e[e]) : d.e[e];
+    st_pack(dZ + id * V, o);
   }
 }
 
 __global__ void k_f32_to_bf16(const float* __restrict__ x, bf16* __restrict__ y, long long n) {
   GRID_LOOP(id, n) y[id] = __float2bfloat16(x[id]);
+}
+
+// A layer's backward start in one pass over Z and dY: dZ = dY * act'(Z) in
+// BF16 (the operand of both gradient products) and the column sums of its
+// FP32 values, the bias gradient.  Separately they took a pass each, with dZ
+// written and read twice in FP32.  A block strides over the rows with a fixed
+// group of V channels per thread (256 groups per blockIdx.y) and
+// leaves one partial sum per channel; k_colsum_blocks adds the blocks' in
+// order.
+constexpr int kGradBlocks = 296;
+template <int V>
+__global__ void __launch_bounds__(256) k_act_grad_sum(const float* __restrict__ Z, const float* __restrict__ dY,
+                                                      bf16* __restrict__ dZb, float* __restrict__ part, long long P,
+                                                      int C, int act) {
+  __shared__ Pack<float, V> sm[256];
+  const int ch0 = blockIdx.y * 256 * V, g = min((C - ch0) / V, 256), rows = 256 / g;  // rows in flight per block
+  const int cg = threadIdx.x % g, r0 = threadIdx.x / g;
+  Pack<float, V> s;
+#pragma unroll
+  for (int e = 0; e < V; ++e) s.e[e] = 0.f;
+  if (r0 < rows)
+    for (long long p = (long long)blockIdx.x * rows + r0; p < P; p += (long long)gridDim.x * rows) {
+      const long long o = p * C + ch0 + V * cg;
+      Pack<float, V> d = ld_pack<float, V>(dY + o);
+      if (act) {
+        const Pack<float, V> z = ld_pack<float, V>(Z + o);
+#pragma unroll
+        for (int e = 0; e < V; ++e) d.e[e] = d.e[e] * gelu_grad(z.e[e]);
+      }
+      Pack<bf16, V> b;
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        b.e[e] = __float2bfloat16(d.e[e]);
+        s.e[e] += d.e[e];
+      }
+      st_pack(dZb + o, b);
+    }
+  sm[threadIdx.x] = s;
+  __syncthreads();
+  if (r0 == 0) {
+    for (int r = 1; r < rows; ++r)
+#pragma unroll
+      for (int e = 0; e < V; ++e) s.e[e] += sm[r * g + cg].e[e];
+    st_pack(part + (size_t)blockIdx.x * C + ch0 + V * cg, s);
+  }
+}
+__global__ void __launch_bounds__(256) k_colsum_blocks(const float* __restrict__ part, float* __restrict__ db,
+                                                       int blocks, int C) {
+  __shared__ float sm[8][33];
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  float s = 0.f;
+  if (c < C)
+    for (int b = threadIdx.y; b < blocks; b += 8) s += part[(size_t)b * C + c];
+  sm[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && c < C) {
+    for (int r = 1; r < 8; ++r) s += sm[r][threadIdx.x];
+    db[c] = s;
+  }
 }
 
 // Column sums db[c] = sum_p dZ[p][c] (fixed order: one thread per column
@@ -263,77 +426,97 @@ __global__ void k_colsum(const float* __restrict__ dZ, float* __restrict__ db, l
 }
 
 // 2 x 2 average pooling, [B][H][W][C] -> [B][H/2][W/2][C] (BF16).
-__global__ void k_pool(const bf16* __restrict__ X, bf16* __restrict__ Y, int B, int H, int W, int C) {
+template <int V>
+__global__ void __launch_bounds__(256) k_pool(const bf16* __restrict__ X, bf16* __restrict__ Y, int B, int H, int W,
+                                              int C) {
   const int h = H / 2, w = W / 2;
-  GRID_LOOP(id, (long long)B * h * w * C) {
-    const int c = (int)(id % C);
-    const long long p = id / C;
-    const int x = (int)(p % w), y = (int)((p / w) % h), b = (int)(p / ((long long)w * h));
-    const long long q = ((long long)b * H + 2 * y) * W + 2 * x;
-    const float s = __bfloat162float(X[q * C + c]) + __bfloat162float(X[(q + 1) * C + c]) +
-                    __bfloat162float(X[(q + W) * C + c]) + __bfloat162float(X[(q + W + 1) * C + c]);
-    Y[id] = __float2bfloat16(0.25f * s);
+  GRID_LOOP(id, (long long)B * h * w * C / V) {
+    const RowCol r = row_col<V>(id, C);
+    const Pix x = pixel(r.p, h, w);
+    const long long q = (x.b * H + 2 * x.y) * W + 2 * x.x;
+    const Pack<bf16, V> a = ld_pack<bf16, V>(X + q * C + r.c), b = ld_pack<bf16, V>(X + (q + 1) * C + r.c),
+                        c = ld_pack<bf16, V>(X + (q + W) * C + r.c), d = ld_pack<bf16, V>(X + (q + W + 1) * C + r.c);
+    Pack<bf16, V> y;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const float s = __bfloat162float(a.e[e]) + __bfloat162float(b.e[e]) + __bfloat162float(c.e[e]) +
+                      __bfloat162float(d.e[e]);
+      y.e[e] = __float2bfloat16(0.25f * s);
+    }
+    st_pack(Y + id * V, y);
   }
 }
 
 // gradient of the pooling: dX[fine] += dY[coarse] / 4 (FP32, channel slice
 // of the coarse rows)
-__global__ void k_pool_grad(const float* __restrict__ dY, float* __restrict__ dX, int B, int H, int W, int C,
-                            int ldy, int c0) {
-  GRID_LOOP(id, (long long)B * H * W * C) {
-    const int c = (int)(id % C);
-    const long long p = id / C;
-    const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((long long)W * H));
-    const long long q = ((long long)b * (H / 2) + y / 2) * (W / 2) + x / 2;
-    dX[id] += 0.25f * dY[q * ldy + c0 + c];
+template <int V>
+__global__ void __launch_bounds__(256) k_pool_grad(const float* __restrict__ dY, float* __restrict__ dX, int B, int H,
+                                                   int W, int C, int ldy, int c0) {
+  GRID_LOOP(id, (long long)B * H * W * C / V) {
+    const RowCol r = row_col<V>(id, C);
+    const Pix x = pixel(r.p, H, W);
+    const long long q = (x.b * (H / 2) + x.y / 2) * (W / 2) + x.x / 2;
+    const Pack<float, V> d = ld_pack<float, V>(dY + q * ldy + c0 + r.c);
+    Pack<float, V> o = ld_pack<float, V>(dX + id * V);
+#pragma unroll
+    for (int e = 0; e < V; ++e) o.e[e] += 0.25f * d.e[e];
+    st_pack(dX + id * V, o);
   }
 }
 
 // nearest 2x upsampling of [B][h][w][C] into a channel slice of the fine
 // rows (ldy)
-__global__ void k_up(const bf16* __restrict__ X, bf16* __restrict__ Y, int B, int h, int w, int C, int ldy,
-                     int c0) {
+template <int V>
+__global__ void __launch_bounds__(256) k_up(const bf16* __restrict__ X, bf16* __restrict__ Y, int B, int h, int w,
+                                            int C, int ldy, int c0) {
   const int H = 2 * h, W = 2 * w;
-  GRID_LOOP(id, (long long)B * H * W * C) {
-    const int c = (int)(id % C);
-    const long long p = id / C;
-    const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((long long)W * H));
-    const long long q = ((long long)b * h + y / 2) * w + x / 2;
-    Y[p * ldy + c0 + c] = X[q * C + c];
+  GRID_LOOP(id, (long long)B * H * W * C / V) {
+    const RowCol r = row_col<V>(id, C);
+    const Pix x = pixel(r.p, H, W);
+    const long long q = (x.b * h + x.y / 2) * w + x.x / 2;
+    st_pack(Y + r.p * ldy + c0 + r.c, ld_pack<bf16, V>(X + q * C + r.c));
   }
 }
 
 // gradient of the upsampling: dX[coarse] = sum of its 4 fine pixels (fixed order)
-__global__ void k_up_grad(const float* __restrict__ dY, float* __restrict__ dX, int B, int h, int w, int C,
-                          int ldy, int c0) {
+template <int V>
+__global__ void __launch_bounds__(256) k_up_grad(const float* __restrict__ dY, float* __restrict__ dX, int B, int h,
+                                                 int w, int C, int ldy, int c0) {
   const int W = 2 * w;
-  GRID_LOOP(id, (long long)B * h * w * C) {
-    const int c = (int)(id % C);
-    const long long p = id / C;
-    const int x = (int)(p % w), y = (int)((p / w) % h), b = (int)(p / ((long long)w * h));
-    const long long q = ((long long)b * 2 * h + 2 * y) * W + 2 * x;
-    dX[id] = dY[q * ldy + c0 + c] + dY[(q + 1) * ldy + c0 + c] + dY[(q + W) * ldy + c0 + c] +
-             dY[(q + W + 1) * ldy + c0 + c];
+  GRID_LOOP(id, (long long)B * h * w * C / V) {
+    const RowCol r = row_col<V>(id, C);
+    const Pix x = pixel(r.p, h, w);
+    const float* q = dY + ((x.b * 2 * h + 2 * x.y) * W + 2 * x.x) * ldy + c0 + r.c;
+    const Pack<float, V> a = ld_pack<float, V>(q), b = ld_pack<float, V>(q + ldy),
+                         c = ld_pack<float, V>(q + (long long)W * ldy), d = ld_pack<float, V>(q + (long long)(W + 1) * ldy);
+    Pack<float, V> o;
+#pragma unroll
+    for (int e = 0; e < V; ++e) o.e[e] = a.e[e] + b.e[e] + c.e[e] + d.e[e];
+    st_pack(dX + id * V, o);
   }
 }
 
 // copy a BF16 [P][C] block into a channel slice of rows of ldy
-__global__ void k_copy_slice(const bf16* __restrict__ X, bf16* __restrict__ Y, long long P, int C, int ldy,
-                             int c0) {
-  GRID_LOOP(id, P * C) {
-    const long long p = id / C;
-    const int c = (int)(id % C);
-    Y[p * ldy + c0 + c] = X[id];
+template <int V>
+__global__ void __launch_bounds__(256) k_copy_slice(const bf16* __restrict__ X, bf16* __restrict__ Y, long long P,
+                                                    int C, int ldy, int c0) {
+  GRID_LOOP(id, P * C / V) {
+    const RowCol r = row_col<V>(id, C);
+    st_pack(Y + r.p * ldy + c0 + r.c, ld_pack<bf16, V>(X + id * V));
   }
 }
 
 // dX += a channel slice of dY (FP32)
-__global__ void k_add_slice(const float* __restrict__ dY, float* __restrict__ dX, long long P, int C, int ldy,
-                            int c0) {
-  GRID_LOOP(id, P * C) {
-    const long long p = id / C;
-    const int c = (int)(id % C);
-    dX[id] += dY[p * ldy + c0 + c];
+template <int V>
+__global__ void __launch_bounds__(256) k_add_slice(const float* __restrict__ dY, float* __restrict__ dX, long long P,
+                                                   int C, int ldy, int c0) {
+  GRID_LOOP(id, P * C / V) {
+    const RowCol r = row_col<V>(id, C);
+    const Pack<float, V> d = ld_pack<float, V>(dY + r.p * ldy + c0 + r.c);
+    Pack<float, V> o = ld_pack<float, V>(dX + id * V);
+#pragma unroll
+    for (int e = 0; e < V; ++e) o.e[e] += d.e[e];
+    st_pack(dX + id * V, o);
   }
 }
 
@@ -387,6 +570,16 @@ __global__ void k_unpad(const float* __restrict__ src, float* __restrict__ dst, 
     const int k = (int)(id % K);
     dst[id] = src[r * Kp + k];
   }
+}
+
+inline bool aligned(const void* p, unsigned n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; }
+// whether the channel-slice kernels may move 16 bytes a thread: 8 BF16 or 4
+// FP32 channels
+inline bool vec8(int C, int ld, int c0, const void* a, const void* b) {
+  return C % 8 == 0 && ld % 8 == 0 && c0 % 8 == 0 && aligned(a, 16) && aligned(b, 16);
+}
+inline bool vec4(int C, int ld, int c0, const void* a, const void* b) {
+  return C % 4 == 0 && ld % 4 == 0 && c0 % 4 == 0 && aligned(a, 16) && aligned(b, 16);
 }
 
 inline unsigned grid_for(long long n) {
@@ -927,14 +1120,39 @@ int bpnet_gemm_status(void* stream) {
 }
 
 int bpnet_im2col(const void* X, void* col, int B, int H, int W, int C, int Kp, int periodic, void* stream) {
-  const long long n = (long long)B * H * W * Kp;
-  k_im2col<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const bf16*)X, (bf16*)col, B, H, W, C, Kp, periodic);
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool v8 = C % 8 == 0 && Kp == 9 * C && aligned(X, 16) && aligned(col, 16);
+  const bool vec = Kp % 8 == 0 && aligned(col, 16);
+  // images per launch: thread numbers fit 32 bits
+  const long long per = (long long)H * W * (v8 ? C / 8 : (Kp + 7) / 8);
+  if (per <= 0) return cudaGetLastError() == cudaSuccess ? 0 : 6;
+  const int nb = (int)std::max(1LL, std::min((long long)B, (1LL << 31) / per));
+  for (int b0 = 0; b0 < B; b0 += nb) {
+    const unsigned P = (unsigned)((long long)std::min(nb, B - b0) * H * W);
+    const bf16* x = (const bf16*)X + (size_t)b0 * H * W * C;
+    bf16* o = (bf16*)col + (size_t)b0 * H * W * Kp;
+    const unsigned blocks = (unsigned)(((long long)P * (v8 ? C / 8 : (Kp + 7) / 8) + 255) / 256);
+    if (v8) k_im2col8<<<blocks, 256, 0, st>>>((const uint4*)x, (uint4*)o, P, H, W, C / 8, periodic);
+    else if (vec) k_im2col_any<true><<<blocks, 256, 0, st>>>(x, o, P, H, W, C, Kp, periodic);
+    else k_im2col_any<false><<<blocks, 256, 0, st>>>(x, o, P, H, W, C, Kp, periodic);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
 int bpnet_col2im(const float* dcol, float* dX, int B, int H, int W, int C, int Kp, int periodic, void* stream) {
-  const long long n = (long long)B * H * W * C;
-  k_col2im<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(dcol, dX, B, H, W, C, Kp, periodic);
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool v4 = C % 4 == 0 && Kp % 4 == 0 && aligned(dcol, 16) && aligned(dX, 16);
+  const long long per = (long long)H * W * (v4 ? C / 4 : C);
+  if (per <= 0) return cudaGetLastError() == cudaSuccess ? 0 : 6;
+  const int nb = (int)std::max(1LL, std::min((long long)B, (1LL << 31) / per));
+  for (int b0 = 0; b0 < B; b0 += nb) {
+    const unsigned P = (unsigned)((long long)std::min(nb, B - b0) * H * W);
+    const float* d = dcol + (size_t)b0 * H * W * Kp;
+    float* o = dX + (size_t)b0 * H * W * C;
+    const unsigned blocks = (unsigned)(((long long)P * (v4 ? C / 4 : C) + 255) / 256);
+    if (v4) k_col2im<4><<<blocks, 256, 0, st>>>(d, o, P, H, W, C / 4, Kp, periodic);
+    else k_col2im<1><<<blocks, 256, 0, st>>>(d, o, P, H, W, C, Kp, periodic);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
@@ -945,13 +1163,37 @@ int bpnet_transpose(const void* in, void* out, int R, int Cc, void* stream) {
 }
 
 int bpnet_act(const float* Z, void* Y, long long P, int C, int ldy, int c0, int act, void* stream) {
-  k_act<<<grid_for(P * C), 256, 0, (cudaStream_t)stream>>>(Z, (bf16*)Y, P, C, ldy, c0, act);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (C % 4 == 0 && ldy % 4 == 0 && c0 % 4 == 0 && aligned(Z, 16) && aligned(Y, 8))
+    k_act<4><<<grid_for(P * C / 4), 256, 0, st>>>(Z, (bf16*)Y, P, C, ldy, c0, act);
+  else
+    k_act<1><<<grid_for(P * C), 256, 0, st>>>(Z, (bf16*)Y, P, C, ldy, c0, act);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
 int bpnet_act_grad(const float* Z, const float* dY, float* dZ, long long P, int C, int ldd, int c0, int act,
                    void* stream) {
-  k_act_grad<<<grid_for(P * C), 256, 0, (cudaStream_t)stream>>>(Z, dY, dZ, P, C, ldd, c0, act);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (C % 4 == 0 && ldd % 4 == 0 && c0 % 4 == 0 && aligned(Z, 16) && aligned(dY, 16) && aligned(dZ, 16))
+    k_act_grad<4><<<grid_for(P * C / 4), 256, 0, st>>>(Z, dY, dZ, P, C, ldd, c0, act);
+  else
+    k_act_grad<1><<<grid_for(P * C), 256, 0, st>>>(Z, dY, dZ, P, C, ldd, c0, act);
+  return cudaGetLastError() == cudaSuccess ? 0 : 6;
+}
+
+// dZ in BF16 and its column sums db [C] in one pass (dY [P][C], part: 296 C
+// floats of scratch).
+int bpnet_act_grad_sum(const float* Z, const float* dY, void* dZb, float* db, float* part, long long P, int C,
+                       int act, void* stream) {
+  if (C <= 0) return 10;
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool v4 = C % 4 == 0 && aligned(Z, 16) && aligned(dY, 16) && aligned(dZb, 8) && aligned(part, 16);
+  const int per = std::min(v4 ? C / 4 : C, 256), rows = 256 / per;
+  const int blocks = (int)std::max(1LL, std::min((long long)kGradBlocks, (P + rows - 1) / rows));
+  const dim3 grid(blocks, ((v4 ? C / 4 : C) + 255) / 256);
+  if (v4) k_act_grad_sum<4><<<grid, 256, 0, st>>>(Z, dY, (bf16*)dZb, part, P, C, act);
+  else k_act_grad_sum<1><<<grid, 256, 0, st>>>(Z, dY, (bf16*)dZb, part, P, C, act);
+  k_colsum_blocks<<<(C + 31) / 32, dim3(32, 8), 0, st>>>(part, db, blocks, C);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
@@ -967,36 +1209,52 @@ int bpnet_colsum(const float* dZ, float* db, long long P, int C, void* stream) {
 
 int bpnet_pool(const void* X, void* Y, int B, int H, int W, int C, void* stream) {
   if ((H % 2) || (W % 2)) return 10;
+  cudaStream_t st = (cudaStream_t)stream;
   const long long n = (long long)B * (H / 2) * (W / 2) * C;
-  k_pool<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const bf16*)X, (bf16*)Y, B, H, W, C);
+  if (C % 8 == 0 && aligned(X, 16) && aligned(Y, 16))
+    k_pool<8><<<grid_for(n / 8), 256, 0, st>>>((const bf16*)X, (bf16*)Y, B, H, W, C);
+  else
+    k_pool<1><<<grid_for(n), 256, 0, st>>>((const bf16*)X, (bf16*)Y, B, H, W, C);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
 int bpnet_pool_grad(const float* dY, float* dX, int B, int H, int W, int C, int ldy, int c0, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
   const long long n = (long long)B * H * W * C;
-  k_pool_grad<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(dY, dX, B, H, W, C, ldy, c0);
+  if (vec4(C, ldy, c0, dY, dX)) k_pool_grad<4><<<grid_for(n / 4), 256, 0, st>>>(dY, dX, B, H, W, C, ldy, c0);
+  else k_pool_grad<1><<<grid_for(n), 256, 0, st>>>(dY, dX, B, H, W, C, ldy, c0);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
 int bpnet_up(const void* X, void* Y, int B, int h, int w, int C, int ldy, int c0, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
   const long long n = (long long)B * 4 * h * w * C;
-  k_up<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>((const bf16*)X, (bf16*)Y, B, h, w, C, ldy, c0);
+  if (vec8(C, ldy, c0, X, Y)) k_up<8><<<grid_for(n / 8), 256, 0, st>>>((const bf16*)X, (bf16*)Y, B, h, w, C, ldy, c0);
+  else k_up<1><<<grid_for(n), 256, 0, st>>>((const bf16*)X, (bf16*)Y, B, h, w, C, ldy, c0);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
 int bpnet_up_grad(const float* dY, float* dX, int B, int h, int w, int C, int ldy, int c0, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
   const long long n = (long long)B * h * w * C;
-  k_up_grad<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(dY, dX, B, h, w, C, ldy, c0);
+  if (vec4(C, ldy, c0, dY, dX)) k_up_grad<4><<<grid_for(n / 4), 256, 0, st>>>(dY, dX, B, h, w, C, ldy, c0);
+  else k_up_grad<1><<<grid_for(n), 256, 0, st>>>(dY, dX, B, h, w, C, ldy, c0);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
 int bpnet_copy_slice(const void* X, void* Y, long long P, int C, int ldy, int c0, void* stream) {
-  k_copy_slice<<<grid_for(P * C), 256, 0, (cudaStream_t)stream>>>((const bf16*)X, (bf16*)Y, P, C, ldy, c0);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (vec8(C, ldy, c0, X, Y))
+    k_copy_slice<8><<<grid_for(P * C / 8), 256, 0, st>>>((const bf16*)X, (bf16*)Y, P, C, ldy, c0);
+  else
+    k_copy_slice<1><<<grid_for(P * C), 256, 0, st>>>((const bf16*)X, (bf16*)Y, P, C, ldy, c0);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
 int bpnet_add_slice(const float* dY, float* dX, long long P, int C, int ldy, int c0, void* stream) {
-  k_add_slice<<<grid_for(P * C), 256, 0, (cudaStream_t)stream>>>(dY, dX, P, C, ldy, c0);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (vec4(C, ldy, c0, dY, dX)) k_add_slice<4><<<grid_for(P * C / 4), 256, 0, st>>>(dY, dX, P, C, ldy, c0);
+  else k_add_slice<1><<<grid_for(P * C), 256, 0, st>>>(dY, dX, P, C, ldy, c0);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 

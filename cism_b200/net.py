@@ -50,6 +50,7 @@ def lib():
             "bpnet_transpose": [vp, vp, i, i, vp],
             "bpnet_act": [vp, vp, ll, i, i, i, i, vp],
             "bpnet_act_grad": [vp, vp, vp, ll, i, i, i, i, vp],
+            "bpnet_act_grad_sum": [vp, vp, vp, vp, vp, ll, i, i, vp],
             "bpnet_to_bf16": [vp, vp, ll, vp],
             "bpnet_colsum": [vp, vp, ll, i, vp],
             "bpnet_pool": [vp, vp, i, i, i, i, vp],
@@ -125,10 +126,11 @@ def transpose(x, ldo: Optional[int] = None):
     torch = _torch()
     R, Cc = x.shape
     ldo = ldo or R
-    out = torch.zeros((Cc, ldo), dtype=torch.bfloat16, device=x.device)
     if ldo == R:
+        out = torch.empty((Cc, ldo), dtype=torch.bfloat16, device=x.device)
         _ck(lib().bpnet_transpose(_p(x), _p(out), R, Cc, _s()), "bpnet_transpose")
     else:
+        out = torch.zeros((Cc, ldo), dtype=torch.bfloat16, device=x.device)
         tmp = torch.empty((Cc, R), dtype=torch.bfloat16, device=x.device)
         _ck(lib().bpnet_transpose(_p(x), _p(tmp), R, Cc, _s()), "bpnet_transpose")
         out[:, :R].copy_(tmp)
@@ -184,13 +186,11 @@ class Conv:
         torch = _torch()
         col, z, (B, H, W), periodic = self.saved
         P = B * H * W
-        dz = torch.empty((P, self.cout), dtype=torch.float32, device=dy.device)
-        _ck(lib().bpnet_act_grad(_p(z), _p(dy), _p(dz), P, self.cout, self.cout, 0, int(self.act), _s()),
-            "act_grad")
         self.gb = torch.empty(self.cout, dtype=torch.float32, device=dy.device)
-        _ck(lib().bpnet_colsum(_p(dz), _p(self.gb), P, self.cout, _s()), "colsum")
         dzb = torch.empty((P, self.cout), dtype=torch.bfloat16, device=dy.device)
-        _ck(lib().bpnet_to_bf16(_p(dz), _p(dzb), P * self.cout, _s()), "to_bf16")
+        part = torch.empty(296 * self.cout, dtype=torch.float32, device=dy.device)
+        _ck(lib().bpnet_act_grad_sum(_p(z), _p(dy), _p(dzb), _p(self.gb), _p(part), P, self.cout, int(self.act),
+                                     _s()), "act_grad_sum")
         P8 = ceil8(P)
         dzt = transpose(dzb, P8)
         colt = transpose(col, P8)

@@ -214,3 +214,95 @@ def test_shipped_network_reduces_iterations_on_held_out_slab(ctx):
     assert st1["picard_iters"] < st0["picard_iters"]
     assert st1["pcg_iters_total"] < 0.8 * st0["pcg_iters_total"]
     assert rel_l2([u1, v1], [u0, v0]) < 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("shape", [(1, 2, 2, 8), (2, 6, 10, 6), (1, 4, 34, 24), (3, 8, 2, 33), (1, 2, 6, 1032)])
+def test_pointwise_kernels_match_torch(shape, offset):
+    """The 16-byte forms and the element forms (channel counts that are not
+    multiples of 4 or 8; addresses one element past a 16-byte boundary) of the
+    data-movement and pointwise kernels.  Copies and sums of at most nine terms
+    in the kernels' order: equal bit for bit; GELU and its gradient to 4 ulp of
+    FP32 before the BF16 rounding (one BF16 ulp, 2^-8); column sums of N terms
+    in FP32 to N 2^-24 of the sum of magnitudes."""
+    torch = pytest.importorskip("torch")
+    from cism_b200 import net as netmod
+
+    L = netmod.lib()
+    B, H, W, C = shape
+    P = B * H * W
+    g = torch.Generator(device="cuda").manual_seed(P + C)
+
+    def rand(*n, dtype=torch.float32):
+        buf = torch.randn(int(np.prod(n)) + 8, generator=g, device="cuda").to(dtype)
+        return buf[offset:offset + int(np.prod(n))].view(*n)
+
+    def new(*n, dtype=torch.float32):
+        buf = torch.full((int(np.prod(n)) + 8,), float("nan"), device="cuda").to(dtype)
+        return buf[offset:offset + int(np.prod(n))].view(*n)
+
+    bf = torch.bfloat16
+    s = netmod._s()
+    p = netmod._p
+    x = rand(B, H, W, C, dtype=bf)
+    for periodic in (0, 1):
+        Kp = netmod.ceil8(9 * C)
+        col = new(P, Kp, dtype=bf)
+        assert L.bpnet_im2col(p(x), p(col), B, H, W, C, Kp, periodic, s) == 0
+        pad = torch.nn.functional.pad(x.float().permute(0, 3, 1, 2), (1, 1, 1, 1),
+                                      mode="circular" if periodic else "constant")
+        ref = torch.stack([pad[:, :, dy:dy + H, dx:dx + W] for dy in range(3) for dx in range(3)], 1)
+        ref = ref.permute(0, 3, 4, 1, 2).reshape(P, 9 * C).to(bf)
+        assert torch.equal(col[:, :9 * C], ref) and not bool((col[:, 9 * C:] != 0).any())
+        d = rand(P, 9 * C)
+        dx_ = new(B, H, W, C)
+        assert L.bpnet_col2im(p(d), p(dx_), B, H, W, C, 9 * C, periodic, s) == 0
+        dd = d.view(B, H, W, 9, C)
+        acc = torch.zeros(B, H, W, C, device="cuda")
+        for tap in range(9):
+            ty, tx = tap // 3 - 1, tap % 3 - 1
+            r = torch.roll(dd[..., tap, :], (ty, tx), (1, 2))
+            if not periodic:
+                r = r.clone()
+                if ty: r[:, 0 if ty > 0 else H - 1] = 0
+                if tx: r[:, :, 0 if tx > 0 else W - 1] = 0
+            acc = acc + r
+        assert torch.equal(dx_, acc)
+    z, dy = rand(P, C), rand(P, C)
+    y = new(P, C + 8, dtype=bf)
+    assert L.bpnet_act(p(z), p(y), P, C, C + 8, 8, 1, s) == 0
+    ref = torch.nn.functional.gelu(z.double())
+    assert bool(((y[:, 8:].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-7).all())
+    dz, dzb, db, part = new(P, C), new(P, C, dtype=bf), new(C), new(296 * C)
+    assert L.bpnet_act_grad(p(z), p(dy), p(dz), P, C, C, 0, 1, s) == 0
+    assert L.bpnet_act_grad_sum(p(z), p(dy), p(dzb), p(db), p(part), P, C, 1, s) == 0
+    assert torch.equal(dzb, dz.to(bf))
+    mag = dz.double().abs().sum(0)
+    assert bool(((db.double() - dz.double().sum(0)).abs() <= (P + 8) * 2.0 ** -24 * mag).all())
+    c2 = new(B, H // 2, W // 2, C, dtype=bf)
+    assert L.bpnet_pool(p(x), p(c2), B, H, W, C, s) == 0
+    f = x.float()
+    ref = f[:, ::2, ::2] + f[:, ::2, 1::2]
+    ref = 0.25 * ((ref + f[:, 1::2, ::2]) + f[:, 1::2, 1::2])
+    assert torch.equal(c2, ref.to(bf))
+    cat = new(P, C + 8, dtype=bf)
+    assert L.bpnet_up(p(c2), p(cat), B, H // 2, W // 2, C, C + 8, 0, s) == 0
+    up = c2.repeat_interleave(2, 1).repeat_interleave(2, 2).reshape(P, C)
+    assert torch.equal(cat[:, :C], up)
+    assert L.bpnet_copy_slice(p(x), p(cat), P, C, C + 8, 8, s) == 0
+    assert torch.equal(cat[:, 8:], x.reshape(P, C))
+    dcat, a = rand(P, C + 8), rand(P, C)
+    b = a.clone() if offset == 0 else new(P, C)
+    b.copy_(a)
+    assert L.bpnet_add_slice(p(dcat), p(b), P, C, C + 8, 8, s) == 0
+    assert torch.equal(b, a + dcat[:, 8:])
+    ug = new(B, H // 2, W // 2, C)
+    assert L.bpnet_up_grad(p(dcat), p(ug), B, H // 2, W // 2, C, C + 8, 0, s) == 0
+    q = dcat[:, :C].reshape(B, H, W, C)
+    assert torch.equal(ug, ((q[:, ::2, ::2] + q[:, ::2, 1::2]) + q[:, 1::2, ::2]) + q[:, 1::2, 1::2])
+    pg = new(B, H, W, C)
+    pg.copy_(a.view(B, H, W, C))
+    assert L.bpnet_pool_grad(p(ug), p(pg), B, H, W, C, C, 0, s) == 0
+    assert torch.equal(pg, a.view(B, H, W, C) + 0.25 * ug.repeat_interleave(2, 1).repeat_interleave(2, 2))
+    torch.cuda.synchronize()
