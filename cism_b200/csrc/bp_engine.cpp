@@ -69,6 +69,38 @@ struct Arena {
   }
 };
 
+// A host buffer that copies to and from the device go through, kept by its
+// context and only growing: page-locked, so that a copy runs at the link's
+// rate, and not fresh memory whose pages are first touched in every call.
+// Pageable where no page-locked memory is left.
+struct Staging {
+  void* p = nullptr;
+  size_t bytes = 0;
+  bool pinned = false;
+  template <typename T>
+  T* get(cudaStream_t s, size_t count) {
+    const size_t need = std::max<size_t>(count, 1) * sizeof(T);
+    if (need > bytes) {
+      CK(cudaStreamSynchronize(s));  // no copy in flight uses the old one
+      release();
+      pinned = cudaMallocHost(&p, need) == cudaSuccess;
+      if (!pinned) {
+        cudaGetLastError();
+        p = std::malloc(need);
+        if (!p) throw CudaError{cudaErrorMemoryAllocation, "host staging buffer"};
+      }
+      bytes = need;
+    }
+    return static_cast<T*>(p);
+  }
+  void release() {
+    if (p && pinned) cudaFreeHost(p);
+    else std::free(p);
+    p = nullptr;
+    bytes = 0;
+  }
+};
+
 // Event pairs around kernel launches, by category.
 struct Timing {
   bool on = false;
@@ -93,6 +125,7 @@ struct bp_ctx {
   cudaStream_t stream = nullptr;
   std::string err;
   Arena arena;                     // for the one-shot entry points
+  Staging staging;                 // calls on a context are serial and end synchronised
   bp::Counters* h_cnt = nullptr;   // pinned, 2 slots
   cudaEvent_t ev[2] = {nullptr, nullptr};
   cudaEvent_t t0 = nullptr, t1 = nullptr, t2 = nullptr, t3 = nullptr;
@@ -917,14 +950,34 @@ void problem_free(bp_problem* P) {
 }
 
 void problem_set_guess(bp_problem* P, double* const* uvel, double* const* vvel) {
-  std::vector<double2> x(P->plan.npad, double2{0.0, 0.0});
+  const HostPlan& p = P->plan;
+  cudaStream_t s = P->c->stream;
   std::vector<int> learned;
-  for (int b = 0; b < P->plan.ninst; ++b) {
-    if (P->plan.guess_mode[b] == BP_GUESS_LEARNED) learned.push_back(b);
-    else gather_velocity(P->plan, b, uvel[b], vvel[b], x.data());
+  for (int b = 0; b < p.ninst; ++b)
+    if (p.guess_mode[b] == BP_GUESS_LEARNED) learned.push_back(b);
+  std::vector<double2> x;
+  if (p.solve2d) {
+    x.assign(p.npad, double2{0.0, 0.0});
+    for (int b = 0; b < p.ninst; ++b) gather_velocity(p, b, uvel[b], vvel[b], x.data());
+    CK(cudaMemcpyAsync(P->x0, x.data(), sizeof(double2) * p.npad, cudaMemcpyHostToDevice, s));
+    P->h2d_bytes += sizeof(double2) * (double)p.nnodes;
+  } else if ((int)learned.size() < p.ninst) {  // columns through the staging buffer, nodes on the device
+    const size_t n = (size_t)p.nnodes;
+    double* host = P->c->staging.get<double>(s, 2 * n);
+    double* dev = reinterpret_cast<double*>(P->v.q);  // scratch between runs
+    for (int b = 0; b < p.ninst; ++b) {
+      if (p.guess_mode[b] == BP_GUESS_LEARNED) continue;
+      gather_columns(p, b, uvel[b], vvel[b], host, host + n);
+      const InstParams& ip = p.inst[b];
+      const size_t t0 = (size_t)ip.col_begin * p.nz, len = (size_t)(ip.col_end - ip.col_begin) * p.nz;
+      if (len == 0) continue;
+      for (size_t o : {t0, n + t0})
+        CK(cudaMemcpyAsync(dev + o, host + o, sizeof(double) * len, cudaMemcpyHostToDevice, s));
+      launch_unpack(P->v, ip.col_begin, ip.col_end, dev, dev + n, P->x0, s);
+      P->h2d_bytes += sizeof(double2) * (double)len;
+    }
+    CK(cudaGetLastError());
   }
-  CK(cudaMemcpyAsync(P->x0, x.data(), sizeof(double2) * P->plan.npad, cudaMemcpyHostToDevice, P->c->stream));
-  P->h2d_bytes += sizeof(double2) * (double)P->plan.nnodes;
   if (!learned.empty()) {  // the network's guess straight into x0, on the device
     if (!P->c->net) throw GuessError{"guess_mode = BP_GUESS_LEARNED needs bp_guess_load"};
     if (guess_net_run(P->c->net, P->plan, P->v, learned, P->x0, P->c->stream, &P->c->net_launches) != BP_OK)
@@ -979,11 +1032,19 @@ void problem_get(bp_problem* P, double* const* uvel, double* const* vvel, double
   const HostPlan& p = P->plan;
   // L1L2 and DIVA: the 3-D velocity, else the solution vector
   const bool v3 = p.l1l2 || p.diva;
-  const size_t nx = v3 ? (size_t)p.ncols * p.nz_out : (size_t)p.npad;
-  std::vector<double2> x(std::max<size_t>(nx, 1));
-  if (nx > 0)
-    CK(cudaMemcpyAsync(x.data(), v3 ? P->v.x3 : P->v.x, sizeof(double2) * nx, cudaMemcpyDeviceToHost,
-                       P->c->stream));
+  const bool columns = !p.solve2d;  // the 3-D solve: by columns (launch_pack)
+  const size_t nx = v3 ? (size_t)p.ncols * p.nz_out : columns ? (size_t)p.nnodes : (size_t)p.npad;
+  double* host = P->c->staging.get<double>(P->c->stream, 2 * nx + (efvs ? p.nefvs : 0));
+  double* ef = host + 2 * nx;
+  double2* x = reinterpret_cast<double2*>(host);
+  if (columns) {
+    double* dev = reinterpret_cast<double*>(P->v.q);  // scratch after a run
+    launch_pack(P->v, P->v.x, dev, dev + nx, P->c->stream);
+    CK(cudaGetLastError());
+    if (nx > 0) CK(cudaMemcpyAsync(host, dev, sizeof(double) * 2 * nx, cudaMemcpyDeviceToHost, P->c->stream));
+  } else if (nx > 0) {
+    CK(cudaMemcpyAsync(x, v3 ? P->v.x3 : P->v.x, sizeof(double2) * nx, cudaMemcpyDeviceToHost, P->c->stream));
+  }
   std::vector<double2> x2, bt;  // DIVA: the mean velocity and the traction
   if (p.diva && p.ncols > 0) {  // the mean velocity in node order (col_node), the traction per column
     x2.resize(p.npad);
@@ -991,23 +1052,57 @@ void problem_get(bp_problem* P, double* const* uvel, double* const* vvel, double
     CK(cudaMemcpyAsync(x2.data(), P->v.x, sizeof(double2) * p.npad, cudaMemcpyDeviceToHost, P->c->stream));
     CK(cudaMemcpyAsync(bt.data(), P->v.col_bt, sizeof(double2) * p.ncols, cudaMemcpyDeviceToHost, P->c->stream));
   }
-  std::vector<double> ef;
-  if (efvs) {
-    ef.resize(std::max(p.nefvs, 1));
-    if (p.nefvs > 0)
-      CK(cudaMemcpyAsync(ef.data(), P->v.efvs, sizeof(double) * p.nefvs, cudaMemcpyDeviceToHost, P->c->stream));
-  }
+  if (efvs && p.nefvs > 0)
+    CK(cudaMemcpyAsync(ef, P->v.efvs, sizeof(double) * p.nefvs, cudaMemcpyDeviceToHost, P->c->stream));
   CK(cudaStreamSynchronize(P->c->stream));
   P->d2h_bytes = sizeof(double2) * (double)(v3 ? nx : (size_t)p.nnodes) +
                  (efvs ? sizeof(double) * (double)p.nefvs : 0.0) + sizeof(double2) * 2.0 * (double)bt.size();
   for (int b = 0; b < p.ninst; ++b) {
     if (uvel && vvel) {
-      if (v3) scatter_velocity_3d(p, b, x.data(), uvel[b], vvel[b]);
-      else scatter_velocity(p, b, x.data(), uvel[b], vvel[b]);
+      if (v3) scatter_velocity_3d(p, b, x, uvel[b], vvel[b]);
+      else if (columns) scatter_columns(p, b, host, host + nx, uvel[b], vvel[b]);
+      else scatter_velocity(p, b, x, uvel[b], vvel[b]);
     }
     if (p.diva) scatter_diva(p, b, x2.empty() ? nullptr : x2.data(), bt.empty() ? nullptr : bt.data());
-    if (efvs && efvs[b]) scatter_efvs(p, b, ef.data(), efvs[b]);
+    if (efvs && efvs[b]) scatter_efvs(p, b, ef, efvs[b]);
   }
+}
+
+// A caller's matrix blocks into the full FP64 storage v.A: rows go through the
+// staging buffer (32 MB at a time) and are put in node order on the device.
+void upload_matrix(bp_ctx* c, Arena& a, const DevView& v, const HostPlan& p, const double* const blocks[4]) {
+  cudaStream_t s = c->stream;
+  const long rows = (long)p.nz * (p.nx[0] - 1) * (p.ny[0] - 1);
+  CK(cudaMemsetAsync(v.A, 0, sizeof(double2) * 2 * 27 * (size_t)p.npad, s));
+  std::vector<int> row_node(rows, -1);
+  for (int g = 0; g < p.ncols; ++g) {
+    const long w = ((long)(p.col_ij[p.ncols + g] - 1) * (p.nx[0] - 1) + (p.col_ij[g] - 1)) * p.nz;
+    for (int k = 0; k < p.nz; ++k) row_node[w + k] = (int)node_of(p, g, k);
+  }
+  int* d_node = a.get<int>(s, "matrix_rows", rows);
+  CK(cudaMemcpyAsync(d_node, row_node.data(), sizeof(int) * rows, cudaMemcpyHostToDevice, s));
+  const long chunk = std::min(rows, (32L << 20) / (4 * 27 * (long)sizeof(double)));
+  const size_t part = 4 * 27 * (size_t)chunk;  // doubles of a chunk; two of them take turns
+  double* host = c->staging.get<double>(s, 2 * part);
+  double* dev = a.get<double>(s, "matrix_raw", 2 * part);
+  int turn = 0;
+  for (long r0 = 0; r0 < rows; r0 += chunk, turn ^= 1) {
+    const long n = std::min(chunk, rows - r0);
+    double *h = host + turn * part, *d = dev + turn * part;
+    if (r0 >= 2 * chunk) CK(cudaEventSynchronize(c->ev[turn]));  // the chunk before last has left h
+    parallel_for(4 * (size_t)n, 4096, [&](size_t i0, size_t i1) {
+      for (size_t i = i0; i < i1;) {  // row i % n of block i / n
+        const size_t q = i / n, e = std::min(i1, (q + 1) * n);
+        std::memcpy(h + i * 27, blocks[q] + ((size_t)r0 + i - q * n) * 27, sizeof(double) * 27 * (e - i));
+        i = e;
+      }
+    });
+    CK(cudaMemcpyAsync(d, h, sizeof(double) * 4 * 27 * (size_t)n, cudaMemcpyHostToDevice, s));
+    CK(cudaEventRecord(c->ev[turn], s));
+    launch_gather_matrix(v, d, d_node, r0, n, s);
+  }
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(s));  // row_node is a host temporary; the staging buffer is free again
 }
 
 }  // namespace
@@ -1059,6 +1154,7 @@ int bp_destroy(bp_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->arena.release();
+  c->staging.release();
   if (c->net) guess_net_free(c->net);
   if (c->h_cnt) cudaFreeHost(c->h_cnt);
   for (auto& e : c->ev)
@@ -1123,10 +1219,23 @@ int bp_problem_get_guess(bp_problem* P, double* const* uvel, double* const* vvel
   if (!P) return BP_ERR_ARGS;
   GUARD_BEGIN(P->c)
   if (!uvel || !vvel || P->plan.l1l2 || P->plan.diva) return BP_ERR_ARGS;
-  std::vector<double2> x(P->plan.npad);
-  CK(cudaMemcpyAsync(x.data(), P->x0, sizeof(double2) * P->plan.npad, cudaMemcpyDeviceToHost, P->c->stream));
-  CK(cudaStreamSynchronize(P->c->stream));
-  for (int b = 0; b < P->plan.ninst; ++b) scatter_velocity(P->plan, b, x.data(), uvel[b], vvel[b]);
+  const HostPlan& p = P->plan;
+  cudaStream_t s = P->c->stream;
+  if (p.solve2d) {
+    std::vector<double2> x(p.npad);
+    CK(cudaMemcpyAsync(x.data(), P->x0, sizeof(double2) * p.npad, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    for (int b = 0; b < p.ninst; ++b) scatter_velocity(p, b, x.data(), uvel[b], vvel[b]);
+    return BP_OK;
+  }
+  const size_t n = (size_t)p.nnodes;
+  double* host = P->c->staging.get<double>(s, 2 * n);
+  double* dev = reinterpret_cast<double*>(P->v.q);  // scratch between runs
+  launch_pack(P->v, P->x0, dev, dev + n, s);
+  CK(cudaGetLastError());
+  if (n > 0) CK(cudaMemcpyAsync(host, dev, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  for (int b = 0; b < p.ninst; ++b) scatter_columns(p, b, host, host + n, uvel[b], vvel[b]);
   return BP_OK;
   GUARD_END
 }
@@ -1405,9 +1514,8 @@ int bp_pcg(bp_ctx* c, int nx, int ny, int nz, int periodic,
   P.v = make_view(*P.arena, c->stream, P.plan, false, P.mixed);
   use_resident_pcg(c, *P.arena, &P.v, P.plan);
   const DevView& v = P.v;
-  std::vector<double2> A(2 * 27 * (size_t)P.plan.npad);
-  gather_matrix(P.plan, Auu, Auv, Avu, Avv, A.data());
-  CK(cudaMemcpyAsync(v.A, A.data(), sizeof(double2) * A.size(), cudaMemcpyHostToDevice, c->stream));
+  const double* blocks[4] = {Auu, Auv, Avu, Avv};
+  upload_matrix(c, *P.arena, v, P.plan, blocks);
   std::vector<double2> x(P.plan.npad, double2{0, 0}), b(P.plan.npad, double2{0, 0});
   gather_velocity(P.plan, 0, xu, xv, x.data());
   gather_velocity(P.plan, 0, bu, bv, b.data());
@@ -1445,9 +1553,8 @@ int bp_matvec(bp_ctx* c, int nx, int ny, int nz, int periodic,
     return BP_ERR_ARGS;
   }
   DevView v = make_view(c->arena, c->stream, p, false, false);
-  std::vector<double2> A(2 * 27 * (size_t)p.npad);
-  gather_matrix(p, Auu, Auv, Avu, Avv, A.data());
-  CK(cudaMemcpyAsync(v.A, A.data(), sizeof(double2) * A.size(), cudaMemcpyHostToDevice, c->stream));
+  const double* blocks[4] = {Auu, Auv, Avu, Avv};
+  upload_matrix(c, c->arena, v, p, blocks);
   std::vector<double2> x(p.npad, double2{0, 0});
   gather_velocity(p, 0, xu, xv, x.data());
   CK(cudaMemcpyAsync(v.x, x.data(), sizeof(double2) * p.npad, cudaMemcpyHostToDevice, c->stream));

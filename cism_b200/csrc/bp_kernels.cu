@@ -2384,6 +2384,58 @@ void launch_matvec_plain(const DevView& v, const double2* x, double2* y, cudaStr
 void launch_dinv(const DevView& v, int precond, cudaStream_t s) {
   k_dinv<<<tile_grid(v), v.tile_threads, 0, s>>>(v, precond);
 }
+// Node layout <-> [column][level] in two arrays, the form in which a host
+// array's columns are one copy each.  Bandwidth: 32 bytes a node and way; the
+// strided side (a column's levels are W nodes apart) is served by L1.
+__global__ void __launch_bounds__(256) k_pack(const __grid_constant__ DevView v, const double2* x, double* u, double* w) {
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long)v.ncols * v.nz) return;
+  const int col = (int)(t / v.nz), k = (int)(t - (long)col * v.nz);
+  const double2 a = x[node_of(v, col, k)];
+  u[t] = a.x;
+  w[t] = a.y;
+}
+__global__ void __launch_bounds__(256) k_unpack(const __grid_constant__ DevView v, long t0, long t1, const double* u,
+                                                const double* w, double2* x) {
+  const long t = t0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= t1) return;
+  const int col = (int)(t / v.nz), k = (int)(t - (long)col * v.nz);
+  x[node_of(v, col, k)] = make_double2(u[t], w[t]);
+}
+void launch_pack(const DevView& v, const double2* x, double* u, double* w, cudaStream_t s) {
+  const long n = (long)v.ncols * v.nz;
+  if (n > 0) k_pack<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(v, x, u, w);
+}
+void launch_unpack(const DevView& v, int col_begin, int col_end, const double* u, const double* w, double2* x,
+                   cudaStream_t s) {
+  const long t0 = (long)col_begin * v.nz, t1 = (long)col_end * v.nz;
+  if (t1 > t0) k_unpack<<<(unsigned)((t1 - t0 + 255) / 256), 256, 0, s>>>(v, t0, t1, u, w, x);
+}
+
+// A caller's matrix rows into the node layout, 32 rows (a warp each block) at
+// a time through shared memory: read and written along their own contiguous
+// direction.
+__global__ void __launch_bounds__(128) k_gather_matrix(const __grid_constant__ DevView v, const double* raw,
+                                                       const int* row_node, long row0, long rows) {
+  __shared__ double sm[4][32 * 27 + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;  // warp: block uu, uv, vu, vv
+  const long r0 = (long)blockIdx.x * 32;
+  const int nr = (int)min(32L, rows - r0);
+  const double* src = raw + (size_t)warp * rows * 27 + r0 * 27;
+  for (int e = lane; e < nr * 27; e += 32) sm[warp][e] = src[e];
+  __syncthreads();
+  const int n = lane < nr ? row_node[row0 + r0 + lane] : -1;
+  if (n < 0) return;
+  const size_t np = (size_t)v.npad;
+  // warps 0, 1 the u-row's entries, 2, 3 the v-row's
+  const int h = warp >> 1;
+  for (int m = warp & 1; m < 27; m += 2)
+    v.A[(size_t)(h * 27 + m) * np + n] = make_double2(sm[2 * h][lane * 27 + m], sm[2 * h + 1][lane * 27 + m]);
+}
+void launch_gather_matrix(const DevView& v, const double* raw, const int* row_node, long row0, long rows,
+                          cudaStream_t s) {
+  if (rows > 0) k_gather_matrix<<<(unsigned)((rows + 31) / 32), 128, 0, s>>>(v, raw, row_node, row0, rows);
+}
 void launch_bb(const DevView& v, cudaStream_t s) { k_bb<<<tile_grid(v), v.tile_threads, 0, s>>>(v); }
 // The 3-D velocity of a shallow-shelf solve (its 2-D solution on every
 // level, :3745-3750) for the post-solve diagnostics.

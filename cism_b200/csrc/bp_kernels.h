@@ -63,6 +63,15 @@ void launch_make_a32(const DevView& v, cudaStream_t s);
 // instances that use it, from the assembled matrix.
 void launch_sia_factor(const DevView& v, cudaStream_t s);
 void launch_matvec_plain(const DevView& v, const double2* x, double2* y, cudaStream_t s);
+// x of every node of the columns [col_begin, col_end) <-> u, v [ncols][nz]
+void launch_pack(const DevView& v, const double2* x, double* u, double* w, cudaStream_t s);
+void launch_unpack(const DevView& v, int col_begin, int col_end, const double* u, const double* w, double2* x,
+                   cudaStream_t s);
+// rows [row0, row0 + rows) of a caller's matrix blocks (27 entries a row, row
+// = vertex * nz + level, rows of the blocks one after another in raw) into
+// the full FP64 storage; row_node: each row's node, -1 = none
+void launch_gather_matrix(const DevView& v, const double* raw, const int* row_node, long row0, long rows,
+                          cudaStream_t s);
 void launch_dinv(const DevView& v, int precond, cudaStream_t s);
 void launch_bb(const DevView& v, cudaStream_t s);
 // element stresses into tau[6][nelem] and the basal frictional heat flux

@@ -4,6 +4,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <system_error>
+#include <thread>
 
 namespace bp {
 
@@ -77,6 +79,29 @@ void set_block_width(HostPlan* p) {
 }
 
 }  // namespace
+
+void parallel_for(size_t n, size_t grain, const std::function<void(size_t, size_t)>& f) {
+  const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+  const size_t nt = std::min({(size_t)8, cores, n / std::max<size_t>(grain, 1)});
+  if (nt <= 1) {
+    f(0, n);
+    return;
+  }
+  std::thread th[8];
+  size_t started = 0;
+  const auto part = [&](size_t t) { return n * t / nt; };
+  try {
+    for (size_t t = 1; t < nt; ++t, ++started) th[t] = std::thread(f, part(t), part(t + 1));
+  } catch (const std::system_error&) {
+  }
+  f(0, part(1));
+  if (started + 1 < nt) f(part(started + 1), n);
+  for (size_t t = 1; t <= started; ++t) th[t].join();
+}
+
+// Columns a thread takes at least: below some thousands the threads cost more
+// than they save.
+constexpr size_t kColumnGrain = 4096;
 
 OwnedRange owned_range(int nx, int ny, int periodic) {
   OwnedRange r;
@@ -451,7 +476,8 @@ bool build_plan(const bp_inputs* in, int n, HostPlan* p, std::string* err) {
     ip.cell_begin = cell_base; ip.cell_end = cell_base + ncl;
     const int epc = solve2d ? 1 : nz - 1;  // elements per cell
     ip.elem_begin = cell_base * epc; ip.elem_end = (cell_base + ncl) * epc;
-    for (int c = 0; c < nc; ++c) {
+    parallel_for(nc, kColumnGrain, [&](size_t c_begin, size_t c_end) {
+    for (int c = (int)c_begin; c < (int)c_end; ++c) {
       const int g = col_base + c;
       const int i = cols[b][c].first, j = cols[b][c].second;
       p->col_inst[g] = b;
@@ -511,7 +537,9 @@ bool build_plan(const bp_inputs* in, int n, HostPlan* p, std::string* err) {
         }
       }
     }
-    for (int c = 0; c < ncl; ++c) {
+    });
+    parallel_for(ncl, kColumnGrain, [&](size_t c_begin, size_t c_end) {
+    for (int c = (int)c_begin; c < (int)c_end; ++c) {
       const int g = cell_base + c;
       const int ic = cells[b][c].first, jc = cells[b][c].second;
       p->cell_inst[g] = b;
@@ -553,12 +581,41 @@ bool build_plan(const bp_inputs* in, int n, HostPlan* p, std::string* err) {
           p->flwafact[(size_t)g * nl + k] = I.flwafact[cel(ic, jc, nx) * nl + k];
       }
     }
+    });
     col_base += nc;
     cell_base += ncl;
   }
   fill_nbn(p);
   p->ntiles = (int)p->tile_start.size();
   return true;
+}
+
+void gather_columns(const HostPlan& p, int b, const double* uvel, const double* vvel, double* u, double* v) {
+  const InstParams& ip = p.inst[b];
+  const int nx = p.nx[b], nz = p.nz, NC = p.ncols;
+  const size_t len = sizeof(double) * nz;
+  parallel_for(ip.col_end - ip.col_begin, kColumnGrain, [&](size_t c0, size_t c1) {
+    for (size_t g = ip.col_begin + c0; g < ip.col_begin + c1; ++g) {
+      const size_t w = vtx(p.col_ij[g], p.col_ij[NC + g], nx) * nz;
+      std::memcpy(u + g * nz, uvel + w, len);
+      std::memcpy(v + g * nz, vvel + w, len);
+    }
+  });
+}
+
+void scatter_columns(const HostPlan& p, int b, const double* u, const double* v, double* uvel, double* vvel) {
+  const InstParams& ip = p.inst[b];
+  const int nx = p.nx[b], nz = p.nz, NC = p.ncols;
+  const size_t len = sizeof(double) * nz;
+  parallel_for(ip.col_end - ip.col_begin, kColumnGrain, [&](size_t c0, size_t c1) {
+    for (size_t g = ip.col_begin + c0; g < ip.col_begin + c1; ++g) {
+      const size_t w = vtx(p.col_ij[g], p.col_ij[NC + g], nx) * nz;
+      std::memcpy(uvel + w, u + g * nz, len);
+      std::memcpy(vvel + w, v + g * nz, len);
+    }
+  });
+  halo_stag(nx, p.ny[b], nz, p.periodic[b], uvel);
+  halo_stag(nx, p.ny[b], nz, p.periodic[b], vvel);
 }
 
 void gather_velocity(const HostPlan& p, int b, const double* uvel,
@@ -669,13 +726,21 @@ void scatter_efvs(const HostPlan& p, int b, const double* efvs_elem,
                   double* efvs) {
   const InstParams& ip = p.inst[b];
   const int nx = p.nx[b], ny = p.ny[b], nz = p.nz_out, NCELL = p.ncells;
-  std::memset(efvs, 0, sizeof(double) * (size_t)(nz - 1) * nx * ny);
-  for (int g = ip.cell_begin; g < ip.cell_end; ++g) {
-    const int ic = p.cell_ij[g], jc = p.cell_ij[NCELL + g];
-    for (int k = 0; k < nz - 1; ++k)  // shallow-shelf: the cell's value on every layer
-      efvs[cel(ic, jc, nx) * (nz - 1) + k] =
-          efvs_elem[p.solve2d && !p.l1l2 && !p.diva ? (size_t)g : (size_t)g * (nz - 1) + k];
-  }
+  const size_t nl = nz - 1, row = nl * nx;
+  const bool ssa = p.solve2d && !p.l1l2 && !p.diva;
+  parallel_for(ny, kColumnGrain / 32, [&](size_t j0, size_t j1) {
+    std::memset(efvs + j0 * row, 0, sizeof(double) * (j1 - j0) * row);
+  });
+  parallel_for(ip.cell_end - ip.cell_begin, kColumnGrain, [&](size_t c0, size_t c1) {
+    for (size_t g = ip.cell_begin + c0; g < ip.cell_begin + c1; ++g) {
+      double* out = efvs + cel(p.cell_ij[g], p.cell_ij[NCELL + g], nx) * nl;
+      if (ssa) {  // shallow-shelf: the cell's value on every layer
+        for (size_t k = 0; k < nl; ++k) out[k] = efvs_elem[g];
+      } else {
+        std::memcpy(out, efvs_elem + g * nl, sizeof(double) * nl);
+      }
+    }
+  });
 }
 
 void gather_matrix(const HostPlan& p, const double* Auu, const double* Auv,

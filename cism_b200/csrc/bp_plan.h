@@ -2,6 +2,7 @@
 // compact column/element form used by the device kernels (pure C++, no CUDA).
 #pragma once
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -86,6 +87,17 @@ struct HaloPlan {
   int max_cols = 0;
 };
 HaloPlan build_halo(const HostPlan& p);
+
+// f(begin, end) over [0, n) on up to eight threads, at least grain items
+// each; on the calling thread alone for small n and where no thread can be
+// started.  f must not throw.
+void parallel_for(size_t n, size_t grain, const std::function<void(size_t, size_t)>& f);
+
+// 3-D solves: velocity (nz,nx-1,ny-1) of instance b <-> u, v [ncols][nz]
+// (a column's levels side by side; launch_pack / launch_unpack turn them
+// into the node layout); scatter_columns ends with the halo update
+void gather_columns(const HostPlan& p, int b, const double* uvel, const double* vvel, double* u, double* v);
+void scatter_columns(const HostPlan& p, int b, const double* u, const double* v, double* uvel, double* vvel);
 
 // velocity (nz,nx-1,ny-1) of instance b <-> node vector
 void gather_velocity(const HostPlan& p, int b, const double* uvel,

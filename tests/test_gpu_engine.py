@@ -255,3 +255,35 @@ def test_staged_matvec_equals_per_node(ctx, variant, mixed):
                 assert all(np.array_equal(x, y) for x, y in zip(a, b)), ms[0].name
             for s, r in zip(got[0][2], other[2]):
                 assert {k: s[k] for k in keys} == {k: r[k] for k in keys}, ms[0].name
+
+
+@pytest.mark.parametrize("dims", [(9, 8, 2, 1, 0.5), (40, 33, 7, 0, 0.8), (110, 97, 11, 1, 0.7), (64, 20, 31, 0, 1.0)])
+def test_matvec_of_a_callers_matrix(ctx, dims):
+    """bp_matvec on matrices the device puts in node order in chunks of at
+    most 38,836 rows: one chunk, a last warp of a few rows, and four chunks in
+    turn in the two halves of the staging buffer.  Products of values in
+    [-1, 1], 54 a row: rounding below 54 x 54 x 2^-53 < 1e-12."""
+    nx, ny, nz, periodic, share = dims
+    rng = np.random.default_rng(nx * nz)
+    V, W = nx - 1, ny - 1
+    A = [rng.uniform(-1, 1, (W, V, nz, 27)) for _ in range(4)]
+    av = (rng.uniform(size=(W, V)) < share).astype(np.int32)
+    m = configs.slab(n=nx - 4, ny_cells=ny - 4, nz=nz).copy(periodic=periodic)
+    assert (m.nx, m.ny) == (nx, ny)
+    xu, xv = (configs.halo_fill_stag(rng.uniform(-1, 1, (W, V, nz)), periodic) for _ in range(2))
+    avh = configs.halo_fill_stag(av.astype(float), periodic)
+    yu, yv = ctx.matvec(m, av, A, xu, xv)
+    js, is_ = m.owned_vertex_slices()
+    own = np.zeros((W, V), bool)
+    own[js, is_] = True
+    # a neighbour counts where it is an owned active vertex or the image of one
+    X = [np.pad(np.where(avh[..., None] != 0, a, 0.0), 1) for a in (xu, xv)]
+    eu, ev = np.zeros((W, V, nz)), np.zeros((W, V, nz))
+    for q in range(27):
+        i, j, k = q % 3, (q // 3) % 3, q // 9
+        su, sv = (a[j:j + W, i:i + V, k:k + nz] for a in X)
+        eu += A[0][..., q] * su + A[1][..., q] * sv
+        ev += A[2][..., q] * su + A[3][..., q] * sv
+    rows = (own & (av != 0))[..., None]
+    assert np.max(np.abs(yu - np.where(rows, eu, 0.0))) <= 1e-12
+    assert np.max(np.abs(yv - np.where(rows, ev, 0.0))) <= 1e-12
