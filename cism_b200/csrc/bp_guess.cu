@@ -33,8 +33,9 @@
 extern "C" {
 int bpnet_gemm_tn(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int lda,
                   int ldb, int ldc, int accum, void* stream);
+int bpnet_gemm_act(const void* A, const void* B, float* Z, const float* bias, void* Y, int M, int N, int K, int lda,
+                   int ldb, int act, void* stream);
 int bpnet_im2col(const void* X, void* col, int B, int H, int W, int C, int Kp, int periodic, void* stream);
-int bpnet_act(const float* Z, void* Y, long long P, int C, int ldy, int c0, int act, void* stream);
 int bpnet_pool(const void* X, void* Y, int B, int H, int W, int C, void* stream);
 int bpnet_up(const void* X, void* Y, int B, int h, int w, int C, int ldy, int c0, void* stream);
 int bpnet_copy_slice(const void* X, void* Y, long long P, int C, int ldy, int c0, void* stream);
@@ -193,7 +194,7 @@ __global__ void k_guess_scatter(DevView v, int col_begin, int col_end, int ilo, 
 // One convolution: x [P][cin] BF16 -> y [P][cout] BF16 (and z, FP32 pre-activation).
 int conv_fwd(GuessNet* N, const GConv& c, const bf16* x, bf16* y, int B, int H, int W, int periodic,
              cudaStream_t s, int* nl) {
-  *nl += (c.k3 ? 1 : 0) + 1 + (y ? 1 : 0);
+  *nl += (c.k3 ? 1 : 0) + 1;
   const long long P = (long long)B * H * W;
   const bf16* col = x;
   if (c.k3) {
@@ -202,10 +203,14 @@ int conv_fwd(GuessNet* N, const GConv& c, const bf16* x, bf16* y, int B, int H, 
     NK(bpnet_im2col(x, cb, B, H, W, c.cin, c.Kp, periodic, s));
     col = cb;
   }
+  if (y) {  // the pre-activation is not kept unless the activation cannot be fused
+    const int rc = bpnet_gemm_act(col, c.wb, nullptr, c.b, y, (int)P, c.cout, c.Kp, c.Kp, c.Kp, c.act, s);
+    if (rc != 10) return rc;
+  }
   float* z = (float*)N->get(y ? "z" : "head", sizeof(float) * (size_t)P * c.cout);
   if (!z) return 6;
-  NK(bpnet_gemm_tn(col, c.wb, z, c.b, (int)P, c.cout, c.Kp, c.Kp, c.Kp, c.cout, 0, s));
-  if (y) NK(bpnet_act(z, y, P, c.cout, c.cout, 0, c.act, s));
+  if (y) NK(bpnet_gemm_act(col, c.wb, z, c.b, y, (int)P, c.cout, c.Kp, c.Kp, c.Kp, c.act, s));
+  else NK(bpnet_gemm_tn(col, c.wb, z, c.b, (int)P, c.cout, c.Kp, c.Kp, c.Kp, c.cout, 0, s));
   return 0;
 }
 

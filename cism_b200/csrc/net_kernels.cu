@@ -350,67 +350,62 @@ __global__ void k_f32_to_bf16(const float* __restrict__ x, bf16* __restrict__ y,
   GRID_LOOP(id, n) y[id] = __float2bfloat16(x[id]);
 }
 
-// A layer's backward start in one pass over Z and dY: dZ = dY * act'(Z) in
-// BF16 (the operand of both gradient products) and the column sums of its
-// FP32 values, the bias gradient.  Separately they took a pass each, with dZ
-// written and read twice in FP32.  A block strides over the rows with a fixed
-// group of V channels per thread (256 groups per blockIdx.y) and
-// leaves one partial sum per channel; k_colsum_blocks adds the blocks' in
-// order.
-constexpr int kGradBlocks = 296;
+// A layer's backward start: dZ = dY * act'(Z) in FP32 (for the column sums)
+// and in BF16 (the operand of both gradient products) in one pass.
 template <int V>
-__global__ void __launch_bounds__(256) k_act_grad_sum(const float* __restrict__ Z, const float* __restrict__ dY,
-                                                      bf16* __restrict__ dZb, float* __restrict__ part, long long P,
-                                                      int C, int act) {
-  __shared__ Pack<float, V> sm[256];
-  const int ch0 = blockIdx.y * 256 * V, g = min((C - ch0) / V, 256), rows = 256 / g;  // rows in flight per block
-  const int cg = threadIdx.x % g, r0 = threadIdx.x / g;
-  Pack<float, V> s;
+__global__ void __launch_bounds__(256) k_act_grad_both(const float* __restrict__ Z, const float* __restrict__ dY,
+                                                       float* __restrict__ dZ, bf16* __restrict__ dZb, long long n,
+                                                       int act) {
+  GRID_LOOP(id, n / V) {
+    Pack<float, V> d = ld_pack<float, V>(dY + id * V);
+    if (act) {
+      const Pack<float, V> z = ld_pack<float, V>(Z + id * V);
 #pragma unroll
-  for (int e = 0; e < V; ++e) s.e[e] = 0.f;
-  if (r0 < rows)
-    for (long long p = (long long)blockIdx.x * rows + r0; p < P; p += (long long)gridDim.x * rows) {
-      const long long o = p * C + ch0 + V * cg;
-      Pack<float, V> d = ld_pack<float, V>(dY + o);
-      if (act) {
-        const Pack<float, V> z = ld_pack<float, V>(Z + o);
-#pragma unroll
-        for (int e = 0; e < V; ++e) d.e[e] = d.e[e] * gelu_grad(z.e[e]);
-      }
-      Pack<bf16, V> b;
-#pragma unroll
-      for (int e = 0; e < V; ++e) {
-        b.e[e] = __float2bfloat16(d.e[e]);
-        s.e[e] += d.e[e];
-      }
-      st_pack(dZb + o, b);
+      for (int e = 0; e < V; ++e) d.e[e] = d.e[e] * gelu_grad(z.e[e]);
     }
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  if (r0 == 0) {
-    for (int r = 1; r < rows; ++r)
+    Pack<bf16, V> b;
 #pragma unroll
-      for (int e = 0; e < V; ++e) s.e[e] += sm[r * g + cg].e[e];
-    st_pack(part + (size_t)blockIdx.x * C + ch0 + V * cg, s);
-  }
-}
-__global__ void __launch_bounds__(256) k_colsum_blocks(const float* __restrict__ part, float* __restrict__ db,
-                                                       int blocks, int C) {
-  __shared__ float sm[8][33];
-  const int c = blockIdx.x * 32 + threadIdx.x;
-  float s = 0.f;
-  if (c < C)
-    for (int b = threadIdx.y; b < blocks; b += 8) s += part[(size_t)b * C + c];
-  sm[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.y == 0 && c < C) {
-    for (int r = 1; r < 8; ++r) s += sm[r][threadIdx.x];
-    db[c] = s;
+    for (int e = 0; e < V; ++e) b.e[e] = __float2bfloat16(d.e[e]);
+    st_pack(dZ + id * V, d);
+    st_pack(dZb + id * V, b);
   }
 }
 
-// Column sums db[c] = sum_p dZ[p][c] (fixed order: one thread per column
-// strides the rows, then a fixed-shape tree within the block).
+// Column sums in a fixed order: 256 running sums per column, the t-th over the
+// rows t, t + 256, ..., then a halving tree over them.  The running sums of
+// all columns are independent chains, one thread each (k_colsum_rows: a warp
+// reads 32 columns of a row, 16 rows of its chain in flight; one block per
+// column, as before, left most of the GPU idle), the tree is a block per column.
+__global__ void __launch_bounds__(256) k_colsum_rows(const float* __restrict__ dZ, float* __restrict__ part,
+                                                     long long P, int C) {
+  const int c = blockIdx.y * 32 + threadIdx.x, t = blockIdx.x * 8 + threadIdx.y;
+  if (c >= C) return;
+  constexpr int U = 16;
+  float s = 0.f;
+  long long p = t;
+  for (; p + 256LL * (U - 1) < P; p += 256LL * U) {
+    float x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) x[u] = __ldg(dZ + (p + 256LL * u) * C + c);
+#pragma unroll
+    for (int u = 0; u < U; ++u) s += x[u];
+  }
+  for (; p < P; p += 256) s += dZ[p * C + c];
+  part[t * C + c] = s;
+}
+__global__ void __launch_bounds__(256) k_colsum_tree(const float* __restrict__ part, float* __restrict__ db, int C) {
+  __shared__ float sm[256];
+  const int c = blockIdx.x;
+  sm[threadIdx.x] = part[threadIdx.x * C + c];
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) db[c] = sm[0];
+}
+
+// The same sums without scratch, one block per column.
 __global__ void k_colsum(const float* __restrict__ dZ, float* __restrict__ db, long long P, int C) {
   __shared__ float sm[256];
   const int c = blockIdx.x;
@@ -768,24 +763,43 @@ __global__ void __launch_bounds__(128) k_gemm_tc(const bf16* __restrict__ A, con
 
 // ---------------------------------------------------------------------
 // The same product with its operands brought in by the Tensor Memory
-// Accelerator: a four-stage ring of shared-memory slices, each filled by
-// 16 cp.async.bulk.tensor boxes (one K chunk of 8 elements by 128 rows of
-// A, or by BN rows of B: exactly one column of core matrices of the
-// no-swizzle K-major layout, so the boxes land where the UMMA descriptors
-// read) that complete on the stage's "full" mbarrier.  One thread issues
-// the loads and the tcgen05.mma of every slice; a stage is refilled with
-// the slice four ahead once the tensor core's commit for it has arrived on
-// the stage's "done" mbarrier, so up to four slices of loads are in flight
-// while the tensor core works.  Out-of-range rows and K columns read as
-// zero (the tensor maps' bounds).  Epilogue as k_gemm_tc.  Every wait is
-// bounded; on a timeout the issuing thread waits (bounded) for its copies
-// and its last multiply in flight, raises g_tc_err, and the CTA frees its
-// tensor memory and returns.  Loads only: no TMA store, no multicast.
+// Accelerator: a four-stage ring of shared-memory slices that complete on the
+// stage's "full" mbarrier.  One thread issues the loads and the tcgen05.mma
+// of every slice; a stage is refilled with the slice four ahead once the
+// tensor core's commit for it has arrived on the stage's "done" mbarrier, so
+// up to four slices of loads are in flight while the tensor core works.
+// Operands lie in shared memory with the 128-byte swizzle, so that a slice is
+// one box of 128-byte rows per operand (16-byte boxes of the unswizzled
+// layout left the copy engine as the limit: 131,072 x 64 x 576 took 83 us, now
+// 47; 32 x 288 x 524,288 362 us, now 148).  Either operand is K-major
+// (element (m, k) at [m * ld + k]: a box of 64 K elements by the tile's rows)
+// or MN-major ([k * ld + m]: boxes of 64 rows of the product by 64 K), which
+// takes the gradient products' operands as the other passes left them, without
+// transposed copies.  Out-of-range rows and K read as zero (the tensor maps'
+// bounds).  Epilogue as k_gemm_tc; ACT also or instead writes the activation
+// of the result in BF16.  Every wait is bounded; on a timeout the issuing
+// thread waits (bounded) for its copies and its last multiply in flight,
+// raises g_tc_err, and the CTA frees its tensor memory and returns.  Loads
+// only: no TMA store, no multicast.
 // ---------------------------------------------------------------------
 constexpr int TM_STAGES = 4;
 
-template <int BN>
-constexpr int tm_smem_bytes() { return TM_STAGES * tc_stage_bytes<BN>() + 1024; }  // + room to align the ring
+// bytes of an operand's slice: rows x 64 K elements; MN-major in whole boxes of 64
+template <int ROWS, bool MN>
+constexpr int tm_operand_bytes() { return (MN ? (ROWS + 63) / 64 * 64 : ROWS) * TC_BK * 2; }
+template <int BN, bool AMN, bool BMN>
+constexpr int tm_stage_bytes() { return tm_operand_bytes<TC_BM, AMN>() + tm_operand_bytes<BN, BMN>(); }
+template <int BN, bool AMN, bool BMN>
+constexpr int tm_smem_bytes() { return TM_STAGES * tm_stage_bytes<BN, AMN, BMN>() + 1024; }  // + room to align the ring
+
+// UMMA shared-memory descriptor with the 128-byte swizzle.  K-major: 8-row
+// groups 1024 bytes apart (the leading offset is not used); MN-major: groups
+// of 8 K rows 1024 bytes apart, boxes of 64 rows of the product 8192.
+template <bool MN>
+__device__ __forceinline__ uint64_t umma_desc_sw(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(MN ? 8192 >> 4 : 1) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
 
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"(bytes), "r"(bar) : "memory");
@@ -801,22 +815,23 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-template <int BN>
+template <int BN, bool AMN, bool BMN>
 __global__ void __launch_bounds__(128) k_gemm_tma(const __grid_constant__ CUtensorMap tmA,
                                                   const __grid_constant__ CUtensorMap tmB, float* __restrict__ C,
                                                   const float* __restrict__ bias, int M, int N, int K, int ldc,
-                                                  int accum, int kchunk, long long cstride) {
+                                                  int accum, int kchunk, long long cstride, bf16* __restrict__ Y,
+                                                  int act) {
   extern __shared__ __align__(1024) uint8_t tc_smem[];
   __shared__ __align__(8) uint64_t full[TM_STAGES], done[TM_STAGES];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_ok;
-  constexpr int STAGE = tc_stage_bytes<BN>();
+  constexpr int STAGE = tm_stage_bytes<BN, AMN, BMN>(), A_BYTES = tm_operand_bytes<TC_BM, AMN>();
   const int tid = threadIdx.x, warp = tid >> 5;
   const int m0 = blockIdx.y * TC_BM, n0 = blockIdx.x * BN;
   const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-  C += (size_t)blockIdx.z * cstride;
+  if (C) C += (size_t)blockIdx.z * cstride;
   const int nk = (kend - kbeg + TC_BK - 1) / TC_BK;
-  // the ring starts on a 1024-byte boundary (the boxes land on 512-byte ones)
+  // the ring starts on a 1024-byte boundary, the swizzle's period
   const uint32_t ring = (smem_u32(tc_smem) + 1023u) & ~1023u;
   uint8_t* ring_ptr = tc_smem + (ring - smem_u32(tc_smem));
   if (warp == 0) {
@@ -837,15 +852,25 @@ __global__ void __launch_bounds__(128) k_gemm_tma(const __grid_constant__ CUtens
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
   if (tid == 0) {
+    // MN-major: boxes past the operand's last row are left out (their rows of
+    // the product are not stored)
+    const int boxa = AMN ? min(TC_BM / 64, (M - m0 + 63) / 64) : 1;
+    const int boxb = BMN ? min((BN + 63) / 64, (N - n0 + 63) / 64) : 1;
+    const uint32_t bytes = (uint32_t)((AMN ? boxa * 8192 : A_BYTES) + (BMN ? boxb * 8192 : STAGE - A_BYTES));
     auto issue = [&](int j) {  // slice j into stage j % TM_STAGES
       const int st = j % TM_STAGES;
-      const uint32_t a = ring + st * STAGE, b = a + TC_A_BYTES, bar = smem_u32(&full[st]);
-      mbar_expect_tx(bar, STAGE);
+      const uint32_t a = ring + st * STAGE, b = a + A_BYTES, bar = smem_u32(&full[st]);
+      mbar_expect_tx(bar, bytes);
       const int k0 = kbeg + j * TC_BK;
-#pragma unroll
-      for (int kc = 0; kc < 8; ++kc) {
-        tma_load_2d(a + kc * (TC_BM / 8) * 128, &tmA, k0 + kc * 8, m0, bar);
-        tma_load_2d(b + kc * (BN / 8) * 128, &tmB, k0 + kc * 8, n0, bar);
+      if (AMN) {
+        for (int x = 0; x < boxa; ++x) tma_load_2d(a + x * 8192, &tmA, m0 + 64 * x, k0, bar);
+      } else {
+        tma_load_2d(a, &tmA, k0, m0, bar);
+      }
+      if (BMN) {
+        for (int x = 0; x < boxb; ++x) tma_load_2d(b + x * 8192, &tmB, n0 + 64 * x, k0, bar);
+      } else {
+        tma_load_2d(b, &tmB, k0, n0, bar);
       }
     };
     bool ok = true;
@@ -859,17 +884,18 @@ __global__ void __launch_bounds__(128) k_gemm_tma(const __grid_constant__ CUtens
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int k0 = kbeg + it * TC_BK;
-      const uint32_t a = ring + st * STAGE, b = a + TC_A_BYTES;
+      const uint32_t a = ring + st * STAGE, b = a + A_BYTES;
 #pragma unroll
       for (int s = 0; s < TC_BK / 16; ++s) {
         if (k0 + 16 * s >= kend) break;
-        const uint64_t ad = umma_desc(a + 2 * s * (TC_BM / 8) * 128, (TC_BM / 8) * 128, 128);
-        const uint64_t bd = umma_desc(b + 2 * s * (BN / 8) * 128, (BN / 8) * 128, 128);
+        // 16 K elements on: 32 bytes along a K-major row, two groups of 8 K rows MN-major
+        const uint64_t ad = umma_desc_sw<AMN>(a + s * (AMN ? 2048 : 32));
+        const uint64_t bd = umma_desc_sw<BMN>(b + s * (BMN ? 2048 : 32));
         const uint32_t acc = (it > 0 || s > 0) ? 1u : 0u;
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem),
-            "l"(ad), "l"(bd), "r"(tc_idesc<BN>()), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+            "l"(ad), "l"(bd), "r"(tc_idesc<BN>() | (AMN ? 1u << 15 : 0u) | (BMN ? 1u << 16 : 0u)), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                        smem_u32(&done[st]))
@@ -921,10 +947,13 @@ __global__ void __launch_bounds__(128) k_gemm_tma(const __grid_constant__ CUtens
         for (int r = 0; r < 32; ++r) {
           const int row = m0 + warp * 32 + r;
           if (row >= M) break;
-          float* dst = C + (size_t)row * ldc + col;
           float x = T[r * 33 + lane] + bc;
-          if (accum) x += *dst;
-          *dst = x;
+          if (C) {
+            float* dst = C + (size_t)row * ldc + col;
+            if (accum) x += *dst;
+            *dst = x;
+          }
+          if (Y) Y[(size_t)row * ldc + col] = __float2bfloat16(act ? gelu(x) : x);
         }
       }
       __syncwarp();
@@ -935,11 +964,11 @@ __global__ void __launch_bounds__(128) k_gemm_tma(const __grid_constant__ CUtens
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
 }
 
-// The 2-D tensor map of a row-major BF16 operand [rows][ld] (K = the first
-// K columns) with boxes of 8 K elements by box_rows rows; false where the
-// driver has no encoder or refuses the operand (address or stride not
-// 16-byte aligned).
-bool tma_map(CUtensorMap* map, const void* ptr, int rows, int K, int ld, int box_rows) {
+// The 2-D tensor map of a row-major BF16 operand, inner x outer elements with
+// rows of ld, in boxes of 64 inner elements (128 bytes, swizzled) by box_outer;
+// false where the driver has no encoder or refuses the operand (address or
+// stride not 16-byte aligned).
+bool tma_map(CUtensorMap* map, const void* ptr, int inner, int outer, int ld, int box_outer) {
   static PFN_cuTensorMapEncodeTiled_v12000 enc = [] {
     void* f = nullptr;
     cudaDriverEntryPointQueryResult q;
@@ -949,12 +978,12 @@ bool tma_map(CUtensorMap* map, const void* ptr, int rows, int K, int ld, int box
     return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
   }();
   if (!enc || (reinterpret_cast<uintptr_t>(ptr) & 15) || ((size_t)ld * 2) % 16) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+  const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {8, (cuuint32_t)box_rows};
+  const cuuint32_t box[2] = {64, (cuuint32_t)box_outer};
   const cuuint32_t es[2] = {1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -996,104 +1025,182 @@ float* splitk_scratch(size_t n) {
   return b.first;
 }
 
-// One tcgen05 product of tile width W: TMA-fed (maps given) or register-staged.
+// One product on the TMA-fed kernel.
+template <int W, bool AMN, bool BMN>
+bool launch_tma(const CUtensorMap& ma, const CUtensorMap& mb, dim3 grid, cudaStream_t st, float* out,
+                const float* bout, int M, int N, int K, int ldo, int acc, int kchunk, long long cs, bf16* Y, int act) {
+  static const bool ok = cudaFuncSetAttribute(k_gemm_tma<W, AMN, BMN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              tm_smem_bytes<W, AMN, BMN>()) == cudaSuccess;
+  if (!ok) return false;
+  k_gemm_tma<W, AMN, BMN><<<grid, 128, tm_smem_bytes<W, AMN, BMN>(), st>>>(ma, mb, out, bout, M, N, K, ldo, acc,
+                                                                           kchunk, cs, Y, act);
+  return true;
+}
 template <int W>
-void launch_tile(bool tma, const CUtensorMap& ma, const CUtensorMap& mb, dim3 grid, cudaStream_t st,
-                 const bf16* A, const bf16* B, float* out, const float* bout, int M, int N, int K, int lda, int ldb,
-                 int ldo, int acc, int kchunk, long long cs) {
-  if (tma)
-    k_gemm_tma<W><<<grid, 128, tm_smem_bytes<W>(), st>>>(ma, mb, out, bout, M, N, K, ldo, acc, kchunk, cs);
-  else
-    k_gemm_tc<W><<<grid, 128, 2 * tc_stage_bytes<W>(), st>>>(A, B, out, bout, M, N, K, lda, ldb, ldo, acc, kchunk,
-                                                             cs);
+bool launch_tma_major(int a_mn, int b_mn, const CUtensorMap& ma, const CUtensorMap& mb, dim3 grid, cudaStream_t st,
+                      float* out, const float* bout, int M, int N, int K, int ldo, int acc, int kchunk, long long cs,
+                      bf16* Y, int act) {
+  if (a_mn && b_mn) return launch_tma<W, true, true>(ma, mb, grid, st, out, bout, M, N, K, ldo, acc, kchunk, cs, Y, act);
+  if (a_mn) return launch_tma<W, true, false>(ma, mb, grid, st, out, bout, M, N, K, ldo, acc, kchunk, cs, Y, act);
+  if (b_mn) return launch_tma<W, false, true>(ma, mb, grid, st, out, bout, M, N, K, ldo, acc, kchunk, cs, Y, act);
+  return launch_tma<W, false, false>(ma, mb, grid, st, out, bout, M, N, K, ldo, acc, kchunk, cs, Y, act);
+}
+template <int W>
+bool launch_tc(dim3 grid, cudaStream_t st, const bf16* A, const bf16* B, float* out, const float* bout, int M, int N,
+               int K, int lda, int ldb, int ldo, int acc, int kchunk, long long cs) {
+  static const bool ok = cudaFuncSetAttribute(k_gemm_tc<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              2 * tc_stage_bytes<W>()) == cudaSuccess;
+  if (!ok) return false;
+  k_gemm_tc<W><<<grid, 128, 2 * tc_stage_bytes<W>(), st>>>(A, B, out, bout, M, N, K, lda, ldb, ldo, acc, kchunk, cs);
+  return true;
 }
 
-template <int W>
-bool tile_smem_ok() {
-  return cudaFuncSetAttribute(k_gemm_tc<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * tc_stage_bytes<W>()) ==
-             cudaSuccess &&
-         cudaFuncSetAttribute(k_gemm_tma<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, tm_smem_bytes<W>()) ==
-             cudaSuccess;
-}
-
-}  // namespace
-
-extern "C" {
-
-// Returns 0, or 10 for arguments the kernels do not take.  A product
-// with few output tiles and a long K (the weight gradients, K = pixels)
-// is split along K over enough CTAs to fill the GPU, its partial products
-// summed in order by k_splitk_sum.
-// The product with an explicit kernel: mode 0 tcgen05 with TMA-fed operands
-// (k_gemm_tma), 1 tcgen05 with register-staged operands (k_gemm_tc), 2 the
-// mma.sync kernel.
-int bpnet_gemm_tn_mode(int mode, const void* A, const void* B, float* C, const float* bias, int M, int N, int K,
-                       int lda, int ldb, int ldc, int accum, void* stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (lda % 8) || (ldb % 8) || mode < 0 || mode > 2) return 10;
-  static const bool smem_ok = tile_smem_ok<32>() && tile_smem_ok<64>() && tile_smem_ok<128>();
-  if (!smem_ok) return 6;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (mode == 2) {
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    k_gemm_tn<<<grid, 128, 0, st>>>((const bf16*)A, (const bf16*)B, C, bias, M, N, K, lda, ldb, ldc, accum);
-    return cudaGetLastError() == cudaSuccess ? 0 : 6;
-  }
+// How a product is cut: tile width bn, split S of K in chunks of kchunk.
+struct GemmCut {
+  int bn, S, kchunk, gx, gy;
+};
+GemmCut cut_gemm(int M, int N, int K) {
+  GemmCut c;
   // tile width: 32 for at most 32 columns (no MMA work on padding); 128
   // for widths that are not a multiple of 64 where it pads no more than 64
   // does (96: one tile instead of 64 + 32, A read once); else 64 (a
   // multiple of 64 keeps twice the CTAs: 128 x 128 tiles measured slower at
   // N = 128 and 1152)
-  int bn = 64;
+  c.bn = 64;
   if (N <= 32)
-    bn = 32;
+    c.bn = 32;
   else if (N % 64 != 0 && (N + 127) / 128 * 128 <= (N + 63) / 64 * 64)
-    bn = 128;
-  const int gx = (N + bn - 1) / bn, gy = (M + TC_BM - 1) / TC_BM, nslices = (K + TC_BK - 1) / TC_BK;
-  int S = 1, kchunk = nslices * TC_BK;
-  if (gx * gy < 296 && nslices >= 64) S = std::min((296 + gx * gy - 1) / (gx * gy), nslices / 16);
+    c.bn = 128;
+  const int nslices = (K + TC_BK - 1) / TC_BK;
+  c.gx = (N + c.bn - 1) / c.bn;
+  c.gy = (M + TC_BM - 1) / TC_BM;
+  c.S = 1;
+  c.kchunk = nslices * TC_BK;
+  // few output tiles and a long K (the weight gradients, K = pixels): split
+  // along K over enough CTAs to fill the GPU
+  if (c.gx * c.gy < 296 && nslices >= 64)
+    c.S = std::min((296 + c.gx * c.gy - 1) / (c.gx * c.gy), nslices / 16);
+  if (c.S > 1) {
+    c.kchunk = (nslices + c.S - 1) / c.S * TC_BK;
+    c.S = (K + c.kchunk - 1) / c.kchunk;  // no empty chunk
+  }
+  return c;
+}
+
+// C = A B^T (+ bias) (+ C) on the tensor cores: tma = 1 the TMA-fed kernel
+// (10 where its operands cannot be mapped), 0 the register-staged one (both
+// operands K-major).  a_mn, b_mn: the operand is MN-major (element (m, k) at
+// [k * ld + m]).  Y (not with a split K or accumulation): act of the result in
+// BF16, rows of ldc; C may then be null.
+int tensor_gemm(int tma, int a_mn, int b_mn, const bf16* A, const bf16* B, float* C, const float* bias, int M, int N,
+                int K, int lda, int ldb, int ldc, int accum, bf16* Y, int act, cudaStream_t st) {
+  const GemmCut c = cut_gemm(M, N, K);
+  if (Y && (c.S > 1 || accum)) return 10;
+  CUtensorMap ma, mb;
+  if (tma &&
+      !(a_mn ? tma_map(&ma, A, M, K, lda, 64) : tma_map(&ma, A, K, M, lda, TC_BM)))
+    return 10;
+  if (tma && !(b_mn ? tma_map(&mb, B, N, K, ldb, 64) : tma_map(&mb, B, K, N, ldb, c.bn))) return 10;
   float* out = C;
   const float* bout = bias;
   int ldo = ldc, acc = accum;
   long long cs = 0;
-  if (S > 1) {  // partial products into the scratch, summed afterwards
-    kchunk = (nslices + S - 1) / S * TC_BK;
-    S = (K + kchunk - 1) / kchunk;  // no empty chunk
+  if (c.S > 1) {  // partial products into the scratch, summed afterwards
     cs = (long long)M * N;
-    out = splitk_scratch((size_t)S * cs);
+    out = splitk_scratch((size_t)c.S * cs);
     if (!out) return 6;
     bout = nullptr;
     ldo = N;
     acc = 0;
   }
-  const dim3 grid(gx, gy, S);
-  CUtensorMap ma, mb;
-  // a product of one K slice has no pipeline to fill: the register-staged
-  // kernel starts sooner (measured faster at K <= 64, slower above)
-  const bool tma =
-      mode == 0 && nslices > 1 && tma_map(&ma, A, M, K, lda, TC_BM) && tma_map(&mb, B, N, K, ldb, bn);
-  const bf16 *a16 = (const bf16*)A, *b16 = (const bf16*)B;
-  if (bn == 32)
-    launch_tile<32>(tma, ma, mb, grid, st, a16, b16, out, bout, M, N, K, lda, ldb, ldo, acc, kchunk, cs);
-  else if (bn == 64)
-    launch_tile<64>(tma, ma, mb, grid, st, a16, b16, out, bout, M, N, K, lda, ldb, ldo, acc, kchunk, cs);
+  const dim3 grid(c.gx, c.gy, c.S);
+  bool ok;
+  if (!tma)
+    ok = c.bn == 32   ? launch_tc<32>(grid, st, A, B, out, bout, M, N, K, lda, ldb, ldo, acc, c.kchunk, cs)
+         : c.bn == 64 ? launch_tc<64>(grid, st, A, B, out, bout, M, N, K, lda, ldb, ldo, acc, c.kchunk, cs)
+                      : launch_tc<128>(grid, st, A, B, out, bout, M, N, K, lda, ldb, ldo, acc, c.kchunk, cs);
   else
-    launch_tile<128>(tma, ma, mb, grid, st, a16, b16, out, bout, M, N, K, lda, ldb, ldo, acc, kchunk, cs);
-  if (S > 1) k_splitk_sum<<<grid_for(cs), 256, 0, st>>>(out, S, cs, C, bias, M, N, ldc, accum);
+    ok = c.bn == 32
+             ? launch_tma_major<32>(a_mn, b_mn, ma, mb, grid, st, out, bout, M, N, K, ldo, acc, c.kchunk, cs, Y, act)
+         : c.bn == 64
+             ? launch_tma_major<64>(a_mn, b_mn, ma, mb, grid, st, out, bout, M, N, K, ldo, acc, c.kchunk, cs, Y, act)
+             : launch_tma_major<128>(a_mn, b_mn, ma, mb, grid, st, out, bout, M, N, K, ldo, acc, c.kchunk, cs, Y, act);
+  if (!ok) return 6;
+  if (c.S > 1) k_splitk_sum<<<grid_for(cs), 256, 0, st>>>(out, c.S, cs, C, bias, M, N, ldc, accum);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
-// The product on the default kernel: tcgen05 with TMA-fed operands (with
-// register-staged ones for a single K slice); BPNET_GEMM=tc selects the
+// The default kernel of the products (bpnet_gemm_tn): BPNET_GEMM=tc selects the
 // register-staged tcgen05 kernel throughout, BPNET_GEMM=mma the mma.sync one.
-int bpnet_gemm_tn(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int lda,
-                  int ldb, int ldc, int accum, void* stream) {
+int gemm_mode() {
   static const int mode = [] {
     const char* e = std::getenv("BPNET_GEMM");
     if (e && std::strcmp(e, "mma") == 0) return 2;
     if (e && std::strcmp(e, "tc") == 0) return 1;
     return 0;
   }();
-  return bpnet_gemm_tn_mode(mode, A, B, C, bias, M, N, K, lda, ldb, ldc, accum, stream);
+  return mode;
+}
+
+}  // namespace
+
+extern "C" {
+
+int bpnet_act(const float* Z, void* Y, long long P, int C, int ldy, int c0, int act, void* stream);
+
+// Returns 0, or 10 for arguments the kernels do not take.
+// The product with an explicit kernel: mode 0 tcgen05 with TMA-fed operands
+// (k_gemm_tma), 1 tcgen05 with register-staged operands (k_gemm_tc), 2 the
+// mma.sync kernel.
+int bpnet_gemm_tn_mode(int mode, const void* A, const void* B, float* C, const float* bias, int M, int N, int K,
+                       int lda, int ldb, int ldc, int accum, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (lda % 8) || (ldb % 8) || mode < 0 || mode > 2) return 10;
+  cudaStream_t st = (cudaStream_t)stream;
+  const bf16 *a16 = (const bf16*)A, *b16 = (const bf16*)B;
+  if (mode == 2) {
+    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+    k_gemm_tn<<<grid, 128, 0, st>>>(a16, b16, C, bias, M, N, K, lda, ldb, ldc, accum);
+    return cudaGetLastError() == cudaSuccess ? 0 : 6;
+  }
+  if (mode == 0) {
+    const int rc = tensor_gemm(1, 0, 0, a16, b16, C, bias, M, N, K, lda, ldb, ldc, accum, nullptr, 0, st);
+    if (rc != 10) return rc;  // operands that TMA cannot map go through registers
+  }
+  return tensor_gemm(0, 0, 0, a16, b16, C, bias, M, N, K, lda, ldb, ldc, accum, nullptr, 0, st);
+}
+
+// The product on the default kernel.
+int bpnet_gemm_tn(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int lda,
+                  int ldb, int ldc, int accum, void* stream) {
+  return bpnet_gemm_tn_mode(gemm_mode(), A, B, C, bias, M, N, K, lda, ldb, ldc, accum, stream);
+}
+
+// The product with its activation: Z = A B^T + bias (FP32, may be null) and Y
+// = act(Z) in BF16, both with rows of N.
+int bpnet_gemm_act(const void* A, const void* B, float* Z, const float* bias, void* Y, int M, int N, int K, int lda,
+                   int ldb, int act, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (lda % 8) || (ldb % 8) || !Y) return 10;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (gemm_mode() == 0) {
+    const int rc = tensor_gemm(1, 0, 0, (const bf16*)A, (const bf16*)B, Z, bias, M, N, K, lda, ldb, N, 0, (bf16*)Y,
+                               act, st);
+    if (rc != 10) return rc;
+  }
+  if (!Z) return 10;
+  const int rc = bpnet_gemm_tn(A, B, Z, bias, M, N, K, lda, ldb, N, 0, stream);
+  return rc ? rc : bpnet_act(Z, Y, M, N, N, 0, act, stream);
+}
+
+// The product of operands of either order (a_mn, b_mn: element (m, k) at
+// [k * ld + m]) on the TMA-fed kernel: the gradient products.  lda, ldb
+// multiples of 8; 10 where the operands cannot be mapped.
+int bpnet_gemm_major(int a_mn, int b_mn, const void* A, const void* B, float* C, int M, int N, int K, int lda, int ldb,
+                     int ldc, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || (lda % 8) || (ldb % 8)) return 10;
+  if ((!a_mn || !b_mn) && K % 8) return 10;
+  if (gemm_mode() != 0) return 10;
+  return tensor_gemm(1, a_mn != 0, b_mn != 0, (const bf16*)A, (const bf16*)B, C, nullptr, M, N, K, lda, ldb, ldc, 0,
+                     nullptr, 0, (cudaStream_t)stream);
 }
 
 // The mma.sync kernel (the comparison of the tcgen05 one).
@@ -1181,19 +1288,20 @@ int bpnet_act_grad(const float* Z, const float* dY, float* dZ, long long P, int 
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
-// dZ in BF16 and its column sums db [C] in one pass (dY [P][C], part: 296 C
-// floats of scratch).
-int bpnet_act_grad_sum(const float* Z, const float* dY, void* dZb, float* db, float* part, long long P, int C,
+// dZ in BF16 and its column sums db [C] (dY [P][C]; scratch: (P + 256) C
+// floats, which receive dZ in FP32 and the running sums).
+int bpnet_act_grad_sum(const float* Z, const float* dY, void* dZb, float* db, float* scratch, long long P, int C,
                        int act, void* stream) {
   if (C <= 0) return 10;
   cudaStream_t st = (cudaStream_t)stream;
-  const bool v4 = C % 4 == 0 && aligned(Z, 16) && aligned(dY, 16) && aligned(dZb, 8) && aligned(part, 16);
-  const int per = std::min(v4 ? C / 4 : C, 256), rows = 256 / per;
-  const int blocks = (int)std::max(1LL, std::min((long long)kGradBlocks, (P + rows - 1) / rows));
-  const dim3 grid(blocks, ((v4 ? C / 4 : C) + 255) / 256);
-  if (v4) k_act_grad_sum<4><<<grid, 256, 0, st>>>(Z, dY, (bf16*)dZb, part, P, C, act);
-  else k_act_grad_sum<1><<<grid, 256, 0, st>>>(Z, dY, (bf16*)dZb, part, P, C, act);
-  k_colsum_blocks<<<(C + 31) / 32, dim3(32, 8), 0, st>>>(part, db, blocks, C);
+  const long long n = P * C;
+  float* part = scratch + n;
+  if (n % 4 == 0 && aligned(Z, 16) && aligned(dY, 16) && aligned(dZb, 8) && aligned(scratch, 16))
+    k_act_grad_both<4><<<grid_for(n / 4), 256, 0, st>>>(Z, dY, scratch, (bf16*)dZb, n, act);
+  else
+    k_act_grad_both<1><<<grid_for(n), 256, 0, st>>>(Z, dY, scratch, (bf16*)dZb, n, act);
+  k_colsum_rows<<<dim3(32, (C + 31) / 32), dim3(32, 8), 0, st>>>(scratch, part, P, C);
+  k_colsum_tree<<<C, 256, 0, st>>>(part, db, C);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 

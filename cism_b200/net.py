@@ -44,6 +44,8 @@ def lib():
             "bpnet_gemm_tn": [vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
             "bpnet_gemm_tn_mma": [vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
             "bpnet_gemm_tn_mode": [i, vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
+            "bpnet_gemm_act": [vp, vp, vp, vp, vp, i, i, i, i, i, i, vp],
+            "bpnet_gemm_major": [i, i, vp, vp, vp, i, i, i, i, i, i, vp],
             "bpnet_gemm_status": [vp],
             "bpnet_im2col": [vp, vp, i, i, i, i, i, i, vp],
             "bpnet_col2im": [vp, vp, i, i, i, i, i, i, vp],
@@ -116,6 +118,16 @@ def gemm_tn(A, B, out, bias, M, N, K, lda, ldb, ldc, accum=False, kernel=None):
     _ck(rc, "bpnet_gemm_tn")
 
 
+def gemm_major(a_mn, b_mn, A, B, out, M, N, K, lda, ldb, ldc) -> bool:
+    """out[M][N] (FP32) = A . B^T with either operand K-major ([m][k]) or MN-major
+    ([k][m]); False where the TMA-fed kernel does not take the operands."""
+    rc = lib().bpnet_gemm_major(int(a_mn), int(b_mn), _p(A), _p(B), _p(out), M, N, K, lda, ldb, ldc, _s())
+    if rc == 10:
+        return False
+    _ck(rc, "bpnet_gemm_major")
+    return True
+
+
 def gemm_status() -> int:
     """1 if a bounded wait of the tcgen05 GEMM ran out since the last call."""
     return int(lib().bpnet_gemm_status(_s()))
@@ -175,9 +187,9 @@ class Conv:
         else:
             col = x
         z = torch.empty((P, self.cout), dtype=torch.float32, device=x.device)
-        gemm_tn(col, self.wb, z, self.b, P, self.cout, self.Kp, self.Kp, self.Kp, self.cout)
         y = torch.empty((P, self.cout), dtype=torch.bfloat16, device=x.device)
-        _ck(lib().bpnet_act(_p(z), _p(y), P, self.cout, self.cout, 0, int(self.act), _s()), "act")
+        _ck(lib().bpnet_gemm_act(_p(col), _p(self.wb), _p(z), _p(self.b), _p(y), P, self.cout, self.Kp, self.Kp,
+                                 self.Kp, int(self.act), _s()), "gemm_act")
         self.saved = (col, z, shape, periodic) if train else None
         return y, z
 
@@ -188,22 +200,21 @@ class Conv:
         P = B * H * W
         self.gb = torch.empty(self.cout, dtype=torch.float32, device=dy.device)
         dzb = torch.empty((P, self.cout), dtype=torch.bfloat16, device=dy.device)
-        part = torch.empty(296 * self.cout, dtype=torch.float32, device=dy.device)
-        _ck(lib().bpnet_act_grad_sum(_p(z), _p(dy), _p(dzb), _p(self.gb), _p(part), P, self.cout, int(self.act),
+        scratch = torch.empty((P + 256, self.cout), dtype=torch.float32, device=dy.device)
+        _ck(lib().bpnet_act_grad_sum(_p(z), _p(dy), _p(dzb), _p(self.gb), _p(scratch), P, self.cout, int(self.act),
                                      _s()), "act_grad_sum")
-        P8 = ceil8(P)
-        dzt = transpose(dzb, P8)
-        colt = transpose(col, P8)
         gwp = torch.empty((self.cout, self.Kp), dtype=torch.float32, device=dy.device)
-        gemm_tn(dzt, colt, gwp, None, self.cout, self.Kp, P8, P8, P8, self.Kp)
+        if not gemm_major(True, True, dzb, col, gwp, self.cout, self.Kp, P, self.cout, self.Kp, self.Kp):
+            P8 = ceil8(P)
+            gemm_tn(transpose(dzb, P8), transpose(col, P8), gwp, None, self.cout, self.Kp, P8, P8, P8, self.Kp)
         self.gw = torch.empty((self.cout, self.K), dtype=torch.float32, device=dy.device)
         _ck(lib().bpnet_unpad(_p(gwp), _p(self.gw), self.cout, self.K, self.Kp, _s()), "unpad")
         self.saved = None
         if not need_dx:
             return None
-        wt = transpose(self.wb)  # [Kp][cout]
         dcol = torch.empty((P, self.Kp), dtype=torch.float32, device=dy.device)
-        gemm_tn(dzb, wt, dcol, None, P, self.Kp, self.cout, self.cout, self.cout, self.Kp)
+        if not gemm_major(False, True, dzb, self.wb, dcol, P, self.Kp, self.cout, self.cout, self.Kp, self.Kp):
+            gemm_tn(dzb, transpose(self.wb), dcol, None, P, self.Kp, self.cout, self.cout, self.cout, self.Kp)
         if not self.k3:
             return dcol
         dx = torch.empty((P, self.cin), dtype=torch.float32, device=dy.device)

@@ -274,10 +274,13 @@ def test_pointwise_kernels_match_torch(shape, offset):
     assert L.bpnet_act(p(z), p(y), P, C, C + 8, 8, 1, s) == 0
     ref = torch.nn.functional.gelu(z.double())
     assert bool(((y[:, 8:].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-7).all())
-    dz, dzb, db, part = new(P, C), new(P, C, dtype=bf), new(C), new(296 * C)
+    dz, dzb, db, part = new(P, C), new(P, C, dtype=bf), new(C), new((P + 256) * C)
     assert L.bpnet_act_grad(p(z), p(dy), p(dz), P, C, C, 0, 1, s) == 0
     assert L.bpnet_act_grad_sum(p(z), p(dy), p(dzb), p(db), p(part), P, C, 1, s) == 0
-    assert torch.equal(dzb, dz.to(bf))
+    assert torch.equal(dzb, dz.to(bf)) and torch.equal(part[:P * C].view(P, C), dz)
+    db1 = new(C)
+    assert L.bpnet_colsum(p(dz), p(db1), P, C, s) == 0
+    assert torch.equal(db, db1)
     mag = dz.double().abs().sum(0)
     assert bool(((db.double() - dz.double().sum(0)).abs() <= (P + 8) * 2.0 ** -24 * mag).all())
     c2 = new(B, H // 2, W // 2, C, dtype=bf)
@@ -306,3 +309,57 @@ def test_pointwise_kernels_match_torch(shape, offset):
     assert L.bpnet_pool_grad(p(ug), p(pg), B, H, W, C, C, 0, s) == 0
     assert torch.equal(pg, a.view(B, H, W, C) + 0.25 * ug.repeat_interleave(2, 1).repeat_interleave(2, 2))
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("a_mn", [0, 1])
+@pytest.mark.parametrize("b_mn", [0, 1])
+@pytest.mark.parametrize("shape", [(64, 64, 64), (24, 40, 72), (136, 136, 8), (96, 864, 1000), (128, 1152, 2056),
+                                   (32, 288, 8192), (264, 56, 4168), (40, 200, 16)])
+def test_gemm_of_either_operand_order(shape, a_mn, b_mn):
+    """K-major and MN-major operands of the TMA-fed kernel: rows that end
+    within a box of 64 and within a tile of 128, K that is not a multiple of a
+    slice or of 16, each tile width, split K; against the FP64 product of the
+    same BF16 operands (1e-5, FP32 accumulation), and bitwise the register-staged
+    kernel's product of the same operands in K-major order."""
+    torch = pytest.importorskip("torch")
+    from cism_b200 import net as netmod
+
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    A = a.t().contiguous() if a_mn else a
+    B = b.t().contiguous() if b_mn else b
+    out = torch.full((M, N + 8), float("nan"), device="cuda")
+    assert netmod.gemm_major(a_mn, b_mn, A, B, out, M, N, K, M if a_mn else K, N if b_mn else K, N + 8)
+    ref = a.double() @ b.double().t()
+    assert float((out[:, :N].double() - ref).norm() / ref.norm()) < 1e-5
+    assert bool(out[:, N:].isnan().all())
+    tc = torch.empty((M, N), device="cuda")
+    netmod.gemm_tn(a, b, tc, None, M, N, K, K, K, N, kernel="tc")
+    assert torch.equal(out[:, :N], tc)
+    assert netmod.gemm_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(130, 24, 56), (256, 96, 864), (64, 128, 1152)])
+@pytest.mark.parametrize("act", [0, 1])
+def test_gemm_with_its_activation(shape, act):
+    """The fused epilogue against the separate kernels: bitwise."""
+    torch = pytest.importorskip("torch")
+    from cism_b200 import net as netmod
+
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    bias = torch.randn(N, generator=g, device="cuda")
+    z, z2 = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    y, y2, y3 = (torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    L, p, s = netmod.lib(), netmod._p, netmod._s()
+    assert L.bpnet_gemm_act(p(a), p(b), p(z), p(bias), p(y), M, N, K, K, K, act, s) == 0
+    assert L.bpnet_gemm_act(p(a), p(b), None, p(bias), p(y3), M, N, K, K, K, act, s) == 0
+    netmod.gemm_tn(a, b, z2, bias, M, N, K, K, K, N)
+    assert L.bpnet_act(p(z2), p(y2), M, N, N, 0, act, s) == 0
+    assert torch.equal(z, z2) and torch.equal(y, y2) and torch.equal(y, y3)
