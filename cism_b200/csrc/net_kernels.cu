@@ -964,11 +964,7 @@ __global__ void __launch_bounds__(128) k_gemm_tma(const __grid_constant__ CUtens
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
 }
 
-// The 2-D tensor map of a row-major BF16 operand, inner x outer elements with
-// rows of ld, in boxes of 64 inner elements (128 bytes, swizzled) by box_outer;
-// false where the driver has no encoder or refuses the operand (address or
-// stride not 16-byte aligned).
-bool tma_map(CUtensorMap* map, const void* ptr, int inner, int outer, int ld, int box_outer) {
+PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 enc = [] {
     void* f = nullptr;
     cudaDriverEntryPointQueryResult q;
@@ -977,6 +973,14 @@ bool tma_map(CUtensorMap* map, const void* ptr, int inner, int outer, int ld, in
       f = nullptr;
     return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
   }();
+  return enc;
+}
+// The 2-D tensor map of a row-major BF16 operand, inner x outer elements with
+// rows of ld, in boxes of 64 inner elements (128 bytes, swizzled) by box_outer;
+// false where the driver has no encoder or refuses the operand (address or
+// stride not 16-byte aligned).
+bool tma_map(CUtensorMap* map, const void* ptr, int inner, int outer, int ld, int box_outer) {
+  const auto enc = tma_encoder();
   if (!enc || (reinterpret_cast<uintptr_t>(ptr) & 15) || ((size_t)ld * 2) % 16) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
@@ -985,6 +989,267 @@ bool tma_map(CUtensorMap* map, const void* ptr, int inner, int outer, int ld, in
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// k_dgrad3's map, 64-byte swizzle: the weights [cout][Kp] in boxes of 32
+// columns by `rows` rows.
+bool dgrad_map(CUtensorMap* mw, const void* w, int C, int Kp, int K, int rows) {
+  const auto enc = tma_encoder();
+  if (!enc || (reinterpret_cast<uintptr_t>(w) & 15) || Kp % 8) return false;
+  const cuuint64_t dw[2] = {(cuuint64_t)K, (cuuint64_t)C}, sw[1] = {(cuuint64_t)Kp * 2};
+  const cuuint32_t bx[2] = {32, (cuuint32_t)rows}, e2[2] = {1, 1};
+  return enc(mw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(w), dw, sw, bx, e2,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// ---------------------------------------------------------------------
+// Input gradient of a 3 x 3 convolution: dX[p][c] = sum over taps, in tap
+// order, of (sum over o of dZ[q][o] w[o][tap * cin + c]), q the pixel whose
+// tap lands on p.
+//
+// As a product over all taps and a gather, its FP32 result (9 cin columns a
+// pixel) is written to memory and read back: 151 MB for 131,072 pixels of 32
+// channels.  Here a CTA takes 8 x 16 pixels by 32 NB input channels.  It
+// copies dZ's 10 x 18 pixels around them once, as planes of 8 channels (16
+// bytes a pixel): in that layout a tap's 128 shifted pixels are the same
+// operand from another start address (8 rows of 16 bytes lie together, the
+// next 8 one row of the copy on), wrapped or zero at the border as copied.
+// The weights, MN-major as they lie, follow in slices of 32 or 64 output channels.
+// For every tap the tensor core forms the tap's product in one of BUFS
+// accumulators while four warps add the last tap's to their sums in registers.
+// Same products in the same order as before: the result is bitwise that of
+// the product and the gather.  A fifth warp issues the multiplies, a sixth the copies.
+// Waits bounded as in k_gemm_tma.
+// Eight 128 x 128 grids with the L2 cold, product and gather -> here: 32 to 32
+// channels 132 -> 32 us, 96 to 32 431 -> 64; 64 x 64, 192 to 64 177 -> 38;
+// 32 x 32, 384 to 128 99 -> 28.  Its bytes take 4 to 9 us: it is bound by the
+// row of waits in a CTA (copy, nine taps, store), hidden by 2 to 4 CTAs an SM.
+// ---------------------------------------------------------------------
+constexpr int DG_W = 8, DG_H = 16, DG_PLANE = (DG_W + 2) * (DG_H + 2) * 16, DG_RING = 16384, DG_MAX_COUT = 256;
+constexpr int DG_BUFS = 2;
+constexpr int dg_cols(int nb) { return nb == 3 ? 256 : 64 * nb; }  // accumulator columns, a power of two
+// the ring of weights, dZ's planes; at least what keeps the CTAs of an SM
+// within its 512 accumulator columns
+constexpr int dg_smem_bytes(int nb, int cout) {
+  const int n = DG_RING * nb + cout / 8 * DG_PLANE + 1024, least = nb == 3 ? 80 * 1024 : nb == 2 ? 56 * 1024 : 0;
+  return n > least ? n : least;
+}
+
+// 64-byte swizzle, MN-major: groups of 8 K rows 512 bytes apart, groups of 32
+// columns `box`
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t addr, uint32_t box) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(box >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
+}
+// no swizzle, K-major: 8 channels on = the next plane, 8 rows on = the next row of the copy
+__device__ __forceinline__ uint64_t umma_desc_planes(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(DG_PLANE >> 4) << 16) |
+         ((uint64_t)((DG_W + 2) * 16 >> 4) << 32) | ((uint64_t)1 << 46);
+}
+
+// KR: output channels of a slice of weights; the ring holds DG_RING bytes per 32 columns.
+template <int NB, int KR>
+__global__ void __launch_bounds__(192, NB == 1 ? 4 : NB == 2 ? 3 : 2) k_dgrad3(const __grid_constant__ CUtensorMap tmW, const bf16* __restrict__ dZ,
+                                                float* __restrict__ dX, int H, int W, int cin, int cout,
+                                                int periodic) {
+  constexpr int BUFS = DG_BUFS, COLS = dg_cols(NB), BOX = KR * 64, STAGE = NB * BOX, STAGES = DG_RING / BOX;
+  extern __shared__ __align__(1024) uint8_t tc_smem[];
+  __shared__ __align__(8) uint64_t full[STAGES], done[STAGES], tap_done[BUFS], tap_free[BUFS];
+  __shared__ uint32_t tmem_slot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tx = (W + DG_W - 1) / DG_W;
+  const int x0 = ((int)blockIdx.x % tx) * DG_W, y0 = ((int)blockIdx.x / tx) * DG_H, b = blockIdx.y;
+  const int c0 = blockIdx.z * (32 * NB), ns = cout / KR;
+  const uint32_t ring = (smem_u32(tc_smem) + 1023u) & ~1023u, planes = ring + STAGES * STAGE;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                 "r"(COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 128) {
+    for (int i = 0; i < STAGES; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[i])));
+    }
+    for (int i = 0; i < BUFS; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&tap_done[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(smem_u32(&tap_free[i])));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp < 4) {
+    // a pixel outside the grid is its wrapped one or zeros
+    const int nc = cout >> 3;
+    for (int i = tid; i < (DG_W + 2) * (DG_H + 2) * nc; i += 128) {
+      const int px = i / nc, c8 = i - px * nc, hy = px / (DG_W + 2);
+      int y = y0 + hy - 1, x = x0 + (px - hy * (DG_W + 2)) - 1;
+      if (periodic) {
+        y = y < 0 ? H - 1 : y == H ? 0 : y;
+        x = x < 0 ? W - 1 : x == W ? 0 : x;
+      }
+      const bool in = y >= 0 && y < H && x >= 0 && x < W;
+      const bf16* src = in ? dZ + (((size_t)b * H + y) * W + x) * cout + c8 * 8 : dZ;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(planes + c8 * DG_PLANE + px * 16), "l"(src),
+                   "r"(in ? 16 : 0)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  bool ok = true;
+  float s[32 * NB];
+  if (warp == 5) {  // the copies of the weights
+    if (lane == 0) {
+      int st = 0, n = 0;  // slice n of stage st; its stage's use before ended at parity `par`
+      uint32_t par = 1;
+      for (int tap = 0; ok && tap < 9; ++tap)
+        for (int o0 = 0; o0 < cout; o0 += KR, ++n) {
+          const uint32_t bar = smem_u32(&full[st]);
+          if (n >= STAGES && !(ok = mbar_wait(smem_u32(&done[st]), par))) break;
+          mbar_expect_tx(bar, STAGE);
+#pragma unroll
+          for (int i = 0; i < NB; ++i)
+            tma_load_2d(ring + st * STAGE + i * BOX, &tmW, tap * cin + c0 + 32 * i, o0, bar);
+          if (++st == STAGES) {
+            st = 0;
+            par ^= 1;
+          }
+        }
+      // no copy may still be in flight when the CTA exits: the last one of each stage issued
+      const int last = n < STAGES ? n : STAGES;
+      for (int i = 0; i < last; ++i) {
+        const int j = n - 1 - i;
+        mbar_wait(smem_u32(&full[j % STAGES]), (j / STAGES) & 1);
+      }
+    }
+  } else if (warp == 4) {  // the multiplies
+    if (lane == 0) {
+      constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(32 * NB >> 3) << 17) |
+                                 ((uint32_t)(128 >> 4) << 24);
+      const uint64_t a0 = umma_desc_planes(planes), b0 = umma_desc_sw64(ring, BOX);
+      int st = 0, buf = 0, last = -1;
+      uint32_t par = 0, free_par = 1;  // (parities of full[st] and, from tap BUFS on, tap_free[buf])
+      for (int tap = 0; ok && tap < 9; ++tap) {
+        // the accumulator's last tap has been read
+        if (tap >= BUFS && !(ok = mbar_wait(smem_u32(&tap_free[buf]), free_par))) break;
+        // the tap (ty, tx) of the pixel (y - ty, x - tx) lands on (y, x); the copy
+        // starts at (y0 - 1, x0 - 1).  Descriptors count 16 bytes.
+        const uint64_t at = a0 + (uint32_t)((1 - (tap / 3 - 1)) * (DG_W + 2) + 1 - (tap % 3 - 1));
+        for (int sl = 0; sl < ns; ++sl) {
+          if (!(ok = mbar_wait(smem_u32(&full[st]), par))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int k = 0; k < KR / 16; ++k) {  // 16 output channels: two planes, two groups of 8 rows of w
+            const uint64_t ad = at + (uint32_t)((sl * (KR / 8) + k * 2) * (DG_PLANE / 16)),
+                           bd = b0 + (uint32_t)((st * STAGE + k * 1024) / 16);
+            const uint32_t acc = (sl > 0 || k > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem +
+                                                                                                      32 * NB * buf),
+                "l"(ad), "l"(bd), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+          }
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                           smem_u32(&done[st]))
+                       : "memory");
+          last = (st << 1) | (int)par;  // (a stage's uses of full and done have the same parity)
+          if (++st == STAGES) {
+            st = 0;
+            par ^= 1;
+          }
+        }
+        if (!ok) break;
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_u32(&tap_done[buf]))
+                     : "memory");
+        if (++buf == BUFS) {
+          buf = 0;
+          free_par ^= 1;
+        }
+      }
+      // no multiply may still be in flight when the CTA exits
+      if (last >= 0 && !mbar_wait(smem_u32(&done[last >> 1]), last & 1)) ok = false;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32 * NB; ++j) s[j] = 0.f;
+    const int m = warp * 32 + lane, y = y0 + m / DG_W, x = x0 + m % DG_W;
+    for (int tap = 0; tap < 9; ++tap) {
+      const int buf = tap % BUFS;
+      // one lane asks: 128 of them asking keep shared memory from the fifth warp
+      if (lane == 0) ok = mbar_wait(smem_u32(&tap_done[buf]), (tap / BUFS) & 1);
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // a pixel outside the grid adds nothing, whatever the weights are
+      const int yq = y - (tap / 3 - 1), xq = x - (tap % 3 - 1);
+      const bool in = periodic || (yq >= 0 && yq < H && xq >= 0 && xq < W);
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+        uint32_t v[32];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+            "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+              "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),
+              "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),
+              "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+            : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(32 * NB * buf + 32 * n)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (n == NB - 1) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tap_free[buf])) : "memory");
+        }
+        if (in) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) s[32 * n + j] += __uint_as_float(v[j]);
+        }
+      }
+    }
+  }
+  ok = __syncthreads_and(ok);
+  if (ok && warp < 4) {
+    // warp w: pixels 32w .. 32w + 31 of the rectangle, through the ring's and
+    // the planes' memory so that a store writes one pixel's 32 channels
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    float* T = reinterpret_cast<float*>(tc_smem + (ring - smem_u32(tc_smem))) + warp * (32 * 33);
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) T[lane * 33 + j] = s[32 * n + j];
+      __syncwarp();
+#pragma unroll 4
+      for (int r = 0; r < 32; ++r) {
+        const int m = warp * 32 + r, y = y0 + m / DG_W, x = x0 + m % DG_W;
+        if (y < H && x < W) dX[(((size_t)b * H + y) * W + x) * cin + c0 + 32 * n + lane] = T[r * 33 + lane];
+      }
+      __syncwarp();
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS));
+}
+
+template <int NB, int KR>
+int launch_dgrad3(const void* dZ, const void* w, float* dX, int B, int H, int W, int cin, int cout, int Kp,
+                  int periodic, cudaStream_t st) {
+  static_assert(4 * 32 * 33 * 4 <= DG_RING + 4 * DG_PLANE, "room for the result's transposition");
+  static const bool ok = cudaFuncSetAttribute(k_dgrad3<NB, KR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              dg_smem_bytes(NB, DG_MAX_COUT)) == cudaSuccess;
+  CUtensorMap mw;
+  if (!ok) return 6;
+  if (!dgrad_map(&mw, w, cout, Kp, 9 * cin, KR)) return 10;
+  const dim3 grid((unsigned)(((W + DG_W - 1) / DG_W) * ((H + DG_H - 1) / DG_H)), B, cin / (32 * NB));
+  k_dgrad3<NB, KR><<<grid, 192, dg_smem_bytes(NB, cout), st>>>(mw, (const bf16*)dZ, dX, H, W, cin, cout, periodic);
+  return cudaGetLastError() == cudaSuccess ? 0 : 6;
 }
 
 // C[r][c] = sum over z of part[z][r][c] in z order (+ bias) (+ C): the
@@ -1303,6 +1568,33 @@ int bpnet_act_grad_sum(const float* Z, const float* dY, void* dZb, float* db, fl
   k_colsum_rows<<<dim3(32, (C + 31) / 32), dim3(32, 8), 0, st>>>(scratch, part, P, C);
   k_colsum_tree<<<C, 256, 0, st>>>(part, db, C);
   return cudaGetLastError() == cudaSuccess ? 0 : 6;
+}
+
+// dX [B][H][W][cin] (FP32) of a 3 x 3 convolution with weights [cout][Kp] from
+// dZ [B][H][W][cout].  10 for what it does not take: channels that are not
+// multiples of 32, more output channels than shared memory holds, operands
+// that are not 16-byte aligned, another GEMM kernel selected, few pixels.
+int bpnet_dgrad3(const void* dZ, const void* w, float* dX, int B, int H, int W, int cin, int cout, int Kp, int periodic,
+                 void* stream) {
+  if (B <= 0 || H <= 0 || W <= 0 || cin <= 0 || cout <= 0) return 10;
+  if (cin % 32 || cout % 32 || cout > DG_MAX_COUT || Kp < 9 * cin || B > 65535 || cin / 32 > 65535) return 10;
+  if (!aligned(dZ, 16) || gemm_mode() != 0) return 10;
+  const long long tiles = (long long)((W + DG_W - 1) / DG_W) * ((H + DG_H - 1) / DG_H);
+  if (tiles > 0x7fffffffLL) return 10;
+  // few CTAs with a long row of slices: the product over all taps spreads wider
+  // (16 x 16 pixels, 256 to 256 channels: 17 us against 29; at 128 CTAs equal)
+  if (cout > 128 && tiles * B * (cin / 32) < 128) return 10;
+  // the widest tile that gives every SM a CTA: 128 x 128 x 8 pixels, 96 to 32
+  // channels, 64 us with 96 columns and 77 with 32; 64 x 64 x 8, 192 to 64, 38 and 48
+  int nb = 1;
+  for (int n = 3; n > 1; --n)
+    if (cin % (32 * n) == 0 && tiles * B * (cin / (32 * n)) >= 148) {
+      nb = n;
+      break;
+    }
+  const auto f = cout % 64 == 0 ? (nb == 3 ? launch_dgrad3<3, 64> : nb == 2 ? launch_dgrad3<2, 64> : launch_dgrad3<1, 64>)
+                                : (nb == 3 ? launch_dgrad3<3, 32> : nb == 2 ? launch_dgrad3<2, 32> : launch_dgrad3<1, 32>);
+  return f(dZ, w, dX, B, H, W, cin, cout, Kp, periodic, (cudaStream_t)stream);
 }
 
 int bpnet_to_bf16(const float* x, void* y, long long n, void* stream) {

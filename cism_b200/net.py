@@ -53,6 +53,7 @@ def lib():
             "bpnet_act": [vp, vp, ll, i, i, i, i, vp],
             "bpnet_act_grad": [vp, vp, vp, ll, i, i, i, i, vp],
             "bpnet_act_grad_sum": [vp, vp, vp, vp, vp, ll, i, i, vp],
+            "bpnet_dgrad3": [vp, vp, vp, i, i, i, i, i, i, i, vp],
             "bpnet_to_bf16": [vp, vp, ll, vp],
             "bpnet_colsum": [vp, vp, ll, i, vp],
             "bpnet_pool": [vp, vp, i, i, i, i, vp],
@@ -212,6 +213,13 @@ class Conv:
         self.saved = None
         if not need_dx:
             return None
+        if self.k3:
+            dx = torch.empty((P, self.cin), dtype=torch.float32, device=dy.device)
+            rc = lib().bpnet_dgrad3(_p(dzb), _p(self.wb), _p(dx), B, H, W, self.cin, self.cout, self.Kp,
+                                    periodic, _s())
+            if rc != 10:
+                _ck(rc, "dgrad3")
+                return dx
         dcol = torch.empty((P, self.Kp), dtype=torch.float32, device=dy.device)
         if not gemm_major(False, True, dzb, self.wb, dcol, P, self.Kp, self.cout, self.cout, self.Kp, self.Kp):
             gemm_tn(dzb, transpose(self.wb), dcol, None, P, self.Kp, self.cout, self.cout, self.cout, self.Kp)

@@ -363,3 +363,32 @@ def test_gemm_with_its_activation(shape, act):
     netmod.gemm_tn(a, b, z2, bias, M, N, K, K, K, N)
     assert L.bpnet_act(p(z2), p(y2), M, N, N, 0, act, s) == 0
     assert torch.equal(z, z2) and torch.equal(y, y2) and torch.equal(y, y3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("periodic", [0, 1])
+@pytest.mark.parametrize("shape", [(1, 8, 8, 32, 32), (2, 13, 26, 64, 96), (1, 130, 6, 32, 64), (1, 2, 200, 96, 32),
+                                   (3, 64, 48, 192, 256), (1, 104, 184, 96, 32), (1, 104, 184, 64, 64),
+                                   (1, 1, 1, 32, 32)])
+def test_direct_input_gradient(shape, periodic):
+    """The input gradient formed tap by tap in one kernel against the product
+    over all taps and the gather: bitwise (the same products, the same order);
+    rectangles that end outside the grid, single-row and single-slice cases,
+    wrapped and zero borders."""
+    torch = pytest.importorskip("torch")
+    from cism_b200 import net as netmod
+
+    B, H, W, cin, cout = shape
+    P, Kp = B * H * W, 9 * cin
+    g = torch.Generator(device="cuda").manual_seed(P)
+    L, p, s = netmod.lib(), netmod._p, netmod._s()
+    dzb = torch.randn(P, cout, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(cout, Kp, generator=g, device="cuda").to(torch.bfloat16)
+    dx = torch.full((P, cin), float("nan"), device="cuda")
+    assert L.bpnet_dgrad3(p(dzb), p(w), p(dx), B, H, W, cin, cout, Kp, periodic, s) == 0
+    dcol = torch.empty(P, Kp, device="cuda")
+    assert netmod.gemm_major(False, True, dzb, w, dcol, P, Kp, cout, cout, Kp, Kp)
+    ref = torch.empty(P, cin, device="cuda")
+    assert L.bpnet_col2im(p(dcol), p(ref), B, H, W, cin, Kp, periodic, s) == 0
+    assert torch.equal(dx, ref)
+    assert netmod.gemm_status() == 0
