@@ -298,7 +298,7 @@ DevView make_view(Arena& a, cudaStream_t s, const HostPlan& p, bool with_cells, 
     v.A32 = blk;
     v.A32d = reinterpret_cast<double2*>(blk + 14 * np);
   }
-  v.partials = a.get<double>(s, "partials", 3 * (size_t)std::max(p.ntiles, 1));
+  v.partials = a.get<double>(s, "partials", 3 * (size_t)std::max(p.ntiles, 1) + 1);  // read in pairs
   v.tile_counter = a.get<unsigned>(s, "tile_counter", p.ninst);
   CK(cudaMemsetAsync(v.tile_counter, 0, sizeof(unsigned) * p.ninst, s));
   return v;
@@ -576,7 +576,8 @@ void autotune(bp_problem* P) {
     }
   }
   const int variant = P->plan.inst.empty() ? 0 : P->plan.inst[0].variant;
-  const auto key = std::make_tuple(P->plan.nnodes >> 14, P->plan.nz, v.sym, v.A32 ? 1 : 0, variant);
+  const bool batch = P->plan.ninst > 1;
+  const auto key = std::make_tuple(P->plan.nnodes >> 14, 2 * P->plan.nz + batch, v.sym, v.A32 ? 1 : 0, variant);
   auto it = c->tuned.find(key);
   if (it != c->tuned.end()) {
     v.minb = it->second[0];
@@ -617,7 +618,11 @@ void autotune(bp_problem* P) {
       const int res = krylov_resident_ctas(v, mode, mb);
       if (res <= 0) continue;
       for (int g : {0, res * c->num_sms}) {
-        if (g > 0 && g >= P->plan.ntiles) continue;
+        // a batch's instances end at different iterations, and a persistent
+        // CTA walks past the tiles of those that have (16 domains: 102 us an
+        // iteration against 98 with a CTA per tile, which the dry pass, all
+        // instances solving, times 1 us slower)
+        if (g > 0 && (g >= P->plan.ntiles || batch)) continue;
         v.minb_k = mb;
         v.grid_k = g;
         const float ms = time_launches(c, [&] { launch_mv(mode, v, c->stream); });

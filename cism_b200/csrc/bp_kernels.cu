@@ -55,7 +55,10 @@ __device__ __forceinline__ void block_reduce(double (&val)[NV], double* sm) {
 
 // Reduce NV values of this tile; the last tile of the instance sums all
 // tile partials of the instance in tile order and calls fin(inst, sums).
-template <int NV, bool MAX0, typename Fin>
+// U: tiles whose partials a thread has in flight there, where the kernel has
+// registers to spare (k_std_update: 15.3 -> 14.1 us at 1,600 tiles; k_resid
+// loses more to its occupancy than the tail gains, 53 -> 66 us).
+template <int NV, bool MAX0, int U = 1, typename Fin>
 __device__ __forceinline__ void tile_finish(const DevView& v, int t, int inst,
                                             double (&val)[NV], Fin fin) {
   __shared__ double sm[NV * 32];
@@ -77,12 +80,21 @@ __device__ __forceinline__ void tile_finish(const DevView& v, int t, int inst,
     double s[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) s[i] = 0.0;
-    for (int tt = ip.tile_begin + threadIdx.x; tt < ip.tile_end; tt += blockDim.x)
+    for (int t0 = ip.tile_begin + threadIdx.x; t0 < ip.tile_end; t0 += U * blockDim.x) {
+      double p[U][NV];
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const double p = __ldcg(v.partials + (size_t)i * v.ntiles + tt);
-        s[i] = (MAX0 && i == 0) ? fmax(s[i], p) : s[i] + p;
-      }
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const int tt = t0 + u * blockDim.x;
+          p[u][i] = U == 1 || tt < ip.tile_end ? __ldcg(v.partials + (size_t)i * v.ntiles + tt) : 0.0;
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (U == 1 || t0 + u * (int)blockDim.x < ip.tile_end)
+#pragma unroll
+          for (int i = 0; i < NV; ++i) s[i] = (MAX0 && i == 0) ? fmax(s[i], p[u][i]) : s[i] + p[u][i];
+    }
     block_reduce<NV, MAX0>(s, sm);
     if (threadIdx.x == 0) {
       v.tile_counter[inst] = 0;
@@ -803,7 +815,7 @@ __global__ void __launch_bounds__(kTile) k_std_update(DevView v) {
       }
     }
     if (!CHECK) {
-      tile_finish<2, false>(v, t, R.inst, part, [&](int inst, const double* s) {
+      tile_finish<2, false, 4>(v, t, R.inst, part, [&](int inst, const double* s) {
         std_update_fin<true>(v, v.inst[inst], v.st[inst], s);
       });
     }
@@ -1513,8 +1525,14 @@ __global__ void __launch_bounds__(PER_SM == 2 ? 192 : kTile, PER_SM) k_pcg_resid
 // of the neighbours' rows in registers and load the next tile's into the
 // same registers as they use this one's.  Sums: each warp stores its
 // tile's, and the CTA adds them, in block_reduce's order, and takes its
-// tickets once, after its last tile.  The arithmetic and its order are the
-// per-node kernels' (bitwise the same results).
+// tickets once, after its last tile.  What follows the last ticket is a chain
+// that no other work hides, so it is kept short: one ticket per warp and
+// instance, an instance's partials fetched to shared memory in one flight
+// instead of a few a thread, the next instance's meanwhile, and the scalar
+// updates of all instances side by side (a tail of 41 -> 13 us with four
+// instances of 2,460 tiles, 20 -> 10 with one of 5,980, 45 -> 15 with 16 of
+// 220).  The arithmetic and its order are the per-node kernels' (bitwise the
+// same results).
 //
 // Barriers, all waits bounded (past the limit the CTA marks the instances'
 // sums as NaN, which ends their solve with BP_ERR_NAN): full[stage] -- the
@@ -1524,12 +1542,14 @@ __global__ void __launch_bounds__(PER_SM == 2 ? 192 : kTile, PER_SM) k_pcg_resid
 //
 // What bounds it: the consumers, six warps a tile (one CTA an SM in FP64,
 // whose two stages are 177 KB; two in FP32), wait on shared memory and on
-// their own chains; DRAM is at 0.6-0.65 of the copy bandwidth in FP64.
+// their own chains; DRAM is at 0.65 of the copy bandwidth in FP64 and L2
+// hands the SMs 8 of the 10 TB/s that it can (the matrix twice, as own rows
+// and as the neighbours').
 // Measured, the fastest per-node shape -> this kernel, a launch of
 // k_cg_mv's work: 400 x 400 x 11 marine sheet, FP64 (1.05 M nodes) 156 ->
-// 123 us; 160 x 160 x 11 slab, FP64, standard PCG 46.5 -> 37.7 us; four
-// 256 x 256 x 11 sheets, FP32 (1.73 M nodes) 172 -> 160 us; 16 uneven domains,
-// FP32 (0.62 M nodes) 65 -> 79 us.  The autotuner times both on the problem.
+// 115 us; 160 x 160 x 11 slab, FP64, standard PCG 46.5 -> 36.5 us; four
+// 256 x 256 x 11 sheets, FP32 (1.73 M nodes) 172 -> 145 us; 16 uneven domains,
+// FP32 (0.62 M nodes) 65 -> 68 us.  The autotuner times both on the problem.
 // ---------------------------------------------------------------------
 constexpr int kStages = 2, kDescs = 4;
 
@@ -1681,16 +1701,26 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
   __syncthreads();
   pdl_wait();
   pdl_launch_next();
-  // the CTA's tiles: every G-th, of the instances that are solving
-  auto next_tile = [&](int t) {
-    for (; t < v.ntiles; t += G)
-      if (v.dry || v.st[v.tile_inst[t]].pcg_active) return t;
-    return -1;
-  };
   bool ok = true;
 
   if (warp == nw) {  // producer
-    int tn = next_tile(blockIdx.x);  // the next tile whose descriptor is fetched
+    // the CTA's tiles: every G-th, of the instances that are solving, looked up
+    // 32 at a time (a tile at a time, a batch with few instances left passed
+    // the others' tiles at two trips to L2 each)
+    unsigned live = 0;  // of the 32 from tile t32 on, those still to come
+    long t32 = (long)blockIdx.x - 32L * G;
+    auto next_tile = [&]() {
+      while (live == 0) {
+        t32 += 32L * G;
+        if (t32 >= v.ntiles) return -1;
+        const long t = t32 + (long)lane * G;
+        live = __ballot_sync(0xffffffffu, t < v.ntiles && (v.dry || v.st[v.tile_inst[t]].pcg_active));
+      }
+      const int q = __ffs(live) - 1;
+      live &= live - 1;
+      return (int)(t32 + (long)q * G);
+    };
+    int tn = next_tile();  // the next tile whose descriptor is fetched
     auto fetch = [&](int j) {        // descriptor j of the sequence (after the last: tile -1)
       unsigned char* d = descs + (j % kDescs) * H.desc;
       if (lane == 0) {
@@ -1702,7 +1732,7 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
           bar_arrive(dfull(j % kDescs));
         }
       }
-      if (tn >= 0) tn = next_tile(tn + G);
+      if (tn >= 0) tn = next_tile();
     };
     fetch(0);
     fetch(1);
@@ -1882,7 +1912,27 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
   // tile the instance's sums (tile_finish's order) and scalar update
   const bool all_ok = __syncthreads_and(ok);
   __shared__ double sm[NV * 32];
-  __shared__ int last;
+  constexpr int kFins = 32;
+  __shared__ int fins[kFins], nfin;
+  __shared__ double fin_sum[kFins][NV];
+  const int bd = v.tile_threads;  // the threads tile_finish sums with
+  // the stages are free: two halves, each for the partials of every sum of
+  // `chunk` tiles (three more for alignment), whole rounds of bd
+  double* buf = reinterpret_cast<double*>(st_sm);
+  const int chunk = ((int)(H.stage / (8 * NV)) - 3) / bd * bd, pitch = (chunk + 3) & ~1;
+  auto stage_partials = [&](int c0, int end, int half) {  // by 16-byte copies
+    const int n = end - c0 < chunk ? end - c0 : chunk;
+#pragma unroll
+    for (int e = 0; e < NV; ++e) {
+      const size_t at = (size_t)e * v.ntiles + c0, at0 = at & ~(size_t)1;
+      const int n16 = (int)((at + n - at0 + 1) >> 1);
+      for (int q = i; q < n16; q += blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_at(buf + (half * NV + e) * pitch + 2 * q)),
+                     "l"(v.partials + at0 + 2 * q)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
   for (int base = blockIdx.x; base < v.ntiles; base += G * blockDim.x) {
     const long tl = (long)base + (long)i * G;
     const int t = tl < v.ntiles ? (int)tl : -1;
@@ -1899,50 +1949,92 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
           v.partials[(size_t)e * v.ntiles + t] = all_ok ? x : __longlong_as_double(0x7ff8000000000000LL);
         }
         __threadfence();
-        const InstParams& ip = v.inst[inst];
-        done = atomicAdd(&v.tile_counter[inst], 1u) == (unsigned)(ip.tile_end - ip.tile_begin) - 1u;
+      } else {
+        inst = -1;
       }
     }
-    while (__syncthreads_or(done)) {
-      if (done) last = i;  // any one of them
+    // one ticket for a warp's tiles of an instance (thousands of atomics on
+    // one address, all at the end, are a queue)
+    const unsigned same = __match_any_sync(0xffffffffu, inst);
+    __syncwarp();
+    if (inst >= 0 && lane == __ffs(same) - 1) {
+      const InstParams& ip = v.inst[inst];
+      const unsigned cnt = __popc(same);
+      done = atomicAdd(&v.tile_counter[inst], cnt) + cnt == (unsigned)(ip.tile_end - ip.tile_begin);
+    }
+    // the instances whose last tickets came to this CTA, a list at a time:
+    // their sums one after the other, each thread in tile_finish's order, the
+    // next one's partials on their way meanwhile, then the scalar updates
+    // side by side
+    for (;;) {
+      if (i == 0) nfin = 0;
       __syncthreads();
-      const int who = last;
-      __syncthreads();
-      if (i == who) {
-        last = inst;
-        done = 0;
+      if (done) {
+        const int p = atomicAdd(&nfin, 1);
+        if (p < kFins) {
+          fins[p] = inst;
+          done = 0;
+        }
       }
       __syncthreads();
-      const int fin = last;
+      const int nf = nfin < kFins ? nfin : kFins;
+      if (nf == 0) break;
       __threadfence();
-      const InstParams& ip = v.inst[fin];
-      const int bd = v.tile_threads;  // the threads tile_finish sums with
+      // what the updates read, on its way meanwhile
+      constexpr int kLines = (sizeof(InstState) + 63) / 64;
+      for (int q = i; q < nf * kLines; q += blockDim.x)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(v.st + fins[q / kLines]) +
+                                                      64 * (q % kLines)));
       double x[NV];
 #pragma unroll
       for (int e = 0; e < NV; ++e) x[e] = 0.0;
-      constexpr int U = 4;
-      if (i < bd)
-        for (int t0 = ip.tile_begin + i; t0 < ip.tile_end; t0 += U * bd) {
-          double p[U][NV];
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int e = 0; e < NV; ++e)
-              p[u][e] = t0 + u * bd < ip.tile_end ? __ldcg(v.partials + (size_t)e * v.ntiles + t0 + u * bd) : 0.0;
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            if (t0 + u * bd < ip.tile_end)
-#pragma unroll
-              for (int e = 0; e < NV; ++e) x[e] += p[u][e];
+      int f = 0, c0 = v.inst[fins[0]].tile_begin, end = v.inst[fins[0]].tile_end, half = 0;
+      stage_partials(c0, end, 0);
+      while (f < nf) {
+        const int n = end - c0 < chunk ? end - c0 : chunk;
+        int f1 = f, c1 = c0 + chunk, end1 = end;
+        if (c1 >= end && ++f1 < nf) {
+          c1 = v.inst[fins[f1]].tile_begin;
+          end1 = v.inst[fins[f1]].tile_end;
         }
-      block_reduce<NV, false>(x, sm);
-      if (i == 0) {
-        v.tile_counter[fin] = 0;
+        if (f1 < nf) {
+          stage_partials(c1, end1, half ^ 1);
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        if (i < bd)
+#pragma unroll
+          for (int e = 0; e < NV; ++e) {
+            const double* p = buf + (half * NV + e) * pitch + (((size_t)e * v.ntiles + c0) & 1);
+#pragma unroll 4
+            for (int t = i; t < n; t += bd) x[e] += p[t];
+          }
+        if (f1 != f) {
+          block_reduce<NV, false>(x, sm);
+#pragma unroll
+          for (int e = 0; e < NV; ++e) {
+            if (i == 0) fin_sum[f][e] = all_ok ? x[e] : __longlong_as_double(0x7ff8000000000000LL);
+            x[e] = 0.0;
+          }
+        }
+        __syncthreads();
+        f = f1;
+        c0 = c1;
+        end = end1;
+        half ^= 1;
+      }
+      if (i < nf) {
+        const int in = fins[i];
+        v.tile_counter[in] = 0;
         if (!v.dry) {
-          if (MODE == MV_STD_A) std_mv_fin<true>(v, v.st[fin], x);
-          else cg_mv_fin<MODE == MV_CG_FIRST, true>(v, v.inst[fin], v.st[fin], x);
+          double x[NV];
+#pragma unroll
+          for (int e = 0; e < NV; ++e) x[e] = fin_sum[i][e];
+          if (MODE == MV_STD_A) std_mv_fin<true>(v, v.st[in], x);
+          else cg_mv_fin<MODE == MV_CG_FIRST, true>(v, v.inst[in], v.st[in], x);
         }
-        __threadfence();
       }
       __syncthreads();
     }

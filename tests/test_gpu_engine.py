@@ -287,3 +287,32 @@ def test_matvec_of_a_callers_matrix(ctx, dims):
     rows = (own & (av != 0))[..., None]
     assert np.max(np.abs(yu - np.where(rows, eu, 0.0))) <= 1e-12
     assert np.max(np.abs(yv - np.where(rows, ev, 0.0))) <= 1e-12
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("variant", [configs.SPARSE_PCG_STANDARD, configs.SPARSE_PCG_CHRONGEAR])
+def test_staged_sums_of_many_and_of_large_instances(ctx, variant, mixed):
+    """The staged matvec's last CTA: 45 instances whose sums all end in one CTA
+    (more than one list of 32, more tiles than threads), and an instance whose
+    partials pass shared memory in several chunks.  Bitwise the per-node
+    kernels' solves, as above."""
+    many = [configs.slab(n=22 + i % 3, nz=11) for i in range(45)]
+    for ms, grid in ((many, 1), ([configs.slab(n=250, nz=11)], 0)):
+        ms = [m.copy(which_sparse=variant, which_precond=configs.PRECOND_SIA, pcg_tol=1e-6, pcg_maxiters=6 + i % 4,
+                     maxiter_nonlinear=1) for i, m in enumerate(ms)]
+        preps = [solver.prepare(m, precision=solver.MIXED if mixed else solver.FP64)[0] for m in ms]
+        zero = [np.zeros(m.vshape3) for m in ms]
+        got = []
+        for config in ("0,0,0,0,0", f"0,0,0,{grid},1"):
+            with _Env(BP_MV_CONFIG=config):
+                prob = ctx.problem(preps)
+                prob.set_guess(zero, zero)
+                st = prob.run()
+                u, v, _ = prob.get()
+                prob.close()
+            got.append((u, v, st))
+        for a, b in zip(got[0][:2], got[1][:2]):
+            assert all(np.array_equal(x, y) for x, y in zip(a, b))
+        keys = ("status", "pcg_iters_total", "refine_steps_total", "pcg_err_last", "L2_norm")
+        for s, r in zip(got[0][2], got[1][2]):
+            assert {k: s[k] for k in keys} == {k: r[k] for k in keys}
