@@ -563,7 +563,7 @@ def run_ours(args, D):
     achieved = total_bytes / (kp["t_mv_ms"] / 1000.0) / 1e9 if kp["n_mv"] else 0.0
     tr = committed_traffic("mixed" if hp.mixed else "fp64")
     roof = {"bound": "hbm",
-            "kernel": "%s (Krylov matvec, thread per node, %s)" % (
+            "kernel": "%s or k_mv_staged, as tuned (Krylov matvec, thread per node, %s)" % (
                 "k_cg_mv" if hp.describe(models[0])["pcg"] == "chronopoulos_gear" else "k_std_mv",
                 "FP32 half storage + compensated FP64 diagonal" if hp.mixed else "FP64 half storage"),
             "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
