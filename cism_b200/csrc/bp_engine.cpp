@@ -584,7 +584,7 @@ void autotune(bp_problem* P) {
     v.grid_cap = it->second[1];
     v.minb_k = it->second[2];
     v.grid_k = it->second[3];
-    v.staged = it->second[4];
+    v.staged = it->second[4] && v.desc ? 1 : 0;
     return;
   }
   const bool log = std::getenv("BP_TUNE_LOG") != nullptr;

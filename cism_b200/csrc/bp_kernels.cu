@@ -2346,6 +2346,28 @@ static void launch_resid_minb(int mode, const DevView& v, cudaStream_t s, int g)
   if (v.minb == 4) launch_resid_store<STORE, 4>(mode, v, s, g);
   else launch_resid_store<STORE, 0>(mode, v, s, g);
 }
+// CTAs of `threads` threads and `smem` bytes of dynamic shared memory that an
+// SM holds of kernel k (0: none, or an error).  The kernel is first allowed all
+// that a block may have: that limit is one value per kernel and device for the
+// whole process, so it is never the size one problem needs -- a problem made
+// later, on this thread or another, would lower it under the launches of those
+// that are alive.
+static int ctas_per_sm(TileKernel k, int threads, size_t smem) {
+  int dev = 0, most = 0, n = 0;
+  cudaFuncAttributes fa;
+  if (cudaGetDevice(&dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+      cudaFuncGetAttributes(&fa, k) == cudaSuccess) {
+    const int room = most - (int)fa.sharedSizeBytes;
+    if (smem <= (size_t)room &&
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, room) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) == cudaSuccess)
+      return n;
+  }
+  cudaGetLastError();
+  return 0;
+}
+
 template <int STORE, int THREADS, int LS>
 static TileKernel staged_kernel_st(int mode) {
   switch (mode) {
@@ -2365,13 +2387,8 @@ int staged_per_sm(const DevView& v) {
   const StagedShape h = staged_shape(v, v.A32 != nullptr);
   int least = 0;
   for (int mode : {(int)MV_STD_A, (int)MV_CG_FIRST, (int)MV_CG1}) {
-    TileKernel k = staged_kernel(v, mode);
-    int n = 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.bytes) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, v.tile_threads + 32, h.bytes) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
+    const int n = ctas_per_sm(staged_kernel(v, mode), v.tile_threads + 32, h.bytes);
+    if (n == 0) return 0;
     least = least == 0 ? n : (n < least ? n : least);
   }
   return least;
@@ -2426,13 +2443,7 @@ static TileKernel resident_kernel(const DevView& v, int variant, size_t* smem) {
 int resident_ctas(const DevView& v, int variant, int num_sms) {
   size_t smem = 0;
   TileKernel k = resident_kernel(v, variant, &smem);
-  int n = 0;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, v.tile_threads, smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return n * num_sms;
+  return ctas_per_sm(k, v.tile_threads, smem) * num_sms;
 }
 cudaError_t launch_pcg_resident(const DevView& v, int variant, cudaStream_t s) {
   size_t smem = 0;
