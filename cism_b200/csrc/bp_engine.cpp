@@ -390,12 +390,14 @@ int max_pcg_iters(const HostPlan& p) {
   return m;
 }
 
-// Launch with optional event timing.
+// Launch with optional event timing.  A refused launch is an error at once: a
+// capture that went on without it would leave a graph that lacks the kernel.
 template <typename F>
 void L(bp_problem* P, int cat, F&& f) {
   Timing& T = P->timing;
   if (!T.on) {
     f();
+    CK(cudaGetLastError());
     return;
   }
   const size_t i = T.cat.size();
@@ -407,6 +409,7 @@ void L(bp_problem* P, int cat, F&& f) {
   }
   CK(cudaEventRecord(T.pool[i].first, P->c->stream));
   f();
+  CK(cudaGetLastError());
   CK(cudaEventRecord(T.pool[i].second, P->c->stream));
   T.cat.push_back(cat);
 }
@@ -455,7 +458,13 @@ void enqueue_chunk(bp_problem* P, int variant, int ncheck) {
     if (!P->chunk_graph) {
       cudaGraph_t g;
       CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      for (int j = 0; j < ncheck; ++j) enqueue_iteration(P, variant, j == ncheck - 1);
+      try {
+        for (int j = 0; j < ncheck; ++j) enqueue_iteration(P, variant, j == ncheck - 1);
+      } catch (const CudaError&) {  // the capture ends with the error
+        if (cudaStreamEndCapture(s, &g) == cudaSuccess) cudaGraphDestroy(g);
+        cudaGetLastError();
+        throw;
+      }
       CK(cudaStreamEndCapture(s, &g));
       CK(cudaGraphInstantiate(&P->chunk_graph, g, 0));
       CK(cudaGraphDestroy(g));
@@ -768,6 +777,7 @@ bool build_loop_graph(bp_problem* P, bool pdl) {
     CK(cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, mode));
     capturing = true;
     launch_loop_cond(hP, v, true, it, cap_picard, true, s);
+    CK(cudaGetLastError());
     CK(cudaStreamEndCapture(s, &g));
     capturing = false;
     cudaGraphNode_t start;
@@ -791,6 +801,7 @@ bool build_loop_graph(bp_problem* P, bool pdl) {
     } else {
       pcg_head(P);
       launch_loop_cond(hK, v, false, it + 1, cap_chunks, true, s);
+      CK(cudaGetLastError());
     }
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t* deps = nullptr;
@@ -813,6 +824,7 @@ bool build_loop_graph(bp_problem* P, bool pdl) {
       capturing = true;
       for (int j = 0; j < ncheck; ++j) enqueue_iteration(P, variant, j == ncheck - 1);
       launch_loop_cond(hK, v, false, it + 1, cap_chunks, false, s);
+      CK(cudaGetLastError());
       CK(cudaStreamEndCapture(s, &bK));
       capturing = false;
       last.assign(1, wK);
@@ -822,6 +834,7 @@ bool build_loop_graph(bp_problem* P, bool pdl) {
     capturing = true;
     picard_tail(P);
     launch_loop_cond(hP, v, true, it, cap_picard, false, s);
+    CK(cudaGetLastError());
     CK(cudaStreamEndCapture(s, &bP));
     capturing = false;
     ok = cudaGraphInstantiate(&P->loop_graph, g, 0) == cudaSuccess;

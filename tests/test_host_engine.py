@@ -1,0 +1,97 @@
+"""CPU tests of the host engine (cism_b200/csrc/bp_engine.cpp) on a fake CUDA
+runtime (tests/hostemu/hostengine.cpp): "device" memory is host memory, every
+linear solve and Picard loop ends at its first update, and launches can be
+refused, to see what the engine makes of an error code."""
+import ctypes as C
+import os
+
+import numpy as np
+import pytest
+
+from cism_b200 import configs, solver
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+_dp = solver._dp
+OK, ERR_CUDA, ERR_ARGS = 0, 6, 10
+
+
+class Engine:
+    """The few calls of the C ABI that the tests need, on the fake."""
+
+    def __init__(self):
+        self.L = C.CDLL(os.path.join(ROOT, "tests", "hostemu", "libhostengine.so"))
+        self.L.fake_nonzero_holes.restype = C.c_long
+        self.L.bp_last_error.restype = C.c_char_p
+        self.L.fake_refuse(0)
+        self.h = C.c_void_p()
+        assert self.L.bp_create(0, C.byref(self.h)) == OK
+
+    def close(self):
+        assert self.L.bp_destroy(self.h) == OK
+
+    def problem(self, models, **kw):
+        preps = [solver.prepare(m, **kw)[0] for m in models]
+        arr = (solver.Inputs * len(preps))(*[p.inputs for p in preps])
+        P = C.c_void_p()
+        assert self.L.bp_problem_create(self.h, len(preps), arr, C.byref(P)) == OK
+        return P
+
+    @staticmethod
+    def ptrs(arrays):
+        return (_dp * len(arrays))(*[C.cast(None, _dp) if a is None else a.ctypes.data_as(_dp) for a in arrays])
+
+    def set_guess(self, P, us, vs):
+        return self.L.bp_problem_set_guess(P, self.ptrs(us), self.ptrs(vs))
+
+    def run(self, P, n=1):
+        return self.L.bp_problem_run(P, (solver.Stats * n)())
+
+    def free(self, P):
+        self.L.bp_problem_destroy(P)
+
+
+@pytest.fixture()
+def eng():
+    e = Engine()
+    yield e
+    e.close()
+
+
+def _slab(n, nz=11, **kw):
+    return configs.slab(n=n, nz=nz).copy(maxiter_nonlinear=2, **kw)
+
+
+def _zero(m):
+    return [np.zeros(m.vshape3)], [np.zeros(m.vshape3)]
+
+
+@pytest.mark.parametrize("variant", [configs.SPARSE_PCG_STANDARD, configs.SPARSE_PCG_CHRONGEAR])
+@pytest.mark.parametrize("precision", [solver.FP64, solver.MIXED])
+def test_refused_launch_in_a_capture_ends_the_run(eng, variant, precision):
+    """A Krylov matvec that is refused while a graph is captured: the run ends
+    with BP_ERR_CUDA, nothing captured without it is launched, then or later,
+    and no capture stays open; without the refusal the problem runs."""
+    m = _slab(60, which_sparse=variant)
+    P = eng.problem([m], precision=precision)
+    assert eng.set_guess(P, *_zero(m)) == OK
+    g0 = eng.L.fake_graph_launches()
+    eng.L.fake_refuse(1)
+    for _ in range(2):
+        assert eng.run(P) == ERR_CUDA
+        assert eng.L.fake_capturing() == 0
+        assert eng.L.fake_graph_launches() == g0
+    eng.L.fake_refuse(0)
+    assert eng.run(P) in (0, 3, 4)
+    assert eng.set_guess(P, *_zero(m)) == OK
+    eng.free(P)
+
+
+def test_refused_launch_outside_a_capture_ends_the_run(eng):
+    m = _slab(60)
+    P = eng.problem([m])
+    assert eng.set_guess(P, *_zero(m)) == OK
+    eng.L.fake_refuse(2)
+    assert eng.run(P) == ERR_CUDA
+    eng.L.fake_refuse(0)
+    assert eng.run(P) in (0, 3, 4)
+    eng.free(P)
