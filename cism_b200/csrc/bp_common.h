@@ -229,6 +229,19 @@ struct StagedDesc {
   static BP_HD constexpr int bytes(int W) { return nodes_at(W) + 4 * (W + halo_cap(W)); }
 };
 
+// Share of block b of g in a ticket that elects the last block to finish: the
+// shares of a launch add up to 2^32, so a counter of 32 bits is back where it
+// was after every launch, whatever its size and whatever overlapped it, and
+// (from 0) only the last block's sum is 0.
+BP_HD unsigned ticket_share(unsigned b, unsigned g) {
+  unsigned q = 0xffffffffu / g, r = 0xffffffffu % g + 1u;  // 2^32 = q g + r
+  if (r == g) {
+    ++q;
+    r = 0u;
+  }
+  return q + (b < r ? 1u : 0u);
+}
+
 // Node of (col, k) in the blocked level-major layout.
 BP_HD size_t node_of(const DevView& v, int col, int k) {
   return (size_t)v.col_node[col] + ((size_t)k << v.lsh);

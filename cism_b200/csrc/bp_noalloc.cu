@@ -18,11 +18,14 @@
 // larger systems are rejected with BP_ERR_ARGS.  The array is global to the
 // process and to each device, and every call reuses it: two calls whose
 // work overlaps on the GPU (different streams, or different host threads on
-// one device) race on the partial sums and give wrong norms.  Serialise
-// them.  The first call on a device (and the first after the device's
-// context was torn down and made again, e.g. by cudaDeviceReset) looks up
-// the array's device address (cudaGetSymbolAddress); make that call before
-// any stream capture.
+// one device) race on the partial sums and give wrong norms, or leave theirs
+// unwritten.  Serialise them.  Calls after an overlap are right again: the
+// ticket is where it was once all of them are done (ticket_share), in graph
+// replays too and without a launch to reset it; a count of blocks that wraps
+// at each launch's own number does not come back.  The first call on a device
+// (and the first after the device's context was torn down and made again, e.g.
+// by cudaDeviceReset) looks up the array's device address
+// (cudaGetSymbolAddress); make that call before any stream capture.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -30,6 +33,7 @@
 #include <mutex>
 
 #include "bp_b200.h"
+#include "bp_common.h"
 
 namespace {
 
@@ -41,7 +45,7 @@ constexpr int kNaMaxDevices = 64;
 
 struct NaScratch {
   double partial[2 * kNaMaxBlocks];  // per block: sum (Ax-b)^2, sum b^2
-  unsigned ticket;                   // blocks finished; wraps to 0 with the last one
+  unsigned ticket;                   // shares of the blocks that have finished; 0 between launches
   unsigned pad[63];
 };
 
@@ -219,7 +223,8 @@ k_resid_ref_layout(int nx, int ny, int nz, int periodic, const int* __restrict__
   if (tid == 0) {
     __stcg(reinterpret_cast<double2*>(S->partial) + blockIdx.x, make_double2(s_r, s_b));
     __threadfence();
-    last = (atomicInc(&S->ticket, gridDim.x - 1) == gridDim.x - 1) ? 1 : 0;
+    const unsigned share = bp::ticket_share(blockIdx.x, gridDim.x);
+    last = atomicAdd(&S->ticket, share) + share == 0u ? 1 : 0;
   }
   if (!__shfl_sync(0xffffffffu, last, 0)) return;
   // the last block sums every partial, each thread in block order

@@ -258,7 +258,8 @@ int bp_assemble(bp_ctx *ctx, const bp_inputs *in, const double *uvel,
  * Work is enqueued on the stream and not waited for.  The reduction scratch
  * is a fixed file-scope device array shared by all calls: at most
  * nz*(nx-1)*(ny-1) = 16,777,216 rows (larger: BP_ERR_ARGS); calls that
- * overlap on the GPU race on it and must be serialised; the first call on
+ * overlap on the GPU race on it and must be serialised (an overlap spoils the
+ * norms of the calls in it, and of no later one); the first call on
  * a device, and the first after its context was made again (e.g. after
  * cudaDeviceReset), looks up the array's address and should precede any
  * stream capture. */

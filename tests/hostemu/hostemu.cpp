@@ -728,3 +728,8 @@ extern "C" int emu_velocity_roundtrip(const bp_inputs* in, const double* uvel, c
   scatter_velocity(E.p, 0, E.x.data(), uout, vout);
   return 0;
 }
+
+// Shares of a reduction ticket of g blocks.
+extern "C" void emu_ticket_shares(unsigned g, unsigned* share) {
+  for (unsigned b = 0; b < g; ++b) share[b] = ticket_share(b, g);
+}

@@ -310,3 +310,27 @@ def test_ctypes_structs_follow_the_header(cname, pystruct):
     emu.emu_sizeof.restype = C.c_long
     emu.emu_sizeof.argtypes = [C.c_char_p]
     assert emu.emu_sizeof(cname.encode()) == C.sizeof(pystruct)
+
+
+def test_ticket_shares_come_back_to_zero():
+    """The ticket of bp_residual_noalloc: for any grid the blocks' shares add
+    up to 2^32 and no proper part of them does, so the last block alone finds
+    0; blocks of launches of different grids that overlap, in any order, leave
+    the counter at 0 for the launches after them."""
+    emu = C.CDLL(EMU)
+    emu.emu_ticket_shares.argtypes = [C.c_uint, C.POINTER(C.c_uint)]
+
+    def shares(g):
+        a = np.zeros(g, np.uint32)
+        emu.emu_ticket_shares(g, a.ctypes.data_as(C.POINTER(C.c_uint)))
+        return a
+
+    rng = np.random.default_rng(3)
+    for g in [1, 2, 3, 7, 10, 32, 148, 1000, 1183, 1184, 65536]:
+        s = shares(g).astype(np.uint64)
+        assert int(s.sum()) % 2 ** 32 == 0 and (g == 1 or (int(s.sum()) == 2 ** 32 and int(s.min()) > 0))
+        run = np.cumsum(rng.permutation(s)) % 2 ** 32
+        assert run[-1] == 0 and np.count_nonzero(run[:-1] == 0) == 0
+    for _ in range(50):
+        a, b = shares(int(rng.integers(1, 1185))), shares(int(rng.integers(1, 1185)))
+        assert int(rng.permutation(np.concatenate([a, b])).astype(np.uint64).sum()) % 2 ** 32 == 0

@@ -131,3 +131,64 @@ def test_noalloc_residual_chunk_edges(dims, offset):
         nrm = dn.cpu().numpy()
         assert abs(nrm[0] - nr) <= 1e-12 * max(nr, 1.0) and abs(nrm[1] - nb) <= 1e-12 * max(nb, 1.0)
         assert abs(nrm[2] - (nr / nb if nb > 0 else 0.0)) <= 1e-11
+
+
+def test_noalloc_calls_after_an_overlap():
+    """Calls of different sizes that overlap on two streams spoil each other's
+    norms (the header says so); the calls after them, direct ones and replays of
+    a captured one, give what they gave before: bitwise, as the sums' order is
+    fixed."""
+    import torch
+
+    lib = solver.lib()
+    lib.bp_residual_noalloc.argtypes = [C.c_int] * 4 + [_dp] * 13
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(5)
+    sizes = [(9, 7, 3, 1), (160, 161, 11, 0), (33, 20, 10, 1)]
+    calls = []
+    for nx, ny, nz, periodic in sizes:
+        n = nz * (nx - 1) * (ny - 1)
+        A = [torch.rand(n * 27, generator=g, device=dev, dtype=torch.float64) for _ in range(4)]
+        d = [torch.rand(n, generator=g, device=dev, dtype=torch.float64) for _ in range(4)]
+        av = torch.ones((nx - 1) * (ny - 1), device=dev, dtype=torch.int32)
+        out = [torch.empty(n, device=dev, dtype=torch.float64) for _ in range(2)]
+        norms = torch.empty(3, device=dev, dtype=torch.float64)
+        calls.append((nx, ny, nz, periodic, av, A, d, out, norms))
+
+    def call(c, stream):
+        nx, ny, nz, periodic, av, A, d, out, norms = c
+        rc = lib.bp_residual_noalloc(nx, ny, nz, periodic, av.data_ptr(), *[a.data_ptr() for a in A],
+                                     *[a.data_ptr() for a in d], *[a.data_ptr() for a in out], norms.data_ptr(),
+                                     stream.cuda_stream)
+        assert rc == 0
+
+    main = torch.cuda.current_stream(dev)
+    streams = [torch.cuda.Stream(dev) for _ in sizes]
+    graphs = []
+    want = []
+    for c in calls:
+        c[-1].fill_(float("nan"))
+        call(c, main)
+        torch.cuda.synchronize(dev)
+        want.append(c[-1].clone())
+        assert not bool(want[-1].isnan().any())
+    for c in calls:
+        gr = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(gr):
+            call(c, torch.cuda.current_stream(dev))
+        graphs.append(gr)
+    for turn in range(20):
+        for _ in range(5):
+            for c, s in zip(calls, streams):
+                call(c, s)
+        if turn % 2:
+            for gr, s in zip(graphs, streams):
+                with torch.cuda.stream(s):
+                    gr.replay()
+        torch.cuda.synchronize(dev)
+        for replay in (False, True):
+            for c, gr, w in zip(calls, graphs, want):
+                c[-1].fill_(float("nan"))
+                gr.replay() if replay else call(c, main)
+                torch.cuda.synchronize(dev)
+                assert torch.equal(c[-1], w), (turn, replay, c[:3])
