@@ -35,6 +35,7 @@ int bpnet_gemm_tn(const void* A, const void* B, float* C, const float* bias, int
                   int ldb, int ldc, int accum, void* stream);
 int bpnet_gemm_act(const void* A, const void* B, float* Z, const float* bias, void* Y, int M, int N, int K, int lda,
                    int ldb, int act, void* stream);
+int bpnet_act_apart(int M, int N, int K);
 int bpnet_im2col(const void* X, void* col, int B, int H, int W, int C, int Kp, int periodic, void* stream);
 int bpnet_pool(const void* X, void* Y, int B, int H, int W, int C, void* stream);
 int bpnet_up(const void* X, void* Y, int B, int h, int w, int C, int ldy, int c0, void* stream);
@@ -203,7 +204,10 @@ int conv_fwd(GuessNet* N, const GConv& c, const bf16* x, bf16* y, int B, int H, 
     NK(bpnet_im2col(x, cb, B, H, W, c.cin, c.Kp, periodic, s));
     col = cb;
   }
-  if (y) {  // the pre-activation is not kept unless the activation cannot be fused
+  // the pre-activation is kept only where the activation is not fused
+  const bool apart = y && bpnet_act_apart((int)P, c.cout, c.Kp);
+  *nl += apart ? 1 : 0;
+  if (y && !apart) {
     const int rc = bpnet_gemm_act(col, c.wb, nullptr, c.b, y, (int)P, c.cout, c.Kp, c.Kp, c.Kp, c.act, s);
     if (rc != 10) return rc;
   }

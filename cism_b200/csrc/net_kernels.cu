@@ -1434,11 +1434,31 @@ int bpnet_gemm_tn_mode(int mode, const void* A, const void* B, float* C, const f
   return tensor_gemm(0, 0, 0, a16, b16, C, bias, M, N, K, lda, ldb, ldc, accum, nullptr, 0, st);
 }
 
+// Whether the default kernel of a K-major product is the register-staged one: a
+// single K slice has no pipeline to fill, and with tiles for two CTAs an SM or
+// more the copies of the other CTAs cover a CTA's own (131,072 x 32 x 56: 30.1
+// us against 32.3 TMA-fed; 131,072 x 64 x 64 32.4 and 34.4; 65,536 x 64 x 56
+// 24.4 and 26.6).  With fewer tiles the one bulk copy is there sooner (16,384
+// x 32 x 56, 128 tiles: 21.4 and 20.4; 4,096 x 22 x 32 17.8 and 16.3).
+int bpnet_gemm_by_registers(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K > TC_BK) return 0;
+  const GemmCut c = cut_gemm(M, N, K);
+  return (long long)c.gx * c.gy >= 296 ? 1 : 0;
+}
+
 // The product on the default kernel.
 int bpnet_gemm_tn(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int lda,
                   int ldb, int ldc, int accum, void* stream) {
-  return bpnet_gemm_tn_mode(gemm_mode(), A, B, C, bias, M, N, K, lda, ldb, ldc, accum, stream);
+  const int mode = gemm_mode() == 0 && bpnet_gemm_by_registers(M, N, K) ? 1 : gemm_mode();
+  return bpnet_gemm_tn_mode(mode, A, B, C, bias, M, N, K, lda, ldb, ldc, accum, stream);
 }
+
+// Whether bpnet_gemm_act leaves the activation to its own pass where it is
+// given room for Z: with the register-staged kernel, which has no such
+// epilogue, and whole 16-byte groups of channels (131,072 x 32 x 56: 41.1 us
+// in two kernels, 44.2 fused; 262,144 rows 55.8, 64.1, and 59.4 fused without Z;
+// 22 channels, element by element: 45.7 and 40.9).
+int bpnet_act_apart(int M, int N, int K) { return N % 4 == 0 && bpnet_gemm_by_registers(M, N, K); }
 
 // The product with its activation: Z = A B^T + bias (FP32, may be null) and Y
 // = act(Z) in BF16, both with rows of N.
@@ -1446,7 +1466,7 @@ int bpnet_gemm_act(const void* A, const void* B, float* Z, const float* bias, vo
                    int ldb, int act, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || (K % 8) || (lda % 8) || (ldb % 8) || !Y) return 10;
   cudaStream_t st = (cudaStream_t)stream;
-  if (gemm_mode() == 0) {
+  if (gemm_mode() == 0 && !(Z && bpnet_act_apart(M, N, K))) {
     const int rc = tensor_gemm(1, 0, 0, (const bf16*)A, (const bf16*)B, Z, bias, M, N, K, lda, ldb, N, 0, (bf16*)Y,
                                act, st);
     if (rc != 10) return rc;

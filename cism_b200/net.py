@@ -46,6 +46,8 @@ def lib():
             "bpnet_gemm_tn_mode": [i, vp, vp, vp, vp, i, i, i, i, i, i, i, vp],
             "bpnet_gemm_act": [vp, vp, vp, vp, vp, i, i, i, i, i, i, vp],
             "bpnet_gemm_major": [i, i, vp, vp, vp, i, i, i, i, i, i, vp],
+            "bpnet_gemm_by_registers": [i, i, i],
+            "bpnet_act_apart": [i, i, i],
             "bpnet_gemm_status": [vp],
             "bpnet_im2col": [vp, vp, i, i, i, i, i, i, vp],
             "bpnet_col2im": [vp, vp, i, i, i, i, i, i, vp],
@@ -109,7 +111,8 @@ GEMM_KERNELS = {"tma": 0, "tc": 1, "mma": 2}
 
 def gemm_tn(A, B, out, bias, M, N, K, lda, ldb, ldc, accum=False, kernel=None):
     """out[M][N] (FP32) = A[M][K] . B[N][K]^T (+ bias) (+ out); BF16 operands.
-    kernel None: the library's default (tcgen05, TMA-fed); "tma", "tc" (tcgen05
+    kernel None: the library's default (tcgen05, TMA-fed, or for large products of
+    one K slice register-staged: bpnet_gemm_by_registers); "tma", "tc" (tcgen05
     with register-staged operands) or "mma" (mma.sync) to choose."""
     if kernel is None:
         rc = lib().bpnet_gemm_tn(_p(A), _p(B), _p(out), _p(bias), M, N, K, lda, ldb, ldc, int(accum), _s())

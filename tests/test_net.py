@@ -392,3 +392,45 @@ def test_direct_input_gradient(shape, periodic):
     assert L.bpnet_col2im(p(dcol), p(ref), B, H, W, cin, Kp, periodic, s) == 0
     assert torch.equal(dx, ref)
     assert netmod.gemm_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,registers", [(296 * 128, 32, 64, 1), (295 * 128, 32, 64, 0), (295 * 128 + 1, 32, 8, 1),
+                                             (296 * 128, 32, 72, 0), (148 * 128, 128, 56, 1), (147 * 128, 128, 56, 0),
+                                             (296 * 128, 96, 56, 1), (961, 32, 56, 0), (2 ** 20, 1152, 64, 1)])
+def test_route_of_products_of_one_slice(M, N, K, registers):
+    """Products of one K slice (64) with 296 tiles or more are the
+    register-staged kernel's, and their activation, for whole groups of four
+    channels, a pass of its own."""
+    pytest.importorskip("torch")
+    from cism_b200 import net as netmod
+
+    L = netmod.lib()
+    assert L.bpnet_gemm_by_registers(M, N, K) == registers
+    assert L.bpnet_act_apart(M, N, K) == registers
+    assert L.bpnet_act_apart(M, N + 2, K) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(296 * 128, 32, 56), (296 * 128 - 127, 32, 8), (295 * 128, 32, 56),
+                                   (148 * 128, 128, 64), (300 * 128, 22, 32), (300 * 128, 24, 72)])
+def test_products_of_one_slice_are_the_same_on_every_route(shape):
+    """Either kernel, the fused activation and the separate one: the same sums
+    in the same order, so bitwise."""
+    torch = pytest.importorskip("torch")
+    from cism_b200 import net as netmod
+
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    bias = torch.randn(N, generator=g, device="cuda")
+    z = [torch.empty(M, N, device="cuda") for _ in range(4)]
+    y = [torch.empty(M, N, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+    L, p, s = netmod.lib(), netmod._p, netmod._s()
+    for out, kernel in zip(z, ("tma", "tc", None)):
+        netmod.gemm_tn(a, b, out, bias, M, N, K, K, K, N, kernel=kernel)
+    assert L.bpnet_gemm_act(p(a), p(b), p(z[3]), p(bias), p(y[0]), M, N, K, K, K, 1, s) == 0
+    assert L.bpnet_gemm_act(p(a), p(b), None, p(bias), p(y[1]), M, N, K, K, K, 1, s) == 0
+    assert L.bpnet_act(p(z[0]), p(y[2]), M, N, N, 0, 1, s) == 0
+    assert all(torch.equal(z[0], other) for other in z[1:])
+    assert all(torch.equal(y[2], other) for other in y[:2])
