@@ -967,6 +967,11 @@ void problem_free(bp_problem* P) {
   delete P;
 }
 
+// Device scratch between runs for velocities in column order (2 nnodes
+// doubles): the Dirichlet moves, which every assembly writes before it reads
+// them.  Not a node vector, whose holes stay zero.
+double* column_scratch(const bp_problem* P) { return P->v.badj; }
+
 void problem_set_guess(bp_problem* P, double* const* uvel, double* const* vvel) {
   const HostPlan& p = P->plan;
   cudaStream_t s = P->c->stream;
@@ -982,7 +987,7 @@ void problem_set_guess(bp_problem* P, double* const* uvel, double* const* vvel) 
   } else if ((int)learned.size() < p.ninst) {  // columns through the staging buffer, nodes on the device
     const size_t n = (size_t)p.nnodes;
     double* host = P->c->staging.get<double>(s, 2 * n);
-    double* dev = reinterpret_cast<double*>(P->v.q);  // scratch between runs
+    double* dev = column_scratch(P);
     for (int b = 0; b < p.ninst; ++b) {
       if (p.guess_mode[b] == BP_GUESS_LEARNED) continue;
       gather_columns(p, b, uvel[b], vvel[b], host, host + n);
@@ -1056,7 +1061,7 @@ void problem_get(bp_problem* P, double* const* uvel, double* const* vvel, double
   double* ef = host + 2 * nx;
   double2* x = reinterpret_cast<double2*>(host);
   if (columns) {
-    double* dev = reinterpret_cast<double*>(P->v.q);  // scratch after a run
+    double* dev = column_scratch(P);
     launch_pack(P->v, P->v.x, dev, dev + nx, P->c->stream);
     CK(cudaGetLastError());
     if (nx > 0) CK(cudaMemcpyAsync(host, dev, sizeof(double) * 2 * nx, cudaMemcpyDeviceToHost, P->c->stream));
@@ -1248,7 +1253,7 @@ int bp_problem_get_guess(bp_problem* P, double* const* uvel, double* const* vvel
   }
   const size_t n = (size_t)p.nnodes;
   double* host = P->c->staging.get<double>(s, 2 * n);
-  double* dev = reinterpret_cast<double*>(P->v.q);  // scratch between runs
+  double* dev = column_scratch(P);
   launch_pack(P->v, P->x0, dev, dev + n, s);
   CK(cudaGetLastError());
   if (n > 0) CK(cudaMemcpyAsync(host, dev, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost, s));

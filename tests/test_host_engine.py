@@ -95,3 +95,24 @@ def test_refused_launch_outside_a_capture_ends_the_run(eng):
     eng.L.fake_refuse(0)
     assert eng.run(P) in (0, 3, 4)
     eng.free(P)
+
+
+def test_velocity_transfers_leave_the_node_vectors_holes_at_zero(eng):
+    """The columns' scratch on the way in and out is no node vector: the slots
+    of the vectors that belong to no column stay zero (make_view)."""
+    ms = [_slab(13), _slab(10)]
+    P = eng.problem(ms)
+    rng = np.random.default_rng(4)
+    us, vs = ([rng.standard_normal(m.vshape3) for m in ms] for _ in range(2))
+    assert eng.set_guess(P, us, vs) == OK
+    assert eng.L.fake_nonzero_holes() == 0
+    out = [[np.zeros(m.vshape3) for m in ms] for _ in range(2)]
+    assert eng.L.bp_problem_get_guess(P, eng.ptrs(out[0]), eng.ptrs(out[1])) == OK
+    assert eng.L.fake_nonzero_holes() == 0
+    for a, b, m in zip(us + vs, out[0] + out[1], ms + ms):
+        js, is_ = m.owned_vertex_slices()
+        assert np.array_equal(a[js, is_], b[js, is_])  # a periodic slab: every owned vertex is active
+    assert eng.run(P, 2) in (0, 3, 4)
+    assert eng.L.bp_problem_get(P, eng.ptrs(out[0]), eng.ptrs(out[1]), None) == OK
+    assert eng.L.fake_nonzero_holes() == 0
+    eng.free(P)
