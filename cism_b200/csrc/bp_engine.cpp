@@ -152,6 +152,7 @@ struct bp_problem {
   double2* x3_0 = nullptr;
   double* eq3_0 = nullptr;
   double2* bt0 = nullptr;
+  std::vector<int> halo_tables;  // as uploaded (use_resident_pcg)
   cudaGraphExec_t chunk_graph = nullptr;
   cudaGraphExec_t inner_graph = nullptr;
   // the device-resident Picard loop (one graph with nested WHILE nodes) and
@@ -184,8 +185,36 @@ void upload(cudaStream_t s, T* dst, const std::vector<T>& src) {
   }
 }
 
-// Allocate and upload the device arrays of a plan.
-DevView make_view(Arena& a, cudaStream_t s, const HostPlan& p, bool with_cells, bool mixed) {
+// 16-byte words of the resident PCG's block (resident_head without the halo
+// tables, of at most one column per neighbour) and of the staged matvec's.  Both
+// lie behind the matrix in its allocation: a cudaMalloc of a megabyte or more
+// takes 0.35 ms, and a problem has one of the two.
+size_t resident_head(const HostPlan& p) {
+  return 2 * (size_t)kXchSumCopies * p.ntiles * 4 + 2 * 2 * (size_t)p.npad + ((size_t)p.ninst + 1) / 2;
+}
+size_t resident_words(const HostPlan& p) {
+  return resident_head(p) + ((size_t)p.ntiles + 1 + 17 * (size_t)p.ncols + 3) / 4;
+}
+size_t staged_words(const HostPlan& p) {
+  return (size_t)p.ntiles * (StagedDesc::bytes(p.W) + 8 * 3 * sizeof(double)) / 16;
+}
+size_t matrix_words(const DevView& v) { return (v.sym ? 2 * 14 : 2 * 27) * (size_t)v.npad; }
+
+// Whether the resident PCG holds all tiles of the problem, by the least shared
+// memory a tile can take (no halo).
+bool may_be_resident(const bp_ctx* c, const DevView& v, const HostPlan& p) {
+  return p.ntiles > 0 && !p.inst.empty() && p.ntiles <= resident_ctas(v, p.inst[0].variant, c->num_sms);
+}
+
+// What lies behind the matrix of a problem that may take either.
+size_t words_behind_matrix(const bp_ctx* c, const DevView& v, const HostPlan& p) {
+  const size_t staged = staged_per_sm(v) > 0 ? staged_words(p) : 0;
+  return may_be_resident(c, v, p) ? std::max(staged, resident_words(p)) : staged;
+}
+
+// Allocate and upload the device arrays of a plan; c_fast: the context of a
+// problem that solves (null: matrix-level calls, without the fast kernels' block).
+DevView make_view(Arena& a, cudaStream_t s, const HostPlan& p, bool with_cells, bool mixed, const bp_ctx* c_fast) {
   DevView v;
   std::memset(&v, 0, sizeof(v));
   v.nz = p.nz; v.ncols = p.ncols; v.nnodes = p.nnodes; v.npad = p.npad;
@@ -277,7 +306,6 @@ DevView make_view(Arena& a, cudaStream_t s, const HostPlan& p, bool with_cells, 
   UP(int, "tile_ncols", p.tile_ncols, tile_ncols);
   UP(int, "tile_col0", p.tile_col0, tile_col0);
 #undef UP
-  v.A = a.get<double2>(s, "A", (v.sym ? 2 * 14 : 2 * 27) * np);
   v.x = a.get<double2>(s, "x", np);
   v.b = a.get<double2>(s, "b", np);
   v.r = a.get<double2>(s, "r", np);
@@ -298,6 +326,7 @@ DevView make_view(Arena& a, cudaStream_t s, const HostPlan& p, bool with_cells, 
     v.A32 = blk;
     v.A32d = reinterpret_cast<double2*>(blk + 14 * np);
   }
+  v.A = a.get<double2>(s, "A", matrix_words(v) + (c_fast ? words_behind_matrix(c_fast, v, p) : 0));
   v.partials = a.get<double>(s, "partials", 3 * (size_t)std::max(p.ntiles, 1) + 1);  // read in pairs
   v.tile_counter = a.get<unsigned>(s, "tile_counter", p.ninst);
   CK(cudaMemsetAsync(v.tile_counter, 0, sizeof(unsigned) * p.ninst, s));
@@ -305,26 +334,24 @@ DevView make_view(Arena& a, cudaStream_t s, const HostPlan& p, bool with_cells, 
 }
 
 // The resident PCG (launch_pcg_resident) where every tile of the problem
-// fits on the GPU at once.
-void use_resident_pcg(bp_ctx* c, Arena& a, DevView* v, const HostPlan& p) {
-  if (p.ntiles == 0 || p.ntiles > kResidentMaxTiles) return;
+// fits on the GPU at once; tables: the problem's, alive until its next wait.
+void use_resident_pcg(bp_ctx* c, DevView* v, const HostPlan& p, std::vector<int>* tables) {
+  if (!may_be_resident(c, *v, p)) return;
   const HaloPlan h = build_halo(p);
   v->halo_max = h.max_cols;
   if (p.ntiles > resident_ctas(*v, p.inst[0].variant, c->num_sms)) return;
   cudaStream_t s = c->stream;
   // one block: the slots, the epochs, then the halo tables
   const size_t sums = 2 * (size_t)kXchSumCopies * p.ntiles * 4, nodes = 2 * 2 * (size_t)p.npad;
-  const size_t epochs = ((size_t)p.ninst + 1) / 2;
-  std::vector<int> tables(h.begin);
-  tables.insert(tables.end(), h.node.begin(), h.node.end());
-  tables.insert(tables.end(), h.col_loc.begin(), h.col_loc.end());
-  const size_t head = sums + nodes + epochs;
-  ulonglong2* block = a.get<ulonglong2>(s, "resident", head + (tables.size() + 3) / 4);
+  const size_t head = resident_head(p);
+  *tables = h.begin;
+  tables->insert(tables->end(), h.node.begin(), h.node.end());
+  tables->insert(tables->end(), h.col_loc.begin(), h.col_loc.end());
+  ulonglong2* block = reinterpret_cast<ulonglong2*>(v->A + matrix_words(*v));
   // epochs count from 1: no slot may hold one from an earlier problem
   CK(cudaMemsetAsync(block, 0, sizeof(ulonglong2) * head, s));
   int* t = reinterpret_cast<int*>(block + head);
-  upload(s, t, tables);
-  CK(cudaStreamSynchronize(s));  // tables is a host temporary
+  upload(s, t, *tables);
   v->xch = block;
   v->xch_node = block + sums;
   v->xch_epoch = reinterpret_cast<unsigned long long*>(block + sums + nodes);
@@ -335,11 +362,11 @@ void use_resident_pcg(bp_ctx* c, Arena& a, DevView* v, const HostPlan& p) {
 
 // The staged Krylov matvec's descriptors, where the problem has its shape
 // and no resident PCG; the autotuner chooses between it and the per-node one.
-void use_staged_mv(bp_ctx* c, Arena& a, DevView* v, const HostPlan& p) {
+void use_staged_mv(bp_ctx* c, DevView* v, const HostPlan& p) {
   if (p.ntiles == 0 || v->xch || staged_per_sm(*v) == 0) return;
   cudaStream_t s = c->stream;
-  unsigned char* d = a.get<unsigned char>(s, "staged_desc", (size_t)p.ntiles * StagedDesc::bytes(p.W));
-  v->wsum = a.get<double>(s, "staged_sums", (size_t)p.ntiles * 8 * 3);
+  unsigned char* d = reinterpret_cast<unsigned char*>(v->A + matrix_words(*v));
+  v->wsum = reinterpret_cast<double*>(d + (size_t)p.ntiles * StagedDesc::bytes(p.W));
   launch_staged_desc(*v, d, s);
   CK(cudaGetLastError());
   v->desc = d;
@@ -940,10 +967,10 @@ bp_problem* problem_new(bp_ctx* c, Arena* arena, int n, const bp_inputs* in, std
   P->mixed = P->plan.inst[0].precision == BP_MIXED;
   CK(cudaEventRecord(c->t0, c->stream));
   g_h2d = 0.0;
-  P->v = make_view(*P->arena, c->stream, P->plan, true, P->mixed);
+  P->v = make_view(*P->arena, c->stream, P->plan, true, P->mixed, c);
   P->h2d_bytes = g_h2d;
-  use_resident_pcg(c, *P->arena, &P->v, P->plan);
-  use_staged_mv(c, *P->arena, &P->v, P->plan);
+  use_resident_pcg(c, &P->v, P->plan, &P->halo_tables);
+  use_staged_mv(c, &P->v, P->plan);
   P->x0 = P->arena->get<double2>(c->stream, "x0", P->plan.npad);
   CK(cudaMemsetAsync(P->x0, 0, sizeof(double2) * P->plan.npad, c->stream));
   if (P->plan.diva) {
@@ -1534,8 +1561,8 @@ int bp_pcg(bp_ctx* c, int nx, int ny, int nz, int periodic,
   ip.inner_tol = 1.0e-4;
   P.mixed = false;
   P.use_graphs = false;
-  P.v = make_view(*P.arena, c->stream, P.plan, false, P.mixed);
-  use_resident_pcg(c, *P.arena, &P.v, P.plan);
+  P.v = make_view(*P.arena, c->stream, P.plan, false, P.mixed, c);
+  use_resident_pcg(c, &P.v, P.plan, &P.halo_tables);
   const DevView& v = P.v;
   const double* blocks[4] = {Auu, Auv, Avu, Avv};
   upload_matrix(c, *P.arena, v, P.plan, blocks);
@@ -1575,7 +1602,7 @@ int bp_matvec(bp_ctx* c, int nx, int ny, int nz, int periodic,
     c->err = e;
     return BP_ERR_ARGS;
   }
-  DevView v = make_view(c->arena, c->stream, p, false, false);
+  DevView v = make_view(c->arena, c->stream, p, false, false, nullptr);
   const double* blocks[4] = {Auu, Auv, Avu, Avv};
   upload_matrix(c, c->arena, v, p, blocks);
   std::vector<double2> x(p.npad, double2{0, 0});
@@ -1608,7 +1635,7 @@ int bp_assemble(bp_ctx* c, const bp_inputs* in, const double* uvel,
     c->err = "bp_assemble: 3-D Blatter-Pattyn systems only";
     return BP_ERR_ARGS;
   }
-  DevView v = make_view(c->arena, c->stream, p, true, false);
+  DevView v = make_view(c->arena, c->stream, p, true, false, nullptr);
   std::vector<double2> x(p.npad, double2{0, 0});
   gather_velocity(p, 0, uvel, vvel, x.data());
   CK(cudaMemcpyAsync(v.x, x.data(), sizeof(double2) * p.npad, cudaMemcpyHostToDevice, c->stream));

@@ -41,7 +41,6 @@ void launch_cg_update(bool check, const DevView& v, cudaStream_t s);
 // to convergence, in one cooperative launch of one CTA per tile.
 // resident_ctas: CTAs of that kernel the GPU holds at once (0 where its
 // shared memory does not fit or on an error); the launch needs v.ntiles of them.
-constexpr int kResidentMaxTiles = 1184;
 int resident_ctas(const DevView& v, int variant, int num_sms);
 cudaError_t launch_pcg_resident(const DevView& v, int variant, cudaStream_t s);
 // The staged Krylov matvec: shared memory of a CTA, the most CTAs an SM

@@ -18,7 +18,7 @@ struct Fake {
   cudaError_t last = cudaSuccess;
   int capturing = 0;       // a capture is open on the stream
   int refuse = 0;          // 1: Krylov matvecs inside a capture, 2: all Krylov matvecs
-  int graph_launches = 0, resident_queries = 0;
+  int graph_launches = 0, resident_halo = 0;
   bool copies_open = false;  // host-to-device copies since the last synchronisation
   DevView v;               // of the last launch
 } F;
@@ -47,7 +47,8 @@ extern "C" {
 void fake_refuse(int what) { F.refuse = what; }
 int fake_capturing() { return F.capturing; }
 int fake_graph_launches() { return F.graph_launches; }
-int fake_resident_queries() { return F.resident_queries; }
+// most halo columns of a tile in the last question for resident CTAs
+int fake_resident_halo() { return F.resident_halo; }
 int fake_copies_open() { return F.copies_open ? 1 : 0; }
 // Slots of the zeroed node vectors that belong to no column (the end of each
 // instance's last tile) and do not hold zero; -1 where there are none.
@@ -168,7 +169,7 @@ namespace bp {
 cudaError_t upload_ref_tables() { return cudaSuccess; }
 void set_pdl(bool) {}
 int resident_ctas(const DevView& v, int, int num_sms) {
-  ++F.resident_queries;
+  F.resident_halo = v.halo_max;
   return v.W * v.nz <= 256 ? num_sms : 0;
 }
 int staged_per_sm(const DevView&) { return 1; }

@@ -116,3 +116,12 @@ def test_velocity_transfers_leave_the_node_vectors_holes_at_zero(eng):
     assert eng.L.bp_problem_get(P, eng.ptrs(out[0]), eng.ptrs(out[1]), None) == OK
     assert eng.L.fake_nonzero_holes() == 0
     eng.free(P)
+
+
+@pytest.mark.parametrize("n,halo", [(48, True), (49, False)])
+def test_halo_tables_are_built_only_where_tiles_may_fit(eng, n, halo):
+    """144 tiles fit the fake's 148 CTAs, 151 do not: the halo's tables (0.3 ms
+    of host time at 600 tiles) are not built to be thrown away."""
+    P = eng.problem([_slab(n)])
+    assert (eng.L.fake_resident_halo() > 0) == halo
+    eng.free(P)
