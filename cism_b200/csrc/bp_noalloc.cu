@@ -5,7 +5,7 @@
 // own layout (matrix blocks (27,nz,nx-1,ny-1), vectors (nz,nx-1,ny-1), halo
 // included and already halo-consistent), plus |A x - b|, |b| and their
 // ratio.  It is the allocation-free variant of the residual kernel of the
-// solver (k_mv<MV_INIT>): its only scratch -- one partial sum pair per
+// solver (k_resid<MV_INIT>): its only scratch -- one partial sum pair per
 // block and the ticket that elects the block doing the final sum -- lives in
 // the file-scope array below instead of in memory from cudaMalloc.
 //
@@ -15,7 +15,8 @@
 // time step can call this with its own buffers and nothing else.
 //
 // Limits and sharing: at most kNaMaxRows = 16,777,216 rows (nz*(nx-1)*(ny-1));
-// larger systems are rejected with BP_ERR_ARGS.  The array is global to the
+// larger systems are rejected with BP_ERR_ARGS (a limit of the call that its
+// users know, not of the scratch: the blocks loop over the rows).  The array is global to the
 // process and to each device, and every call reuses it: two calls whose
 // work overlaps on the GPU (different streams, or different host threads on
 // one device) race on the partial sums and give wrong norms, or leave theirs
@@ -39,17 +40,16 @@ namespace {
 
 constexpr int kNaRows = 32;           // rows of a chunk; a block is one warp
 constexpr int kNaBlocks = 8 * 148;    // resident blocks of the GPU (27 KB of shared memory each)
-constexpr int kNaMaxBlocks = 65536;   // pairs the scratch holds
-constexpr long kNaMaxRows = 256L * kNaMaxBlocks;
+constexpr long kNaMaxRows = 1L << 24;
 constexpr int kNaMaxDevices = 64;
 
 struct NaScratch {
-  double partial[2 * kNaMaxBlocks];  // per block: sum (Ax-b)^2, sum b^2
+  double partial[2 * kNaBlocks];     // per block: sum (Ax-b)^2, sum b^2
   unsigned ticket;                   // shares of the blocks that have finished; 0 between launches
   unsigned pad[63];
 };
 
-// 1 MiB + 256 B on every device that loads the library, held until exit.
+// 19 KB on every device that loads the library, held until exit.
 static __device__ __align__(256) NaScratch g_na_scratch;
 
 std::mutex g_na_mutex;
@@ -84,8 +84,9 @@ __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
 // shared memory (27 doubles apart: no bank conflict).  BULK = false copies
 // with plain loads, for matrix pointers that are not 16-byte aligned (a
 // bulk copy must start on 16 bytes).  A pair of rows is 27 x 16 B, so
-// copies start on even rows; an odd last row of the arrays is loaded
-// plainly.  Bound: DRAM.  A round ice sheet on 160 x 160 x 11 (16 thousand
+// copies start and end on even rows; the pair of the last active row never
+// passes the end of the arrays, whose last column is no owned one (i <= nx - 2
+// and j <= ny - 2, while the arrays end with column (nx - 1, ny - 1)).  Bound: DRAM.  A round ice sheet on 160 x 160 x 11 (16 thousand
 // active columns, 165 MB): 35 us, 4.7 TB/s, against 82 us for the thread-per-
 // row loads with the ticket's memset before each launch; 31 x 31 x 10: the
 // call is bound by the host's one launch (10.2 us a call against 13.0).
@@ -126,26 +127,22 @@ k_resid_ref_layout(int nx, int ny, int nz, int periodic, const int* __restrict__
     const unsigned act = __ballot_sync(0xffffffffu, mine);
     if (act) {
       const int r0 = (__ffs((int)act) - 1) & ~1;
-      int r1 = (33 - __clz((int)act)) & ~1;  // [r0, r1) holds the active rows, both even
-      const bool odd_end = t0 + r1 > rows;  // the pair would pass the end of the arrays
-      if (odd_end) r1 -= 2;
+      const int r1 = (33 - __clz((int)act)) & ~1;  // [r0, r1) holds the active rows, both even
       if (BULK) {
         if (tid == 0) {
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          const unsigned bytes = r1 > r0 ? (unsigned)(r1 - r0) * 216u : 0u;
+          const unsigned bytes = (unsigned)(r1 - r0) * 216u;
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"(4u * bytes),
                        "r"(smem_addr(&bar))
                        : "memory");
-          if (bytes) {
-            const double* src[4] = {Auu, Auv, Avu, Avv};
+          const double* src[4] = {Auu, Auv, Avu, Avv};
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-              asm volatile(
-                  "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                      smem_addr(na_sm + (q * kNaRows + r0) * 27)),
-                  "l"(src[q] + (t0 + r0) * 27), "r"(bytes), "r"(smem_addr(&bar))
-                  : "memory");
-          }
+          for (int q = 0; q < 4; ++q)
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                    smem_addr(na_sm + (q * kNaRows + r0) * 27)),
+                "l"(src[q] + (t0 + r0) * 27), "r"(bytes), "r"(smem_addr(&bar))
+                : "memory");
         }
       } else {
         for (int e = r0 * 27 + tid; e < r1 * 27; e += kNaRows) {
@@ -154,12 +151,6 @@ k_resid_ref_layout(int nx, int ny, int nz, int periodic, const int* __restrict__
           na_sm[2 * kNaRows * 27 + e] = Avu[t0 * 27 + e];
           na_sm[3 * kNaRows * 27 + e] = Avv[t0 * 27 + e];
         }
-      }
-      if (odd_end && tid < 27) {  // row r1, the arrays' last
-        na_sm[r1 * 27 + tid] = Auu[(t0 + r1) * 27 + tid];
-        na_sm[(kNaRows + r1) * 27 + tid] = Auv[(t0 + r1) * 27 + tid];
-        na_sm[(2 * kNaRows + r1) * 27 + tid] = Avu[(t0 + r1) * 27 + tid];
-        na_sm[(3 * kNaRows + r1) * 27 + tid] = Avv[(t0 + r1) * 27 + tid];
       }
       // the source values while the copies are in flight: neighbours are
       // read directly at (halo) indices, as the reference does, at one
