@@ -104,6 +104,7 @@ struct Staging {
 // Event pairs around kernel launches, by category.
 struct Timing {
   bool on = false;
+  bool as_run = false;  // the kernels of an untimed run (the resident PCG where it is used)
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> pool;
   std::vector<int> cat;
   double ms[BP_NUM_KERNEL_CATEGORIES] = {0};
@@ -527,8 +528,9 @@ int pcg_head(bp_problem* P) {
   return n;
 }
 
-// Timing runs (events around every launch) keep the launched PCG.
-bool resident_pcg(const bp_problem* P) { return P->v.xch && !P->timing.on; }
+// Timing runs (events around every launch) keep the launched PCG, unless they
+// are to time what an untimed run launches.
+bool resident_pcg(const bp_problem* P) { return P->v.xch && (!P->timing.on || P->timing.as_run); }
 
 // FP64 PCG for all instances with pcg_active, after MV_INIT: one launch of
 // the resident kernel, or the head, then check chunks until the device counter shows no active instance (the
@@ -540,7 +542,7 @@ void run_pcg_fp64(bp_problem* P) {
   bp_ctx* c = P->c;
   const int variant = p.inst[0].variant;
   if (resident_pcg(P)) {
-    CK(launch_pcg_resident(v, variant, c->stream));
+    L(P, C_MV, [&] { CK(launch_pcg_resident(v, variant, c->stream)); });
     return;
   }
   const int ncheck = std::max(1, p.inst[0].ncheck);
@@ -1418,9 +1420,12 @@ int bp_timer_stop(bp_ctx* c, float* ms) {
 int bp_problem_timing(bp_problem* P, int enable) {
   if (!P) return BP_ERR_ARGS;
   P->timing.on = enable != 0;
+  P->timing.as_run = enable == 2;
   P->timing.reset();
   return BP_OK;
 }
+
+int bp_problem_resident(bp_problem* P) { return P && P->v.xch ? 1 : 0; }
 
 int bp_problem_kernel_times(bp_problem* P, double* ms, int* launches) {
   if (!P) return BP_ERR_ARGS;

@@ -164,6 +164,7 @@ def lib():
         L.bp_problem_get.argtypes = [C.c_void_p, C.POINTER(_dp), C.POINTER(_dp), C.POINTER(_dp)]
         L.bp_problem_destroy.argtypes = [C.c_void_p]
         L.bp_problem_timing.argtypes = [C.c_void_p, C.c_int]
+        L.bp_problem_resident.argtypes = [C.c_void_p]
         L.bp_problem_kernel_times.argtypes = [C.c_void_p, _dp, _ip]
         L.bp_problem_info.argtypes = [C.c_void_p] + [C.POINTER(C.c_long)] * 3 + [_dp, _dp]
         L.bp_problem_tune_mv.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
@@ -506,8 +507,14 @@ class Problem:
         rc = lib().bp_problem_tune_mv(self.h, store, minb, grid, reps, C.byref(ms))
         return ms.value if rc == 0 else None
 
-    def timing(self, enable: bool):
-        lib().bp_problem_timing(self.h, 1 if enable else 0)
+    def timing(self, enable: bool, as_run: bool = False):
+        """Events around every launch of the runs that follow.  as_run: of what
+        an untimed run launches; else a PCG step is always its own launches."""
+        lib().bp_problem_timing(self.h, (2 if as_run else 1) if enable else 0)
+
+    def resident(self) -> bool:
+        """Whether the (untimed) runs take the resident PCG."""
+        return bool(lib().bp_problem_resident(self.h))
 
     def kernel_times(self):
         ms = (C.c_double * len(KERNEL_CATEGORIES))()

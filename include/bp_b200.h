@@ -334,9 +334,14 @@ int bp_problem_diagnostics(bp_problem *p, int which_bfric, double *const *tau_xz
  * the runs made while enabled (CUDA graphs are bypassed while enabled).
  * Categories: 0 FP64 PCG matvec, 1 FP64 PCG vector update, 2 FP64
  * residual check, 3 FP32 inner matvec, 4 FP32 inner update, 5 assembly
- * pass 1, 6 assembly pass 2, 7 right-hand side, 8 other. */
+ * pass 1, 6 assembly pass 2, 7 right-hand side, 8 other.
+ * enable 1: every step of the PCG is a launch of its own, also in a problem
+ * whose untimed runs take the resident PCG (one launch per linear solve);
+ * 2: what an untimed run launches, the resident PCG in category 0. */
 #define BP_NUM_KERNEL_CATEGORIES 9
 int bp_problem_timing(bp_problem *p, int enable);
+/* 1 if the problem's (untimed) runs take the resident PCG. */
+int bp_problem_resident(bp_problem *p);
 /* Device-side wall clock of a region of work on the context's stream:
  * CUDA events recorded at start and stop (ms). */
 int bp_timer_start(bp_ctx *ctx);

@@ -125,3 +125,25 @@ def test_halo_tables_are_built_only_where_tiles_may_fit(eng, n, halo):
     P = eng.problem([_slab(n)])
     assert (eng.L.fake_resident_halo() > 0) == halo
     eng.free(P)
+
+
+def test_timing_runs_of_a_resident_problem(eng):
+    """A timing run launches the PCG's steps one by one; one of the kernels
+    that run untimed (2) has one PCG launch per Picard iteration.  A problem
+    that is not resident is timed the same way in both."""
+    for n, resident in ((20, 1), (60, 0)):
+        m = _slab(n)
+        P = eng.problem([m])
+        assert eng.L.bp_problem_resident(P) == resident
+        count = {}
+        for mode in (1, 2):
+            assert eng.set_guess(P, *_zero(m)) == OK
+            assert eng.L.bp_problem_timing(P, mode) == OK
+            assert eng.run(P) in (0, 3, 4)
+            ms, k = (C.c_double * 9)(), (C.c_int * 9)()
+            assert eng.L.bp_problem_kernel_times(P, ms, k) == OK
+            count[mode] = list(k)
+        assert count[1][0] > 1 and count[1][1] > 1  # matvecs, updates
+        assert count[2][:2] == ([1, 0] if resident else count[1][:2])
+        assert count[2][2:] == count[1][2:] or resident
+        eng.free(P)
