@@ -1229,10 +1229,12 @@ const char* bp_last_error(const bp_ctx* c) { return c ? c->err.c_str() : "no con
 #define GUARD_END                                                      \
   }                                                                    \
   catch (const CudaError& e) {                                         \
+    cudaStreamSynchronize(c_->stream); /* as a call that succeeds */   \
     c_->err = std::string(e.what) + ": " + cudaGetErrorString(e.e);    \
     return BP_ERR_CUDA;                                                \
   }                                                                    \
   catch (const GuessError& e) {                                        \
+    cudaStreamSynchronize(c_->stream);                                 \
     c_->err = e.what;                                                  \
     return BP_ERR_ARGS;                                                \
   }                                                                    \

@@ -147,3 +147,19 @@ def test_timing_runs_of_a_resident_problem(eng):
         assert count[2][:2] == ([1, 0] if resident else count[1][:2])
         assert count[2][2:] == count[1][2:] or resident
         eng.free(P)
+
+
+def test_a_call_that_fails_ends_synchronised(eng):
+    """A batch of a given and a learned guess without a network: the call is
+    refused with no copy from the context's staging buffer still on its way
+    (the next call writes there)."""
+    ms = [_slab(12), _slab(13)]
+    preps = [solver.prepare(m, guess_mode=g)[0] for m, g in zip(ms, (solver.GUESS_GIVEN, solver.GUESS_LEARNED))]
+    arr = (solver.Inputs * 2)(*[p.inputs for p in preps])
+    P = C.c_void_p()
+    assert eng.L.bp_problem_create(eng.h, 2, arr, C.byref(P)) == OK
+    z = np.zeros(ms[0].vshape3)
+    assert eng.set_guess(P, [z, None], [z, None]) == ERR_ARGS
+    assert b"bp_guess_load" in eng.L.bp_last_error(eng.h)
+    assert eng.L.fake_copies_open() == 0
+    eng.free(P)
