@@ -3,7 +3,10 @@
 // plan, so the compaction, periodic images and assembly indexing can be
 // checked against the oracle without a GPU.  Not part of the product
 // library and never loaded by it.
+#include <atomic>
 #include <cstring>
+#include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -732,4 +735,80 @@ extern "C" int emu_velocity_roundtrip(const bp_inputs* in, const double* uvel, c
 // Shares of a reduction ticket of g blocks.
 extern "C" void emu_ticket_shares(unsigned g, unsigned* share) {
   for (unsigned b = 0; b < g; ++b) share[b] = ticket_share(b, g);
+}
+
+// parallel_for over n items of at least `grain`: hits[i] counts the calls that
+// covered item i; returns the number of ranges.
+extern "C" int emu_parallel_for(long n, long grain, int* hits) {
+  std::atomic<int> ranges{0};
+  parallel_for((size_t)n, (size_t)grain, [&](size_t a, size_t b) {
+    ++ranges;
+    for (size_t i = a; i < b; ++i) ++hits[i];
+  });
+  return ranges;
+}
+
+// The 3-D solve's velocities by columns (gather_columns, scatter_columns and
+// the node layout of launch_unpack / launch_pack) against node by node
+// (gather_velocity, scatter_velocity), for n instances: 0 where both node
+// vectors and all output arrays are the same bytes.
+extern "C" int emu_columns(int n, const bp_inputs* in, const double* const* u, const double* const* v) {
+  HostPlan p;
+  std::string err;
+  if (!build_plan(in, n, &p, &err)) return -1;
+  std::vector<double> cu((size_t)p.nnodes, -1.0), cv(cu);
+  std::vector<double2> x0(p.npad, double2{0, 0}), x1(x0);
+  for (int b = 0; b < n; ++b) {
+    gather_velocity(p, b, u[b], v[b], x0.data());
+    gather_columns(p, b, u[b], v[b], cu.data(), cv.data());
+  }
+  for (int g = 0; g < p.ncols; ++g)
+    for (int k = 0; k < p.nz; ++k)
+      x1[node_of(p, g, k)] = double2{cu[(size_t)g * p.nz + k], cv[(size_t)g * p.nz + k]};
+  if (std::memcmp(x0.data(), x1.data(), sizeof(double2) * x0.size())) return 1;
+  for (int b = 0; b < n; ++b) {
+    const size_t len = (size_t)p.nz * (p.nx[b] - 1) * (p.ny[b] - 1);
+    std::vector<double> ou(len, 7.0), ov(len, 7.0), pu(ou), pv(ou);  // 7: what neither writes
+    scatter_velocity(p, b, x0.data(), ou.data(), ov.data());
+    scatter_columns(p, b, cu.data(), cv.data(), pu.data(), pv.data());
+    if (std::memcmp(ou.data(), pu.data(), 8 * len) || std::memcmp(ov.data(), pv.data(), 8 * len)) return 2;
+  }
+  return 0;
+}
+
+// build_halo against its definition: every tile's list holds each column of
+// another tile that one of its columns has for a neighbour, once and in column
+// order, and col_loc names every neighbour's slot.
+extern "C" int emu_halo(int n, const bp_inputs* in) {
+  HostPlan p;
+  std::string err;
+  if (!build_plan(in, n, &p, &err)) return -1;
+  const HaloPlan h = build_halo(p);
+  const size_t NC = (size_t)p.ncols;
+  if ((int)h.begin.size() != p.ntiles + 1 || h.begin[0] != 0 || h.col_loc.size() != 9 * NC) return 1;
+  int most = 0;
+  for (int t = 0; t < p.ntiles; ++t) {
+    const int c0 = p.tile_col0[t], c1 = c0 + p.tile_ncols[t];
+    std::set<int> want;
+    for (int c = c0; c < c1; ++c)
+      for (int q = 0; q < 9; ++q) {
+        const int nb = p.col_nbr[q * NC + c];
+        if (nb >= 0 && (nb < c0 || nb >= c1)) want.insert(nb);
+      }
+    const int nh = h.begin[t + 1] - h.begin[t];
+    most = std::max(most, nh);
+    if (nh != (int)want.size()) return 2;
+    std::map<int, int> slot;
+    int i = 0;
+    for (int c : want) {
+      if (h.node[h.begin[t] + i] != p.col_node[c]) return 3;
+      slot[c] = p.W + i++;
+    }
+    for (int c = c0; c < c1; ++c)
+      for (int q = 0; q < 9; ++q) {
+        const int nb = p.col_nbr[q * NC + c], loc = h.col_loc[q * NC + c];
+        if (loc != (nb < 0 ? -1 : nb >= c0 && nb < c1 ? nb - c0 : slot[nb])) return 4;
+      }
+  }
+  return h.max_cols == most && (size_t)h.begin[p.ntiles] == h.node.size() ? 0 : 5;
 }

@@ -334,3 +334,51 @@ def test_ticket_shares_come_back_to_zero():
     for _ in range(50):
         a, b = shares(int(rng.integers(1, 1185))), shares(int(rng.integers(1, 1185)))
         assert int(rng.permutation(np.concatenate([a, b])).astype(np.uint64).sum()) % 2 ** 32 == 0
+
+
+@pytest.mark.parametrize("n,grain", [(0, 1), (1, 1), (5, 4096), (8191, 4096), (8192, 4096), (100_003, 4096), (9, 1),
+                                     (100, 0)])
+def test_parallel_for_covers_every_item_once(n, grain):
+    emu = C.CDLL(EMU)
+    emu.emu_parallel_for.argtypes = [C.c_long, C.c_long, _ip]
+    hits = np.zeros(max(n, 1), np.int32)
+    ranges = emu.emu_parallel_for(n, grain, _p(hits))
+    assert np.all(hits[:n] == 1) and 1 <= ranges <= min(8, max(1, n // max(grain, 1)))
+
+
+def _batches():
+    """One domain, uneven domains in a batch (periodic and not), one past a
+    thread's grain of columns, one with scattered holes, one without ice."""
+    holes = configs.slab(n=40)
+    keep = np.random.default_rng(8).uniform(size=holes.thck.shape) < 0.5
+    holes = holes.copy(thck=configs.halo_fill_cells(np.where(keep, holes.thck, 0.0)))
+    bare = configs.slab(n=12)
+    bare = bare.copy(thck=np.zeros_like(bare.thck))
+    return {"dome": [configs.dome()], "uneven": [configs.slab(n=21), configs.dome(n=15, nz=11, radius=11.0e3),
+                                                 configs.marine(n=24, dx=4000.0).copy(
+                                                     periodic=0, which_sparse=configs.SPARSE_PCG_STANDARD)],
+            "large": [configs.slab(n=101)], "holes": [holes], "bare": [bare, configs.slab(n=9)],
+            "levels": [configs.dome(n=13, nz=64, radius=7.0e3)], "two": [configs.slab(n=30, nz=2)]}
+
+
+BATCHES = _batches()
+
+
+@pytest.mark.parametrize("name", list(BATCHES))
+def test_velocities_by_columns_equal_node_by_node(name):
+    emu = C.CDLL(EMU)
+    ms = BATCHES[name]
+    preps = [solver.prepare(m)[0] for m in ms]
+    arr = (solver.Inputs * len(ms))(*[p.inputs for p in preps])
+    rng = np.random.default_rng(1)
+    u, v = ([rng.standard_normal(m.vshape3) for m in ms] for _ in range(2))
+    ptrs = lambda a: (_dp * len(a))(*[_p(x) for x in a])  # noqa: E731
+    assert emu.emu_columns(len(ms), arr, ptrs(u), ptrs(v)) == 0
+
+
+@pytest.mark.parametrize("name", list(BATCHES))
+def test_halo_tables_follow_their_definition(name):
+    emu = C.CDLL(EMU)
+    preps = [solver.prepare(m)[0] for m in BATCHES[name]]
+    arr = (solver.Inputs * len(preps))(*[p.inputs for p in preps])
+    assert emu.emu_halo(len(preps), arr) == 0
