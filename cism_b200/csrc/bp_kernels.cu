@@ -1534,9 +1534,10 @@ __global__ void __launch_bounds__(PER_SM == 2 ? 192 : kTile, PER_SM) k_pcg_resid
 // 220).  The arithmetic and its order are the per-node kernels' (bitwise the
 // same results).
 //
-// Barriers, all waits bounded (past the limit the CTA marks the instances'
-// sums as NaN, which ends their solve with BP_ERR_NAN): full[stage] -- the
-// stage's copies have landed (32 producer lanes and the bulk bytes);
+// Barriers, all waits bounded (past the limit a warp leaves as one, the producer
+// once its copies have landed or after another limit, and the CTA marks the
+// instances' sums as NaN, which ends their solve with BP_ERR_NAN): full[stage]
+// -- the stage's copies have landed (32 producer lanes and the bulk bytes);
 // empty[stage] -- every consumer warp is done with it; dfull[slot] -- a
 // descriptor (ring of four, two tiles ahead of the copies) has landed.
 //
@@ -1736,17 +1737,18 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
     };
     fetch(0);
     fetch(1);
-    for (int j = 0; ok; ++j) {
+    int j = 0;
+    for (; ok; ++j) {
       const int b = j % kStages;
       if (j >= kStages) ok = bar_wait(empty(b), ((j / kStages) - 1) & 1);
       ok = ok && bar_wait(dfull(j % kDescs), (j / kDescs) & 1);
-      if (!ok) break;
       const unsigned char* d = descs + (j % kDescs) * H.desc;
-      const int4 m = *reinterpret_cast<const int4*>(d);  // tile, columns, halo columns, instance
-      if (m.x < 0) break;
+      // tile, columns, halo columns, instance
+      const int4 m = ok ? *reinterpret_cast<const int4*>(d) : make_int4(-1, 0, 0, 0);
       const int nc = m.z < 0 ? 0 : W + m.z;
-      if (lane == 0) bar_expect(full(b), nc ? 16u * slots * NOWN : 0u);
-      __syncwarp();
+      if (lane == 0 && m.x >= 0) bar_expect(full(b), nc ? 16u * slots * NOWN : 0u);
+      ok = __all_sync(0xffffffffu, ok);  // the lanes leave together
+      if (!ok || m.x < 0) break;
       if (nc) {
         const size_t n0 = (size_t)m.x * slots, np = (size_t)v.npad;
         if (lane < NOWN) {
@@ -1768,6 +1770,10 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
       fetch(j + 2);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!ok) {  // the bulk copies of j tiles and j + 2 descriptors still land in this CTA's memory
+      for (int q = max(j - kStages, 0); q < j; ++q) bar_wait(full(q % kStages), (q / kStages) & 1);
+      for (int q = max(j + 2 - kDescs, 0); q < j + 2; ++q) bar_wait(dfull(q % kDescs), (q / kDescs) & 1);
+    }
   } else {  // consumers: thread i is node i of every tile
     const bool inside = i < slots;
     const int k = inside ? i >> v.lsh : 0, c = i & (W - 1);
@@ -1802,7 +1808,7 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
       const int4* p = reinterpret_cast<const int4*>(descs + (j % kDescs) * H.desc + 32 + 64 * c);
       return Nodes{p[0], p[1], p[2].x};
     };
-    ok = bar_wait(dfull(0), 0);
+    ok = __all_sync(0xffffffffu, bar_wait(dfull(0), 0));
     int4 m = ok ? desc_meta(0) : make_int4(-1, 0, 0, 0);
     uint4 rec = make_uint4(0, 0, 0, 0);
     Nodes nb = {make_int4(0, 0, 0, 0), make_int4(0, 0, 0, 0), 0};
@@ -1825,7 +1831,6 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
       if (mn.x >= 0) nb = desc_nodes(j + 1);  // after the last tile its own entries once more
       const uint4 recn = mn.x >= 0 ? desc_rec(j + 1) : rec;
       ok = ok && bar_wait(full(b), (j / kStages) & 1);
-      if (!ok) break;
       double yu = 0.0, yv = 0.0;
       double2 sn = make_double2(0.0, 0.0);
       const double2* src = stage_src(b);
@@ -1868,7 +1873,8 @@ __global__ void __launch_bounds__(THREADS, STORE == ST_SYM32 ? 2 : 1)
           }
         }
       }
-      __syncwarp();
+      ok = __all_sync(0xffffffffu, ok);  // the lanes leave together, with nothing stored
+      if (!ok) break;
       if (lane == 0) bar_arrive(empty(b));
       if (m.z < 0 || fp64) {
         if (mine) {
