@@ -477,110 +477,111 @@ bool build_plan(const bp_inputs* in, int n, HostPlan* p, std::string* err) {
     const int epc = solve2d ? 1 : nz - 1;  // elements per cell
     ip.elem_begin = cell_base * epc; ip.elem_end = (cell_base + ncl) * epc;
     parallel_for(nc, kColumnGrain, [&](size_t c_begin, size_t c_end) {
-    for (int c = (int)c_begin; c < (int)c_end; ++c) {
-      const int g = col_base + c;
-      const int i = cols[b][c].first, j = cols[b][c].second;
-      p->col_inst[g] = b;
-      p->col_ij[g] = i;
-      p->col_ij[NC + g] = j;
-      p->col_h[g] = I.stagthck[vtx(i, j, nx)];
-      for (int jA = -1; jA <= 1; ++jA)
-        for (int iA = -1; iA <= 1; ++iA)
-          p->col_nbr[(size_t)((jA + 1) * 3 + (iA + 1)) * NC + g] = cms[b].lookup(i + iA, j + jA);
-      // cells (i,j), (i+1,j), (i,j+1), (i+1,j+1): the reference's element order
-      const int ci[4] = {i, i + 1, i, i + 1}, cj[4] = {j, j, j + 1, j + 1};
-      for (int q = 0; q < 4; ++q) {
-        int id = -1;
-        if (ci[q] >= 1 && ci[q] <= nx && cj[q] >= 1 && cj[q] <= ny)
-          id = cellid[b][cel(ci[q], cj[q], nx)];
-        p->col_cells[(size_t)q * NC + g] = id;
-      }
-      if (I.sliding) {  // recomputed on the device at every Picard iteration
-        p->col_beta[g] = 0.0;
-        p->col_slide[g] = I.sliding->f_ground[vtx(i, j, nx)];
-        slide_vertex(*I.sliding, i, j, nx, &p->col_slide[(size_t)NC + g], &p->col_slide[2 * (size_t)NC + g]);
-      } else {
-        p->col_beta[g] = I.beta_internal[vtx(i, j, nx)];
-      }
-      if (diva) {
-        const size_t w = vtx(i, j, nx);
-        p->x2d_0[g] = double2{I.diva->uvel_2d[w], I.diva->vvel_2d[w]};
-        p->col_bt0[g] = double2{I.diva->btractx[w], I.diva->btracty[w]};
-        uint8_t bits = 0;
-        for (int q = 0; q < 4; ++q)
-          if (ci[q] >= 1 && ci[q] <= nx && cj[q] >= 1 && cj[q] <= ny &&
-              I.diva->ice_plus_land_mask[cel(ci[q], cj[q], nx)] == 1)
-            bits |= (uint8_t)(1u << q);
-        p->col_ipl[g] = bits;
-      }
-      if (l1l2) {
-        p->col_ds[g] = I.l1l2->dusrf_dx[vtx(i, j, nx)];
-        p->col_ds[(size_t)NC + g] = I.l1l2->dusrf_dy[vtx(i, j, nx)];
-      }
-      if (solve2d) {
-        // load summed over the levels (:2123-2137); the bed level's
-        // Dirichlet masks (:2878)
-        double lu = 0.0, lv = 0.0;
-        for (int k = 0; k < nz_in; ++k) {
-          lu = lu + I.loadu[vtx(i, j, nx) * nz_in + k];
-          lv = lv + I.loadv[vtx(i, j, nx) * nz_in + k];
+      for (int c = (int)c_begin; c < (int)c_end; ++c) {
+        const int g = col_base + c;
+        const int i = cols[b][c].first, j = cols[b][c].second;
+        p->col_inst[g] = b;
+        p->col_ij[g] = i;
+        p->col_ij[NC + g] = j;
+        p->col_h[g] = I.stagthck[vtx(i, j, nx)];
+        for (int jA = -1; jA <= 1; ++jA)
+          for (int iA = -1; iA <= 1; ++iA)
+            p->col_nbr[(size_t)((jA + 1) * 3 + (iA + 1)) * NC + g] = cms[b].lookup(i + iA, j + jA);
+        // cells (i,j), (i+1,j), (i,j+1), (i+1,j+1): the reference's element order
+        const int ci[4] = {i, i + 1, i, i + 1}, cj[4] = {j, j, j + 1, j + 1};
+        for (int q = 0; q < 4; ++q) {
+          int id = -1;
+          if (ci[q] >= 1 && ci[q] <= nx && cj[q] >= 1 && cj[q] <= ny)
+            id = cellid[b][cel(ci[q], cj[q], nx)];
+          p->col_cells[(size_t)q * NC + g] = id;
         }
-        p->load[p->col_node[g]] = double2{lu, lv};
-        const size_t bed = vtx(i, j, nx) * nz_in + (nz_in - 1);
-        p->dmask[p->col_node[g]] = (uint8_t)((I.umask_dirichlet[bed] == 1 ? 1 : 0) | (I.vmask_dirichlet[bed] == 1 ? 2 : 0));
-      } else {
-        for (int k = 0; k < nz; ++k) {
-          const size_t src = vtx(i, j, nx) * nz + k;
-          p->load[node_of(*p, g, k)] = double2{I.loadu[src], I.loadv[src]};
-          p->dmask[node_of(*p, g, k)] =
-              (uint8_t)((I.umask_dirichlet[src] == 1 ? 1 : 0) | (I.vmask_dirichlet[src] == 1 ? 2 : 0));
+        if (I.sliding) {  // recomputed on the device at every Picard iteration
+          p->col_beta[g] = 0.0;
+          p->col_slide[g] = I.sliding->f_ground[vtx(i, j, nx)];
+          slide_vertex(*I.sliding, i, j, nx, &p->col_slide[(size_t)NC + g], &p->col_slide[2 * (size_t)NC + g]);
+        } else {
+          p->col_beta[g] = I.beta_internal[vtx(i, j, nx)];
+        }
+        if (diva) {
+          const size_t w = vtx(i, j, nx);
+          p->x2d_0[g] = double2{I.diva->uvel_2d[w], I.diva->vvel_2d[w]};
+          p->col_bt0[g] = double2{I.diva->btractx[w], I.diva->btracty[w]};
+          uint8_t bits = 0;
+          for (int q = 0; q < 4; ++q)
+            if (ci[q] >= 1 && ci[q] <= nx && cj[q] >= 1 && cj[q] <= ny &&
+                I.diva->ice_plus_land_mask[cel(ci[q], cj[q], nx)] == 1)
+              bits |= (uint8_t)(1u << q);
+          p->col_ipl[g] = bits;
+        }
+        if (l1l2) {
+          p->col_ds[g] = I.l1l2->dusrf_dx[vtx(i, j, nx)];
+          p->col_ds[(size_t)NC + g] = I.l1l2->dusrf_dy[vtx(i, j, nx)];
+        }
+        if (solve2d) {
+          // load summed over the levels (:2123-2137); the bed level's
+          // Dirichlet masks (:2878)
+          double lu = 0.0, lv = 0.0;
+          for (int k = 0; k < nz_in; ++k) {
+            lu = lu + I.loadu[vtx(i, j, nx) * nz_in + k];
+            lv = lv + I.loadv[vtx(i, j, nx) * nz_in + k];
+          }
+          p->load[p->col_node[g]] = double2{lu, lv};
+          const size_t bed = vtx(i, j, nx) * nz_in + (nz_in - 1);
+          p->dmask[p->col_node[g]] =
+              (uint8_t)((I.umask_dirichlet[bed] == 1 ? 1 : 0) | (I.vmask_dirichlet[bed] == 1 ? 2 : 0));
+        } else {
+          for (int k = 0; k < nz; ++k) {
+            const size_t src = vtx(i, j, nx) * nz + k;
+            p->load[node_of(*p, g, k)] = double2{I.loadu[src], I.loadv[src]};
+            p->dmask[node_of(*p, g, k)] =
+                (uint8_t)((I.umask_dirichlet[src] == 1 ? 1 : 0) | (I.vmask_dirichlet[src] == 1 ? 2 : 0));
+          }
         }
       }
-    }
     });
     parallel_for(ncl, kColumnGrain, [&](size_t c_begin, size_t c_end) {
-    for (int c = (int)c_begin; c < (int)c_end; ++c) {
-      const int g = cell_base + c;
-      const int ic = cells[b][c].first, jc = cells[b][c].second;
-      p->cell_inst[g] = b;
-      p->cell_ij[g] = ic;
-      p->cell_ij[NCELL + g] = jc;
-      const int vi[4] = {ic - 1, ic, ic, ic - 1}, vj[4] = {jc - 1, jc - 1, jc, jc};
-      for (int q = 0; q < 4; ++q) {
-        const size_t v = vtx(vi[q], vj[q], nx);
-        p->cell_cols[(size_t)q * NCELL + g] = cms[b].lookup(vi[q], vj[q]);
-        p->cell_s[(size_t)q * NCELL + g] = I.stagusrf[v];
-        p->cell_h[(size_t)q * NCELL + g] = I.stagthck[v];
-        p->cell_beta[(size_t)q * NCELL + g] = I.sliding ? 0.0 : I.beta_internal[v];
+      for (int c = (int)c_begin; c < (int)c_end; ++c) {
+        const int g = cell_base + c;
+        const int ic = cells[b][c].first, jc = cells[b][c].second;
+        p->cell_inst[g] = b;
+        p->cell_ij[g] = ic;
+        p->cell_ij[NCELL + g] = jc;
+        const int vi[4] = {ic - 1, ic, ic, ic - 1}, vj[4] = {jc - 1, jc - 1, jc, jc};
+        for (int q = 0; q < 4; ++q) {
+          const size_t v = vtx(vi[q], vj[q], nx);
+          p->cell_cols[(size_t)q * NCELL + g] = cms[b].lookup(vi[q], vj[q]);
+          p->cell_s[(size_t)q * NCELL + g] = I.stagusrf[v];
+          p->cell_h[(size_t)q * NCELL + g] = I.stagthck[v];
+          p->cell_beta[(size_t)q * NCELL + g] = I.sliding ? 0.0 : I.beta_internal[v];
+          if (l1l2) {
+            p->cell_ds[(size_t)q * NCELL + g] = I.l1l2->dusrf_dx[v];
+            p->cell_ds[(size_t)(4 + q) * NCELL + g] = I.l1l2->dusrf_dy[v];
+          }
+        }
         if (l1l2) {
-          p->cell_ds[(size_t)q * NCELL + g] = I.l1l2->dusrf_dx[v];
-          p->cell_ds[(size_t)(4 + q) * NCELL + g] = I.l1l2->dusrf_dy[v];
+          p->cell_thck[g] = I.l1l2->thck[cel(ic, jc, nx)];
+          for (int k = 0; k < nl; ++k) p->cell_flwa[(size_t)g * nl + k] = I.l1l2->flwa[cel(ic, jc, nx) * nl + k];
+        }
+        if (diva) {  // efvs_qp_3d starts from the last solve's efvs on every point (:1166-1170)
+          p->cell_thck[g] = I.diva->thck[cel(ic, jc, nx)];
+          for (int q = 0; q < 4; ++q)
+            for (int k = 0; k < nl; ++k)
+              p->eq3_0[((size_t)g * 4 + q) * nl + k] = I.diva->efvs ? I.diva->efvs[cel(ic, jc, nx) * nl + k] : 0.0;
+        }
+        if (ssa) {
+          for (int k = 0; k < nl; ++k)
+            p->flwafact_layers[(size_t)g * nl + k] = I.flwafact[cel(ic, jc, nx) * nl + k];
+        }
+        if (ssa) {  // glissade_vertical_average (glissade_grid_operators.F90:1172-1236)
+          double f = 0.0;
+          for (int k = 0; k < nz_in - 1; ++k)
+            f = f + I.flwafact[cel(ic, jc, nx) * (nz_in - 1) + k] * (I.sigma[k + 1] - I.sigma[k]);
+          p->flwafact[g] = f;
+        } else {  // per layer (3-D elements; the L1L2 layer viscosities)
+          for (int k = 0; k < nl; ++k)
+            p->flwafact[(size_t)g * nl + k] = I.flwafact[cel(ic, jc, nx) * nl + k];
         }
       }
-      if (l1l2) {
-        p->cell_thck[g] = I.l1l2->thck[cel(ic, jc, nx)];
-        for (int k = 0; k < nl; ++k) p->cell_flwa[(size_t)g * nl + k] = I.l1l2->flwa[cel(ic, jc, nx) * nl + k];
-      }
-      if (diva) {  // efvs_qp_3d starts from the last solve's efvs on every point (:1166-1170)
-        p->cell_thck[g] = I.diva->thck[cel(ic, jc, nx)];
-        for (int q = 0; q < 4; ++q)
-          for (int k = 0; k < nl; ++k)
-            p->eq3_0[((size_t)g * 4 + q) * nl + k] = I.diva->efvs ? I.diva->efvs[cel(ic, jc, nx) * nl + k] : 0.0;
-      }
-      if (ssa) {
-        for (int k = 0; k < nl; ++k)
-          p->flwafact_layers[(size_t)g * nl + k] = I.flwafact[cel(ic, jc, nx) * nl + k];
-      }
-      if (ssa) {  // glissade_vertical_average (glissade_grid_operators.F90:1172-1236)
-        double f = 0.0;
-        for (int k = 0; k < nz_in - 1; ++k)
-          f = f + I.flwafact[cel(ic, jc, nx) * (nz_in - 1) + k] * (I.sigma[k + 1] - I.sigma[k]);
-        p->flwafact[g] = f;
-      } else {  // per layer (3-D elements; the L1L2 layer viscosities)
-        for (int k = 0; k < nl; ++k)
-          p->flwafact[(size_t)g * nl + k] = I.flwafact[cel(ic, jc, nx) * nl + k];
-      }
-    }
     });
     col_base += nc;
     cell_base += ncl;
