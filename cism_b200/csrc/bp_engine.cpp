@@ -657,9 +657,12 @@ void autotune(bp_problem* P) {
       if (res <= 0) continue;
       for (int g : {0, res * c->num_sms}) {
         // a batch's instances end at different iterations, and a persistent
-        // CTA walks past the tiles of those that have (16 domains: 102 us an
-        // iteration against 98 with a CTA per tile, which the dry pass, all
-        // instances solving, times 1 us slower)
+        // CTA walks past the tiles of those that have, which the dry pass, all
+        // instances solving, does not show.  Whole solves of six batches (16 to
+        // 64 uneven domains, 4 and 8 equal sheets, both precisions), persistent
+        // against a CTA per tile at the same occupancy target: 7 to 38% slower,
+        // but for target 8 in FP64 standard PCG (3% and 4% faster, where target 6
+        // with a CTA per tile is another 18% ahead)
         if (g > 0 && (g >= P->plan.ntiles || batch)) continue;
         v.minb_k = mb;
         v.grid_k = g;

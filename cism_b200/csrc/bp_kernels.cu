@@ -973,14 +973,16 @@ __global__ void __launch_bounds__(kTile) k_cg_update(DevView v) {
 //
 // What bounds it: the trips through L2.  One slot takes about 500 cycles to
 // another SM of the same die and 900 to the other die, an iteration makes
-// two trips in a row (three with a sum between), and each is followed by
-// two shuffle trees; the product from shared memory (864 B a node) is 1,900
-// of the 11,000 cycles of an iteration of the 34-tile dome.
-// Measured, launched kernels -> this one: 31 x 31 x 10 dome, FP64, standard
-// PCG, 34 tiles: 21 -> 6.1 us an iteration; 128 x 128 2-D marine sheet,
-// Chronopoulos-Gear, 39 tiles: 18 -> 5.7 us; 48 x 48 x 11 slab, 144 tiles:
-// 23 -> 7.1 us.  The limit (every tile resident: 148 tiles of FP64 rows, 296
-// of FP32 ones) is where shared memory ends.
+// two trips in a row (z and the halo's arrive with the second sum, or follow
+// the one sum of Chronopoulos-Gear), and each is followed by two shuffle
+// trees; the product from shared memory (864 B a node) is 1,900 of the 11,000
+// cycles of an iteration of the 34-tile dome.
+// Measured, launched kernels -> this one, diagonal preconditioner: 31 x 31 x
+// 10 dome, FP64, standard PCG, 34 tiles: 21 -> 5.6 us an iteration (7.8 with
+// the column preconditioner); 128 x 128 2-D marine sheet, Chronopoulos-Gear,
+// 39 tiles: 18 -> 5.1 us; 48 x 48 x 11 slab, 144 tiles: 23 -> 6.3 us.
+// The limit (every tile resident: 148 tiles of FP64 rows, 296 of FP32 ones) is
+// where shared memory ends.
 // ---------------------------------------------------------------------
 constexpr int kXchSpins = 1 << 22;  // a second or more of polling
 
